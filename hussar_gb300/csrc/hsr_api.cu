@@ -186,22 +186,21 @@ static hsr_status ensure_guide(SceneDev &sc, int P, GuideMem &out) {
     return HSR_OK;
 }
 
-static constexpr int32_t kTile = 4096;  // samples per work item
+static constexpr int32_t kTile = 4096;  // most samples a CTA takes at once
 
 // One trace launch over the poses' current budgets/offsets/weights in scratch.
-// `tile` is the samples per work item: 0 takes the scene's autotuned tile (or kTile);
-// the guided iterations pass their own (smaller tiles keep the SMs busy when a pass has
-// few samples). The autotuned CTAs per SM and queue threshold apply to plain passes.
+// The autotuned tile, CTAs per SM and queue threshold apply to plain passes.
 static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_config *rf, int32_t N,
                                const hsr_tracer_flags *fl, int32_t P, float sample_weight, bool per_pose_weights,
                                int32_t phase_mode, int32_t splat_mode, cudaStream_t st, const GuideMem *g,
-                               void *records = nullptr, int max_rec = 0, unsigned long long *counters = nullptr,
-                               int32_t tile = 0) {
-    const bool tuned = tile == 0 && !fl->doGuiding;
-    if (tile == 0) tile = (tuned && sc.tuned.tile > 0) ? sc.tuned.tile : kTile;
+                               void *records = nullptr, int max_rec = 0, unsigned long long *counters = nullptr) {
+    const bool wave = g_path_kernel == 0 && fl->useGeometricalOptics && !records && !counters;
+    const bool tuned = !fl->doGuiding;
+    const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile : kTile;
+    const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     cudaError_t e;
     if ((e = cudaMemsetAsync(s.counters + 2, 0, 8, st)) != cudaSuccess) return cuda_fail(e, "memset counter");
-    if (launch_tile_prefix(s.budget, P, tile, s.tile_start, st) != 0)
+    if (launch_tile_prefix(s.budget, P, items.samples, s.tile_start, st) != 0)
         return cuda_fail(cudaGetLastError(), "tile prefix launch");
     TraceParams p{};
     p.nodes = sc.nodes;
@@ -216,7 +215,8 @@ static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_conf
     p.offset = s.offset;
     p.tile_start = s.tile_start;
     p.sample_weight = sample_weight;
-    p.tile = tile;
+    p.tile = items.samples;
+    p.item_run = items.run;
     p.acc = s.acc;
     p.status = s.counters;
     p.work_counter = s.counters + 2;
@@ -240,7 +240,6 @@ static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_conf
     } else {
         p.flags.doGuiding = 0;
     }
-    const bool wave = g_path_kernel == 0 && fl->useGeometricalOptics && !records && !counters;
     int per_sm = wave ? wave_blocks_per_sm(N, false, p.do_guide != 0) : trace_blocks_per_sm(N, splat_mode, 0);
     if (wave && tuned) {
         if (sc.tuned.ctas_per_sm > 0) per_sm = std::min(per_sm, sc.tuned.ctas_per_sm);
@@ -355,7 +354,6 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
     std::vector<unsigned char> blk(K * it_bytes);
     std::vector<double> tw(P, 0.0);
     std::vector<char> any_clear(K, 0), any_active(K, 0);
-    std::vector<int64_t> iter_samples(K, 0);
     for (size_t k = 0; k < K; ++k) {
         unsigned char *h = blk.data() + k * it_bytes;
         int64_t *b = reinterpret_cast<int64_t *>(h);
@@ -376,7 +374,6 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
                 if (it.clear) tw[p] = 0.0;
                 tw[p] += double(it.budget) * double(it.weight);  // path.h:445, 466-475
                 active[p] = k + 1 < sched[p].size() ? 1 : 0;
-                iter_samples[k] += it.budget;
             } else {
                 b[p] = 0;
                 o[p] = 0;
@@ -409,11 +406,7 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
                                 : launch_clear_rows(s.acc, P, N, si.clear, st);
             if (rc != 0) return cuda_fail(cudaGetLastError(), "clear rows");
         }
-        // about four work items per resident CTA in this iteration
-        const int64_t per_item = (iter_samples[k] + 8 * int64_t(sc.sm_count) - 1) / (8 * int64_t(sc.sm_count));
-        int32_t tile = 256;
-        while (tile < kTile && tile < per_item) tile *= 2;
-        r = enqueue_pass(sc, si, rf, N, fl, P, 1.f, true, phase_mode, splat_mode, st, &g, nullptr, 0, nullptr, tile);
+        r = enqueue_pass(sc, si, rf, N, fl, P, 1.f, true, phase_mode, splat_mode, st, &g);
         if (r != HSR_OK) return r;
         if (any_active[k] &&
             launch_guide_step(P, si.active, g.samp_child, g.samp_p, g.train_child, g.train_acc, g.train_count, st) != 0)
@@ -1008,12 +1001,8 @@ hsr_status hsr_backend_run_guided(hsr_scene *s, const hsr_rf_config *rf, const h
         return cuda_fail(e, "guided run set-up");
     hsr_tracer_flags g = *fl;
     g.doGuiding = 1;
-    // about four work items per resident CTA, as the guided schedule's iterations use
-    const int64_t per_item = (budget + 8 * int64_t(s->dev.sm_count) - 1) / (8 * int64_t(s->dev.sm_count));
-    int32_t tile = 256;
-    while (tile < kTile && tile < per_item) tile *= 2;
     if ((st = enqueue_pass(s->dev, sc, rf, N, &g, 1, sample_weight, false, phase_mode, HSR_SPLAT_DIRICHLET16, strm,
-                           &guide->g, nullptr, 0, nullptr, tile)) != HSR_OK)
+                           &guide->g)) != HSR_OK)
         return st;
     if (launch_finalize(sc.acc, 1, N, sc.budget, sample_weight, nullptr, 0, sc.rows, strm) != 0)
         return cuda_fail(cudaGetLastError(), "finalize launch");

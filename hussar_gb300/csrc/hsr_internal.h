@@ -30,7 +30,7 @@ struct SynthOperand {
 
 // Launch shape of the plain wavefront pass chosen by the autotuner (0 fields: default).
 struct LaunchConfig {
-    int32_t tile = 0;             // samples per work item
+    int32_t tile = 0;             // most samples a CTA takes at once
     int32_t ctas_per_sm = 0;      // persistent grid: SMs x this (<= the occupancy limit)
     int32_t queue_threshold = 0;  // see TraceParams::queue_threshold
     int32_t field_on_hit = 0;     // see TraceParams::field_on_hit
@@ -40,6 +40,18 @@ struct LaunchConfig {
 constexpr int kWaveMaxQueueThreshold = 256;  // thresholds above 128: the 512-entry stack
 constexpr int kWaveDefaultQueue = 128;       // threshold 0 (the default) and up to 128: 384 entries
 constexpr int kWaveSmallQueue = 64;          // thresholds up to this run with a 320-entry stack
+// The work items of a wavefront launch whose tile (the most samples a CTA takes at once;
+// 4096 where none was chosen) is `tile`: one GENERATE stage each, pulled in runs of up to a
+// tile that shrink towards the end of the launch (pull_items in hsr_wave.cuh). A tile that
+// is no multiple of the stage is pulled whole.
+constexpr int32_t kWaveItem = 256;
+struct WaveItems {
+    int32_t samples;  // TraceParams::tile
+    int32_t run;      // TraceParams::item_run
+};
+inline WaveItems wave_items(int32_t tile) {
+    return tile % kWaveItem == 0 ? WaveItems{kWaveItem, tile / kWaveItem} : WaveItems{tile, 0};
+}
 
 // A resident scene: triangles + BVH on the device, plus per-scene scratch reused by
 // every simulate call on this scene (calls on one scene must not overlap).
@@ -143,6 +155,7 @@ struct TraceParams {
     const int64_t *tile_start;  // [pose_count + 1] prefix sum of tiles per pose
     float sample_weight;
     int32_t tile;           // samples per work item
+    int32_t item_run;       // wavefront kernel: most work items of one pull (0: always one)
     double *acc;            // [pose_count][N] complex (re, im) accumulators
     unsigned *status;       // status word
     unsigned *work_counter; // dynamic work item counter

@@ -138,11 +138,13 @@ extern "C" hsr_status hsr_simulate_batch_device_noalloc(hsr_scene *scene, const 
         set_last_error(std::string("clearing the static scratch: ") + cudaGetErrorString(e));
         return HSR_ERR_CUDA;
     }
-    // the scene's tuned work-item size where it has one, else 4096 samples (the prefix
-    // holds pose_count + 1 entries whatever the tile)
+    // the scene's tuned tile where it has one, else 4096 samples (the prefix holds
+    // pose_count + 1 entries whatever the tile)
+    const bool wave = g_path_kernel == 0 && flags->useGeometricalOptics != 0;
     const int32_t tile = sc->tuned.tile > 0 ? sc->tuned.tile : 4096;
+    const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     int64_t *tile_start = reinterpret_cast<int64_t *>(s->tile_start);
-    if (launch_tile_prefix(d_budget, P, tile, tile_start, strm) != 0) {
+    if (launch_tile_prefix(d_budget, P, items.samples, tile_start, strm) != 0) {
         set_last_error("tile prefix launch failed");
         return HSR_ERR_CUDA;
     }
@@ -159,12 +161,12 @@ extern "C" hsr_status hsr_simulate_batch_device_noalloc(hsr_scene *scene, const 
     p.offset = d_index_offset;
     p.tile_start = tile_start;
     p.sample_weight = 1.f;
-    p.tile = tile;
+    p.tile = items.samples;
+    p.item_run = items.run;
     p.acc = s->acc;
     p.status = s->counters;
     p.work_counter = s->counters + 2;
     std::string err;
-    const bool wave = g_path_kernel == 0 && flags->useGeometricalOptics != 0;
     int per_sm = wave ? wave_blocks_per_sm(N, false) : trace_blocks_per_sm(N, HSR_SPLAT_DIRICHLET16, 0);
     if (wave) {
         if (sc->tuned.ctas_per_sm > 0) per_sm = std::min(per_sm, sc->tuned.ctas_per_sm);

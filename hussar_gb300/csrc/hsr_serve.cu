@@ -396,6 +396,7 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
     int32_t tick_tile = kServeTile;
     while (tick_tile < kServeMaxTile && tick_samples >= 2 * int64_t(tick_tile) * kTilesPerCta * resident_ctas)
         tick_tile *= 2;
+    const WaveItems items = wave_items(tick_tile);
 
     // fill the tick block: segments in ascending remainder (shortest first)
     std::vector<int> order(n);
@@ -464,7 +465,7 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
                        std::memcmp(&(*first)->r.rf, &q->r.rf, sizeof(hsr_rf_config)) != 0) {
                 uniform = false;
             }
-            tile[P + 1] = tile[P] + (chunk[i] + tick_tile - 1) / tick_tile;
+            tile[P + 1] = tile[P] + (chunk[i] + items.samples - 1) / items.samples;
             maxN = std::max(maxN, q->r.samples_per_chirp);
             queue_threshold = std::min(queue_threshold, std::max(q->scene->tuned.queue_threshold, kWaveSmallQueue));
             if (q->scene->tuned.queue_threshold <= kWaveSmallQueue) queue_threshold = kWaveSmallQueue;
@@ -545,7 +546,8 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
         p.offset = reinterpret_cast<const int64_t *>(t.d_in + layout.offset);
         p.tile_start = reinterpret_cast<const int64_t *>(t.d_in + layout.tile);
         p.sample_weight = 1.f;
-        p.tile = tick_tile;
+        p.tile = items.samples;
+        p.item_run = items.run;
         p.acc = d_arena;
         p.status = reinterpret_cast<unsigned *>(t.d_in + layout.counters);
         p.work_counter = p.status + 2;

@@ -16,7 +16,8 @@
 // window offset l-16 of Frame::splat<16>, so one contribution's 33 bins are 33 distinct
 // shared-memory addresses updated in one pass. The CTA's range row lives in shared
 // memory and is flushed to the pose's FP64 accumulators when the CTA changes pose.
-// Work items are (pose, 4096-sample tile) pairs pulled from a device counter.
+// Work items are (pose, tile) pairs pulled from a device counter, one at a time or in
+// runs that shrink as the counter nears its end (pull_items).
 //
 // The kernel is a template over the phase mode; hsr_wave.cu instantiates the FP32
 // reference-phase forms without multiply-add contraction (so the float expressions round
@@ -58,6 +59,8 @@ template <int kCap> struct WaveShared {
     int count;
     int pose, pending_pose, exhausted;
     long long gen, gen_end, pending_first, pending_last;
+    long long item, item_end;   // work items pulled and not yet started
+    int item_want;              // length of the last run of items pulled
     long long since_flush;      // samples generated since the row was last flushed
     PoseJob job;                // mixed batches: the current pose's scene, chirp and row
     int cell_count[kThreads / 32][kPrimaryCells];  // GENERATE: samples per warp and cell
@@ -173,6 +176,33 @@ __device__ __forceinline__ float max_distance(const hsr_rf_config &rf) {
 }
 __device__ __forceinline__ float chirp_bandwidth(const hsr_rf_config &rf) { return rf.freqSlope * rf.rampTime; }
 
+// Pulls the run of work items a CTA takes next: [S.item, S.item_end), empty (false) once
+// the counter has passed `total`. With p.item_run = 0 it is one item. With p.item_run = R
+// it is half the CTA's share of what is left, between 1 and R items (guided
+// self-scheduling, Polychronopoulos and Kuck 1987): long runs of one pose while there is
+// plenty, which drain the path stack and flush the row rarely, and single 256-sample items
+// at the end, so that the CTAs finish together. What is left is estimated from the CTA's
+// last run, assuming that every other CTA has pulled as much since: a fresh look at the
+// counter would cost a second trip to the L2 per pull.
+// Fixed 4096-sample items left the chip idle wherever a launch had few of them, since one
+// item is milliseconds of a CTA's time on a dense scene. Whole calls, fixed items -> runs:
+// one dihedral pose of 2^14 samples (4 items for 608 CTAs) 137 -> 98 us; 33 poses on
+// 100 k triangles of boxes (1.7 M samples) 21.9 -> 12.2 ms; 27 far-field poses x 2^14
+// 747 -> 480 us; urban, 12 x 2^19 samples, 8.3 -> 7.3 ms; 96 poses on 1 M triangles (14 M
+// samples) 101 -> 91 ms.
+template <class Shared>
+__device__ __forceinline__ bool pull_items(const TraceParams &p, Shared &S, long long total) {
+    long long want = 1;
+    if (p.item_run > 0) {
+        const long long left = total - S.item_end - S.item_want * (long long)gridDim.x;
+        want = min((long long)p.item_run, max(1ll, left / (2ll * gridDim.x)));
+        S.item_want = int(want);
+    }
+    S.item = (long long)atomicAdd((unsigned long long *)p.work_counter, (unsigned long long)want);
+    S.item_end = min(S.item + want, total);
+    return S.item < total;
+}
+
 // FP64 accumulator row of a pose: the pose's job row (mixed), its listed row, or
 // pose-major rows of 2N.
 template <bool kMixed, class Shared>
@@ -218,6 +248,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
         S.pending_pose = -1;
         S.exhausted = 0;
         S.gen = S.gen_end = 0;
+        S.item = S.item_end = 0;
+        S.item_want = 0;
         S.since_flush = 0;
     }
     __syncthreads();
@@ -229,14 +261,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
         // thread 0 pulls work items while the generation range is used up
         if (tid == 0) {
             while (S.gen >= S.gen_end && !S.exhausted && S.pending_pose < 0) {
-                const long long item = (long long)atomicAdd((unsigned long long *)p.work_counter, 1ull);
-                if (item >= total) {
+                if (S.item >= S.item_end && !pull_items(p, S, total)) {
                     S.exhausted = 1;
                     break;
                 }
-                const int pose = find_pose(p.tile_start, p.pose_count, item);
-                const long long first = (item - __ldg(&p.tile_start[pose])) * p.tile;
-                const long long last = min(first + (long long)p.tile, (long long)__ldg(&p.budget[pose]));
+                // the pulled items of one pose are one sample range
+                const int pose = find_pose(p.tile_start, p.pose_count, S.item);
+                const long long pose_first = __ldg(&p.tile_start[pose]);
+                const long long stop = min(S.item_end, (long long)__ldg(&p.tile_start[pose + 1]));
+                const long long first = (S.item - pose_first) * p.tile;
+                const long long last = min((stop - pose_first) * p.tile, (long long)__ldg(&p.budget[pose]));
+                S.item = stop;
                 if (pose == S.pose) {
                     S.gen = first;
                     S.gen_end = last;
