@@ -299,12 +299,21 @@ __device__ __forceinline__ void ff_sample(const FfAnt &a, float u0, float u1, f3
 }
 
 // Returns false when the estimate is occluded or skipped (no record, no splat).
+// The occlusion query comes last, and only where its answer matters: an estimate that is
+// exactly zero (the receiver behind the surface, the reflected ray further from the
+// receiver than the filter's taper reaches, 3.7 m at 77 GHz) adds the same nothing either
+// way. Urban canyon (1 M triangles, 5 bounces): 3.02 -> 2.16 rays and 59 -> 40 nodes per
+// path, a 12 x 2^19-sample frame 6.6-7.3 -> 5.6 ms; sphere + ground 1.86 -> 1.83 rays; the
+// dense boxes, whose paths stay within metres of the sensor, skip none and run the same
+// (sweep of 96 poses 91 ms either way). kEvery (the recording
+// kernel) asks for every estimate, so that a record exists exactly where the path sees
+// the receiver.
 // depth == 0: direct TX->RX connection (only with onlyIndirect = false).
 // `nodes`/`tris` are the scene the pose traces, `rf`/`samples` its chirp and range bins
 // (uniform over a launch, or the pose's PoseJob in a mixed batch). kFF: far-field TX and
 // RX (`ff_rx` the receiver): FFAntenna::nee replaces NFAntenna::nee, and the direct term
 // is zero (FFAntenna::evaluate zeroes the ray, emitter.h:253-255).
-template <int kPhase, bool kCount, bool kFF = false>
+template <int kPhase, bool kCount, bool kFF = false, bool kEvery = false>
 __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *nodes, const DTri *tris,
                                          const hsr_rf_config &rf, int samples, const Ant &tx, const Ant &rx, int depth,
                                          f3 o, f3 d, f3 tmpd, f3 hit_n, const c3 &inc_H, const c3 &H, float time,
@@ -333,10 +342,6 @@ __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *node
         Hrx = mulcv(rx.rot, awr_eval(mulTv(rx.rot, neg3(nd))));
     }
     const float tMax = rr;
-    if (!fl.poDiffraction) {
-        if (kCount) (*rays)++;
-        if (any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt)) return false;
-    }
     const float nt = tMax;
     f3 no = o;
     float ntime = time;
@@ -419,10 +424,14 @@ __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *node
     out.splat = false;
     out.sample = 0.f;
     out.value = cf{0.f, 0.f};
-    // Integrator::splat (integrator.h:113-135)
-    if (!fl.produceDebugImage) {
-        if (sampleWeight == 0.f || v.re == 0.f || v.im == 0.f) return true;
+    // Integrator::splat's early-out (integrator.h:113-135)
+    const bool splats = fl.produceDebugImage || !(sampleWeight == 0.f || v.re == 0.f || v.im == 0.f);
+    const bool trains = p.do_guide && !(gw.re == 0.f && gw.im == 0.f);
+    if (!fl.poDiffraction && (kEvery || splats || trains)) {
+        if (kCount) (*rays)++;
+        if (any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt)) return false;
     }
+    if (!splats) return true;
     float sample;
     cf ph;
     if (kPhase == HSR_PHASE_REFERENCE_FP32) {
