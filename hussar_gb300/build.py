@@ -26,6 +26,7 @@ UNITS = {
     "hsr_api.cu": [],
     "hsr_bvh.cu": [],
     "hsr_guide.cu": [],
+    "hsr_local.cu": [],
     "hsr_synth.cu": [],
     "hsr_noalloc.cu": [],
     "hsr_serve.cu": [],

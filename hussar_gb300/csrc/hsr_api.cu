@@ -75,13 +75,14 @@ struct Scratch {
     double *acc;
     double *fine;  // fine-histogram rows (HSR_SPLAT_FINE_SYNTH), P x kFineRowPerBin N FP64 sums
     float *rows;
+    LocalList *local;    // neighbourhood lists (dense scenes)
     unsigned *counters;  // [0] status word, [2..3] 64-bit work counter
     size_t bytes;
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-static Scratch carve(void *base, int32_t P, int32_t N, bool fine) {
+static Scratch carve(void *base, int32_t P, int32_t N, bool fine, bool local) {
     Scratch s;
     char *p = static_cast<char *>(base);
     size_t off = 0;
@@ -106,6 +107,7 @@ static Scratch carve(void *base, int32_t P, int32_t N, bool fine) {
     s.acc = reinterpret_cast<double *>(take(sizeof(double) * 2 * size_t(P) * N));
     s.fine = fine ? reinterpret_cast<double *>(take(sizeof(double) * kFineRowPerBin * size_t(P) * N)) : nullptr;
     s.rows = reinterpret_cast<float *>(take(sizeof(float) * 2 * size_t(P) * N));
+    s.local = local ? reinterpret_cast<LocalList *>(take(sizeof(LocalList) * size_t(P))) : nullptr;
     s.bytes = off;
     return s;
 }
@@ -114,7 +116,8 @@ static Scratch carve(void *base, int32_t P, int32_t N, bool fine) {
 // the status word on `st`: every call reports the device status of its own work only.
 static hsr_status ensure_scratch(SceneDev &sc, int32_t P, int32_t N, Scratch &out, cudaStream_t st,
                                  bool fine = false) {
-    Scratch need = carve(nullptr, P, N, fine);
+    const bool local = sc.local_radius > 0.f;
+    Scratch need = carve(nullptr, P, N, fine, local);
     if (need.bytes > sc.scratch_bytes) {
         if (sc.scratch) {
             cudaDeviceSynchronize();
@@ -129,7 +132,7 @@ static hsr_status ensure_scratch(SceneDev &sc, int32_t P, int32_t N, Scratch &ou
         if (e != cudaSuccess) return cuda_fail(e, "scratch clear");
         sc.scratch_bytes = need.bytes;
     }
-    out = carve(sc.scratch, P, N, fine);
+    out = carve(sc.scratch, P, N, fine, local);
     cudaError_t e = cudaMemsetAsync(out.counters, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return cuda_fail(e, "status clear");
     return HSR_OK;
@@ -248,6 +251,11 @@ static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_conf
         p.coherent_order = sc.tuned.coherent_order;
     }
     int grid = sc.sm_count * per_sm;
+    if (wave && s.local && !s.far_field) {
+        if (launch_local_build(p, sc.local_radius, s.local, st) != 0)
+            return cuda_fail(cudaGetLastError(), "neighbourhood lists launch");
+        p.local = s.local;
+    }
     // timing events only outside stream capture (a captured graph must not record the
     // scene's events: it may outlive them)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -661,6 +669,7 @@ hsr_status hsr_scene_rebuild(hsr_scene *s, const float *vertices, int64_t vertex
         std::swap(a.vertex_count, b.vertex_count);
         std::swap(a.refit_order, b.refit_order);
         std::swap(a.refit_levels, b.refit_levels);
+        std::swap(a.local_radius, b.local_radius);
     }
     return hsr_scene_destroy(fresh);  // frees the old BVH, now held by `fresh`
 }
@@ -1501,7 +1510,8 @@ hsr_status hsr_batch_graph_create(hsr_scene *s, const hsr_rf_config *rf, int32_t
     std::unique_ptr<hsr_batch_graph> g(new hsr_batch_graph());
     g->scene = s;
     const bool fine = splat_mode == HSR_SPLAT_FINE_SYNTH;
-    const Scratch need = carve(nullptr, P, N, fine);
+    const bool local = s->dev.local_radius > 0.f;
+    const Scratch need = carve(nullptr, P, N, fine, local);
     std::string aerr;
     if (!dev_alloc(&g->scratch, need.bytes, aerr)) return fail(HSR_ERR_OUT_OF_MEMORY, "graph scratch: " + aerr);
     cudaError_t e;
@@ -1529,7 +1539,7 @@ hsr_status hsr_batch_graph_create(hsr_scene *s, const hsr_rf_config *rf, int32_t
             return st != HSR_OK ? st : cuda_fail(e, "graph synthesis operand");
         }
     }
-    const Scratch sc = carve(g->scratch, P, N, fine);
+    const Scratch sc = carve(g->scratch, P, N, fine, local);
     g->status = sc.counters;
     cudaStream_t cs = nullptr;
     if ((e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking)) != cudaSuccess) {

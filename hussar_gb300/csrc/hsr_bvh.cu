@@ -1182,6 +1182,11 @@ int bvh_build(SceneDev &s, const float *d_v, int64_t nv, const int32_t *d_idx, i
         cudaMemcpy(hd, depth, sizeof(hd), cudaMemcpyDeviceToHost);
         s.max_depth = hd[1];
         s.leaf_count = nt;
+        const int mrc = measure_density(s, st, err);
+        if (mrc) {
+            fail(mrc);
+            break;
+        }
     } while (false);
     cudaFree(lo);
     cudaFree(hi);

@@ -40,6 +40,7 @@ struct LaunchConfig {
 constexpr int kWaveMaxQueueThreshold = 256;  // thresholds above 128: the 512-entry stack
 constexpr int kWaveDefaultQueue = 128;       // threshold 0 (the default) and up to 128: 384 entries
 constexpr int kWaveSmallQueue = 64;          // thresholds up to this run with a 320-entry stack
+constexpr int kWaveLocalQueue = 256;         // launches with neighbourhood lists: 512 entries
 // The work items of a wavefront launch whose tile (the most samples a CTA takes at once;
 // 4096 where none was chosen) is `tile`: one GENERATE stage each, pulled in runs of up to a
 // tile that shrink towards the end of the launch (pull_items in hsr_wave.cuh). A tile that
@@ -82,6 +83,9 @@ struct SceneDev {
     void *frame_buf = nullptr;  // MIMO radar cube (hsr_simulate_frame), grown as needed
     size_t frame_bytes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // the radius of a neighbourhood list in this scene where it is dense enough for the
+    // poses to have one (hsr_local.cuh), else 0
+    float local_radius = 0.f;
     LaunchConfig tuned;  // set by hsr_autotune_batch / hsr_set_launch_config
     float last_kernel_ms = 0.f;
     bool timing_valid = false;
@@ -136,9 +140,25 @@ struct PoseJob {
     const DTri *tris;
     hsr_rf_config rf;
     int32_t samples;     // N of this pose (<= TraceParams::samples, which sizes the CTA row)
-    int32_t reserved;
+    float local_radius;  // SceneDev::local_radius of its scene
     int64_t acc_offset;  // first double of the pose's 2N accumulators in TraceParams::acc
 };
+
+// A pose's neighbourhood list (hsr_local.cuh): the triangles nearest its receiver, grouped
+// by plane, and the cube around the receiver that only they reach. planes 0: the pose has
+// none.
+constexpr int kLocalTris = 64;
+struct LocalList {
+    float4 plane[kLocalTris];  // n . (p - centre) = w
+    int slot[kLocalTris];      // plane j's triangles: slot[start[j]] .. slot[start[j + 1] - 1]
+    unsigned char start[kLocalTris + 4];
+    float cx, cy, cz;          // the receiver
+    float h;                   // half the cube's edge
+    float eps;                 // margin of the plane test
+    int planes;
+    int pad;
+};
+static_assert(sizeof(LocalList) % 16 == 0, "copied in 16-byte words");
 
 // Launch parameters of the trace kernels (POD, passed by value).
 struct TraceParams {
@@ -198,7 +218,15 @@ struct TraceParams {
     // guided launches: the guiding-tree slot of each pose in the g_* arrays (a serving
     // tick's requests own trees of the server's pool); nullptr: the pose index
     const int32_t *guide_slot;
+    // near-field wavefront launches on dense scenes: each pose's neighbourhood list;
+    // nullptr: every query goes to the BVH
+    const LocalList *local;
 };
+
+// SceneDev::local_radius of a freshly built scene. Returns 0, 2 or 3.
+int measure_density(SceneDev &s, cudaStream_t st, std::string &err);
+// The neighbourhood lists of a launch's poses (p.tx, p.rx and the scene or jobs set).
+int launch_local_build(const TraceParams &p, float radius, LocalList *out, cudaStream_t st);
 
 
 size_t guide_bytes_per_pose();

@@ -1,0 +1,276 @@
+// Builds the poses' neighbourhood lists (hsr_local.cuh) before a trace launch, and measures
+// whether a scene is dense enough for them.
+#include <algorithm>
+#include <vector>
+
+#include "hsr_local.cuh"
+
+namespace hsr {
+
+namespace {
+
+constexpr int kFrontier = 512;   // nodes of one tree level a search holds
+constexpr int kCandidates = 192;  // triangles a search holds
+constexpr int kSearchSteps = 14;
+
+// A scene whose point queries visit fewer nodes than this keeps to the BVH: the list's
+// plane tests cost as much as some ten divergent node visits per query, and the lists of
+// open scenes settle few queries (an urban canyon: 20 %, its point queries visit 10 nodes).
+constexpr float kDenseNodes = 48.f;
+
+struct Search {
+    int frontier[2][kFrontier];
+    int slot[kCandidates];
+    float dist[kCandidates];
+    int next, found;
+};
+
+// Chebyshev distance of a point to a box.
+__device__ __forceinline__ float box_distance(f3 c, float lx, float hx, float ly, float hy, float lz, float hz) {
+    return fmaxf(0.f, fmaxf(fmaxf(lx - c.x, c.x - hx), fmaxf(fmaxf(ly - c.y, c.y - hy), fmaxf(lz - c.z, c.z - hz))));
+}
+
+// The triangles whose bounding boxes come within h of c, by one warp, level by level down
+// the tree. Returns their number (S.slot, S.dist), or -1 when there are more than fit;
+// `visited` counts the nodes whose children were looked at.
+__device__ int collect(Search &S, const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 c, float h,
+                       int &visited) {
+    const int lane = threadIdx.x;
+    int cur = 0, n = 1;
+    visited = 0;
+    if (lane == 0) {
+        S.frontier[0][0] = 0;
+        S.found = 0;
+    }
+    while (n > 0) {
+        if (lane == 0) S.next = 0;
+        __syncwarp();
+        visited += n;
+        for (int i = lane; i < n; i += 32) {
+            const DNode N = load_node(nodes, S.frontier[cur][i]);
+            for (int w = 0; w < 2; ++w) {
+                const float dist = w == 0 ? box_distance(c, N.a.x, N.a.y, N.a.z, N.a.w, N.c.x, N.c.y)
+                                          : box_distance(c, N.b.x, N.b.y, N.b.z, N.b.w, N.c.z, N.c.w);
+                if (!(dist <= h)) continue;
+                const int child = w == 0 ? N.d.x : N.d.y;
+                if (child >= 0) {
+                    const int k = atomicAdd(&S.next, 1);
+                    if (k < kFrontier) S.frontier[cur ^ 1][k] = child;
+                    continue;
+                }
+                const int first = ~child >> 3, last = first + (~child & 7);
+                for (int s = first; s <= last; ++s) {
+                    const DTri T = load_tri(tris, s);
+                    const float ax = T.v0.x + T.e1.x, bx = T.v0.x + T.e2.x;
+                    const float ay = T.v0.y + T.e1.y, by = T.v0.y + T.e2.y;
+                    const float az = T.v0.z + T.e1.z, bz = T.v0.z + T.e2.z;
+                    const float td = box_distance(
+                        c, fminf(T.v0.x, fminf(ax, bx)), fmaxf(T.v0.x, fmaxf(ax, bx)), fminf(T.v0.y, fminf(ay, by)),
+                        fmaxf(T.v0.y, fmaxf(ay, by)), fminf(T.v0.z, fminf(az, bz)), fmaxf(T.v0.z, fmaxf(az, bz)));
+                    if (!(td <= h)) continue;
+                    const int k = atomicAdd(&S.found, 1);
+                    if (k < kCandidates) {
+                        S.slot[k] = s;
+                        S.dist[k] = td;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        n = S.next;
+        cur ^= 1;
+        if (n > kFrontier || S.found > kCandidates) return -1;
+        __syncwarp();
+    }
+    return S.found;
+}
+
+// A radius within which between kLocalTris + 1 and kCandidates triangles lie (their number
+// is returned, the search holds them), or 0 where the scene has no such radius.
+__device__ int find_radius(Search &S, const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 c, float &h) {
+    float lo = 0.f, hi = 0.f;  // too few within lo, too many within hi (0: not known)
+    for (int step = 0; step < kSearchSteps; ++step) {
+        int visited;
+        const int n = collect(S, nodes, tris, c, h, visited);
+        if (n > kLocalTris) return n;
+        if (n < 0)
+            hi = h;
+        else
+            lo = h;
+        h = lo == 0.f ? 0.4f * hi : hi == 0.f ? 2.5f * lo : sqrtf(lo * hi);
+        __syncwarp();
+    }
+    return 0;
+}
+
+// One warp per pose. The list is left empty (planes 0: the pose's queries all go to the
+// BVH) where the transmitter lies outside the cube or fewer than a quarter of 32 rays from
+// it, spread over the sphere, are settled by the list.
+__global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ jobs, const DNode *nodes,
+                                                    const DTri *tris, const hsr_antenna *__restrict__ tx,
+                                                    const hsr_antenna *__restrict__ rx, float guess,
+                                                    LocalList *__restrict__ out) {
+    __shared__ Search S;
+    __shared__ LocalList L;
+    __shared__ int near_slot[kLocalTris];
+    __shared__ float4 near_plane[kLocalTris];
+    __shared__ unsigned char near_group[kLocalTris];
+    const int pose = blockIdx.x, lane = threadIdx.x;
+    if (jobs) {
+        nodes = jobs[pose].nodes;
+        tris = jobs[pose].tris;
+        guess = jobs[pose].local_radius;
+    }
+    const f3 c = mk3(rx[pose].position[0], rx[pose].position[1], rx[pose].position[2]);
+    const f3 s = mk3(tx[pose].position[0], tx[pose].position[1], tx[pose].position[2]);
+    float h = guess;
+    const int n = guess > 0.f ? find_radius(S, nodes, tris, c, h) : 0;
+    if (n <= kLocalTris) {
+        if (lane == 0) out[pose].planes = 0;
+        return;
+    }
+    // the kLocalTris nearest in order, and the cube up to the next triangle's box
+    for (int i = lane; i < n; i += 32) {
+        const float di = S.dist[i];
+        int rank = 0;
+        for (int k = 0; k < n; ++k) rank += S.dist[k] < di || (S.dist[k] == di && S.slot[k] < S.slot[i]);
+        if (rank < kLocalTris) near_slot[rank] = S.slot[i];
+        if (rank == kLocalTris) L.h = local_half_edge(di, c);
+    }
+    __syncwarp();
+    const float half = L.h;
+    float eps = 0.f;
+    for (int j = lane; j < kLocalTris; j += 32) {
+        float e;
+        near_plane[j] = local_plane(load_tri(tris, near_slot[j]), c, half, e);
+        eps = fmaxf(eps, e);
+    }
+    for (int off = 16; off; off >>= 1) eps = fmaxf(eps, __shfl_xor_sync(0xffffffffu, eps, off));
+    eps += local_merge_margin(half);
+    __syncwarp();
+    // the planes in order of their nearest triangle: each triangle joins the first group
+    // whose plane it shares (lane l compares with groups l and l + 32)
+    static_assert(kLocalTris == 64, "two groups per lane");
+    int groups = 0, size[2] = {0, 0};
+    for (int j = 0; j < kLocalTris; ++j) {
+        const float4 pl = near_plane[j];
+        const unsigned lo = __ballot_sync(0xffffffffu, lane < groups && local_same_plane(L.plane[lane], pl, half));
+        const unsigned hi =
+            __ballot_sync(0xffffffffu, lane + 32 < groups && local_same_plane(L.plane[lane + 32], pl, half));
+        const int g = lo ? __ffs(int(lo)) - 1 : hi ? 31 + __ffs(int(hi)) : groups;
+        if (g == groups) {
+            if (lane == 0) L.plane[g] = pl;
+            ++groups;
+        }
+        if (lane == 0) near_group[j] = (unsigned char)g;
+        if (lane == (g & 31)) ++size[g >> 5];
+        __syncwarp();
+    }
+    // where each group starts, then its triangles
+    int first[2], total = 0;
+    for (int k = 0; k < 2; ++k) {
+        int sum = size[k];
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, off);
+            if (lane >= off) sum += v;
+        }
+        first[k] = total + sum - size[k];
+        total += __shfl_sync(0xffffffffu, sum, 31);
+        L.start[lane + 32 * k] = (unsigned char)first[k];
+    }
+    if (lane == 0) L.start[kLocalTris] = (unsigned char)kLocalTris;
+    for (int j = 0; j < kLocalTris; ++j) {
+        const int g = near_group[j];
+        if (lane == (g & 31)) L.slot[first[g >> 5]++] = near_slot[j];
+    }
+    if (lane == 0) {
+        L.cx = c.x;
+        L.cy = c.y;
+        L.cz = c.z;
+        L.eps = eps;
+        L.planes = groups;
+    }
+    __syncwarp();
+    bool settled = false;
+    if (L.h > 0.f && local_holds(L, s)) {
+        // 32 directions spread evenly over the sphere (a Fibonacci lattice)
+        const float y = 1.f - (2.f * lane + 1.f) / 32.f, r = sqrtf(fmaxf(0.f, 1.f - y * y));
+        float sn, cs;
+        sincosf(2.39996323f * lane, &sn, &cs);
+        float t;
+        settled = closest_local(L, tris, s, mk3(r * cs, y, r * sn), t) >= 0;
+    }
+    const int hits = __popc(__ballot_sync(0xffffffffu, settled));
+    if (lane == 0 && hits < 8) L.planes = 0;
+    __syncwarp();
+    const int *src = reinterpret_cast<const int *>(&L);
+    int *dst = reinterpret_cast<int *>(out + pose);
+    for (int k = lane; k < int(sizeof(LocalList) / sizeof(int)); k += 32) dst[k] = src[k];
+}
+
+// At kDensityPoints triangle centroids spread over the scene: the nodes a point query
+// visits and the radius of a neighbourhood.
+constexpr int kDensityPoints = 128;
+
+__global__ void __launch_bounds__(32) k_density(const DNode *__restrict__ nodes, const DTri *__restrict__ tris,
+                                                int64_t nt, float guess, float2 *__restrict__ out) {
+    __shared__ Search S;
+    const DTri T = load_tri(tris, int(nt * blockIdx.x / gridDim.x));
+    const f3 c = mk3(T.v0.x + (T.e1.x + T.e2.x) / 3.f, T.v0.y + (T.e1.y + T.e2.y) / 3.f,
+                     T.v0.z + (T.e1.z + T.e2.z) / 3.f);
+    int visited;
+    collect(S, nodes, tris, c, 0.f, visited);
+    __syncwarp();
+    float h = guess;
+    const int n = float(visited) >= 0.5f * kDenseNodes ? find_radius(S, nodes, tris, c, h) : 0;
+    if (threadIdx.x == 0) out[blockIdx.x] = make_float2(float(visited), n > 0 ? h : 0.f);
+}
+
+}  // namespace
+
+int measure_density(SceneDev &s, cudaStream_t st, std::string &err) {
+    s.local_radius = 0.f;
+    if (s.node_count < 4 * kDenseNodes) return 0;
+    DNode root;
+    float2 *d = nullptr;
+    if (!dev_alloc(&d, sizeof(float2) * kDensityPoints, err)) return 3;
+    cudaError_t e = cudaMemcpyAsync(&root, s.nodes, sizeof(root), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    std::vector<float2> v(kDensityPoints);
+    if (e == cudaSuccess) {
+        // a first radius: the cube that would hold a neighbourhood were the triangles
+        // spread evenly over the scene's box
+        const float ex = std::max(root.a.y, root.b.y) - std::min(root.a.x, root.b.x);
+        const float ey = std::max(root.a.w, root.b.w) - std::min(root.a.z, root.b.z);
+        const float ez = std::max(root.c.y, root.c.w) - std::min(root.c.x, root.c.z);
+        const float guess = 0.5f * std::max(ex, std::max(ey, ez)) * std::cbrt(float(kLocalTris) / float(s.tri_count));
+        k_density<<<kDensityPoints, 32, 0, st>>>(s.nodes, s.tris, s.tri_count, guess > 0.f ? guess : 1.f, d);
+        note_launches(1);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(v.data(), d, sizeof(float2) * kDensityPoints, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    if (e != cudaSuccess) {
+        err = std::string("density: ") + cudaGetErrorString(e);
+        return 2;
+    }
+    float visited = 0.f;
+    std::vector<float> radius;
+    for (const float2 &x : v) {
+        visited += x.x / kDensityPoints;
+        if (x.y > 0.f) radius.push_back(x.y);
+    }
+    if (visited < kDenseNodes || radius.size() < kDensityPoints / 2) return 0;
+    std::nth_element(radius.begin(), radius.begin() + radius.size() / 2, radius.end());
+    s.local_radius = radius[radius.size() / 2];
+    return 0;
+}
+
+int launch_local_build(const TraceParams &p, float radius, LocalList *out, cudaStream_t st) {
+    k_local_build<<<p.pose_count, 32, 0, st>>>(p.jobs, p.nodes, p.tris, p.tx, p.rx, radius, out);
+    note_launches(1);
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+}  // namespace hsr

@@ -9,6 +9,7 @@
 #include "hsr_common.cuh"
 #include "hsr_internal.h"
 #include "hsr_guide.cuh"
+#include "hsr_local.cuh"
 #include "hsr_traverse.cuh"
 
 namespace hsr {
@@ -312,14 +313,15 @@ __device__ __forceinline__ void ff_sample(const FfAnt &a, float u0, float u1, f3
 // `nodes`/`tris` are the scene the pose traces, `rf`/`samples` its chirp and range bins
 // (uniform over a launch, or the pose's PoseJob in a mixed batch). kFF: far-field TX and
 // RX (`ff_rx` the receiver): FFAntenna::nee replaces NFAntenna::nee, and the direct term
-// is zero (FFAntenna::evaluate zeroes the ray, emitter.h:253-255).
+// is zero (FFAntenna::evaluate zeroes the ray, emitter.h:253-255). `local`: the pose's
+// neighbourhood list where `o` lies in its cube, which then answers the occlusion query.
 template <int kPhase, bool kCount, bool kFF = false, bool kEvery = false>
 __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *nodes, const DTri *tris,
                                          const hsr_rf_config &rf, int samples, const Ant &tx, const Ant &rx, int depth,
                                          f3 o, f3 d, f3 tmpd, f3 hit_n, const c3 &inc_H, const c3 &H, float time,
                                          double plen, float r, float cosTheta, float freq, float sampleWeight,
                                          NeeOut &out, TraversalCounters *cnt, unsigned *rays,
-                                         const FfAnt *ff_rx = nullptr) {
+                                         const FfAnt *ff_rx = nullptr, const LocalList *local = nullptr) {
     const hsr_tracer_flags &fl = p.flags;
     f3 nd;
     float rr;
@@ -429,7 +431,9 @@ __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *node
     const bool trains = p.do_guide && !(gw.re == 0.f && gw.im == 0.f);
     if (!fl.poDiffraction && (kEvery || splats || trains)) {
         if (kCount) (*rays)++;
-        if (any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt)) return false;
+        if (local ? any_local(*local, tris, o, nd, tMax)
+                  : any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt))
+            return false;
     }
     if (!splats) return true;
     float sample;

@@ -456,7 +456,7 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
             j.tris = q->scene->tris;
             j.rf = q->r.rf;
             j.samples = q->r.samples_per_chirp;
-            j.reserved = 0;
+            j.local_radius = 0.f;
             j.acc_offset = q->arena_off / int64_t(sizeof(double));
             acc_row[P] = j.acc_offset;
             if (!first) {

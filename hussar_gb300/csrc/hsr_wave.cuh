@@ -56,7 +56,8 @@ template <int kCap> struct WaveShared {
     // the phase input: time of flight (FP32 reference phase, as float) or the FP64 path
     // length (split phase); each mode carries only its own
     double tlen[kCap];
-    int count;
+    int count;      // paths stacked from entry 0 up
+    int count_far;  // neighbourhood lists: paths stacked from the last entry down
     int pose, pending_pose, exhausted;
     long long gen, gen_end, pending_first, pending_last;
     long long item, item_end;   // work items pulled and not yet started
@@ -79,17 +80,25 @@ struct Guided {  // the guiding part of a path's state
 // weight) in five more [kCap] arrays after the training sums (`gst`, null otherwise).
 constexpr int kGuideStackFields = 5;
 
-template <int kPhase, int kCap>
+// Neighbourhood lists: the mark on a stacked path's depth that its origin, direction and
+// field are those of a ray the list did not settle; without it they are a hit's.
+constexpr int kRayPending = 1 << 30;
+
+// `far`: onto the upper end of the stack (kLocal).
+template <int kPhase, bool kLocal, int kCap>
 __device__ __forceinline__ void push_path(WaveShared<kCap> &S, float *gst, f3 o, f3 d, const c3 &H, f3 n, float time,
-                                          float r, float cosT, float freq, int depth, double plen, const Guided &g) {
-    // one shared atomic per warp: the lanes pushing here take consecutive slots
+                                          float r, float cosT, float freq, int depth, double plen, const Guided &g,
+                                          bool far = false) {
+    // one shared atomic per warp and end: the lanes pushing there take consecutive slots
     const unsigned active = __activemask();
     const int lane = threadIdx.x & 31;
-    const int leader = __ffs(active) - 1;
+    const unsigned mine = kLocal ? __match_any_sync(active, far) : active;
+    const int leader = __ffs(mine) - 1;
     int base = 0;
-    if (lane == leader) base = atomicAdd(&S.count, __popc(active));
+    if (lane == leader) base = atomicAdd(kLocal && far ? &S.count_far : &S.count, __popc(mine));
     base = __shfl_sync(active, base, leader);
-    const int slot = base + __popc(active & ((1u << lane) - 1u));  // < kCap by construction (see k_wave)
+    int slot = base + __popc(mine & ((1u << lane) - 1u));  // < kCap by construction (see k_wave)
+    if (kLocal && far) slot = kCap - 1 - slot;
     S.ox[slot] = o.x;
     S.oy[slot] = o.y;
     S.oz[slot] = o.z;
@@ -149,16 +158,10 @@ template <int kCap> __device__ __forceinline__ void order_by_key(WaveShared<kCap
     __syncthreads();
 }
 
-// Closest hit of the segment (o, d) and the bookkeeping of path.h:407-442 (GO mode).
-// Returns true (and the new state) when the path continues with a stored hit. The
-// reference's zero-field test (path.h:413, 439) is the caller's: in GO mode the field
-// does not change across the hit, so testing it before or after is the same.
-__device__ __forceinline__ bool walk(const TraceParams &p, const DNode *nodes, const DTri *tris, f3 o, f3 d,
-                                     float &time, float &r, double &plen, f3 &hp, f3 &n, float &cosT) {
-    float th;
-    int primh;
-    const int slot = closest_hit<false>(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status, nullptr);
-    if (slot < 0) return false;
+// The bookkeeping of a hit of the segment (o, d) (path.h:407-442, GO mode): the triangle
+// slot and its distance. Returns true (and the new state) when the path continues.
+__device__ __forceinline__ bool arrive(const DTri *tris, int slot, float th, f3 o, f3 d, float &time, float &r,
+                                       double &plen, f3 &hp, f3 &n, float &cosT) {
     DTri T = load_tri(tris, slot);
     n = hit_normal(T, d);
     hp = add3(o, scl3(th, d));
@@ -168,6 +171,18 @@ __device__ __forceinline__ bool walk(const TraceParams &p, const DNode *nodes, c
     time += th / kSpeedOfLight;
     plen += double(th);
     return true;
+}
+
+// Closest hit of the segment (o, d) and its bookkeeping. Returns true (and the new state)
+// when the path continues with a stored hit. The reference's zero-field test (path.h:413,
+// 439) is the caller's: in GO mode the field does not change across the hit, so testing it
+// before or after is the same.
+__device__ __forceinline__ bool walk(const TraceParams &p, const DNode *nodes, const DTri *tris, f3 o, f3 d,
+                                     float &time, float &r, double &plen, f3 &hp, f3 &n, float &cosT) {
+    float th;
+    int primh;
+    const int slot = closest_hit<false>(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status, nullptr);
+    return slot >= 0 && arrive(tris, slot, th, o, d, time, r, plen, hp, n, cosT);
 }
 
 // PathTracer::run's derived chirp quantities (path.h:240, radar.h:128-130).
@@ -211,11 +226,34 @@ __device__ __forceinline__ double *pose_row(const TraceParams &p, const Shared &
     return p.acc + (p.acc_row ? __ldg(&p.acc_row[pose]) : 2 * int64_t(pose) * p.samples);
 }
 
+// Dynamic shared memory of a launch: the stack, the range row of N bins and, guided, the
+// CTA's training sums and the guiding part of the stacked paths; then, on dense scenes, the
+// pose's neighbourhood list (local_offset).
+template <int kCap> __host__ __device__ constexpr size_t wave_smem_of(int samples, bool guided) {
+    return sizeof(WaveShared<kCap>) + 2 * size_t(samples) * sizeof(float) +
+           (guided ? (kGuideMaxNodes + kGuideStackFields * kCap) * sizeof(float) : 0);
+}
+template <int kCap> __host__ __device__ constexpr size_t local_offset(int samples, bool guided) {
+    return (wave_smem_of<kCap>(samples, guided) + 15) & ~size_t(15);
+}
+template <int kQueue> size_t wave_smem_for(int samples, bool guided, bool local = false) {
+    constexpr int kCap = kThreads + kQueue;
+    return local ? local_offset<kCap>(samples, guided) + sizeof(LocalList) : wave_smem_of<kCap>(samples, guided);
+}
+
 // Four CTAs per SM (64 registers): the spills cost less than the latency the extra
 // warps hide (measured: 1.2x on the sphere bench, 1.13x on the serving mix over two).
 // kLazy (the field_on_hit launch shape): with indirect-only paths, a primary ray's
 // antenna field is formed only once the ray has hit something.
-template <int kPhase, bool kMixed, int kQueue, bool kFF = false, bool kLazy = false>
+// kLocal (dense scenes): each pose has a neighbourhood list (p.local, hsr_local.cuh). The
+// stack (512 entries: 384 ran 2 % slower) then has two ends. Paths whose hit point lies in the list's cube are at the lower
+// end; their EXTEND asks the list alone: the occlusion query is settled by it, and a
+// closest-hit query that is not becomes a pending ray at the upper end. The upper end holds
+// those and the paths outside the cube; its EXTEND asks the BVH. A stage works on one end
+// (the fuller one), so a warp never waits for one lane's tree traversal among 31 list
+// lookups. Active lanes 14 -> 26 of 32, instructions per path a fifth (boxes, 1 M triangles).
+// field_on_hit and coherent_order don't apply here.
+template <int kPhase, bool kMixed, int kQueue, bool kFF = false, bool kLazy = false, bool kLocal = false>
 __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
     constexpr int kCap = kThreads + kQueue;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -225,6 +263,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
     // guided launches: the CTA's training sums (second moment per training-tree node)
     float *s_g = s_re + 2 * p.samples;
     float *gst = p.do_guide ? s_g + kGuideMaxNodes : nullptr;
+    // the pose's list, after the row (and the guiding part): 16-byte aligned
+    LocalList &L = *reinterpret_cast<LocalList *>(
+        smem_raw + (kLocal ? local_offset<kCap>(p.samples, p.do_guide != 0) : 0));
     const int tid = threadIdx.x;
     const hsr_tracer_flags &fl = p.flags;
     // the scene, chirp and row of the current pose: launch-uniform, or the pose's job
@@ -244,6 +285,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
         for (int k = tid; k < kGuideMaxNodes; k += kThreads) s_g[k] = 0.f;
     if (tid == 0) {
         S.count = 0;
+        S.count_far = 0;
         S.pose = -1;
         S.pending_pose = -1;
         S.exhausted = 0;
@@ -283,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             }
         }
         __syncthreads();
-        const int count = S.count;
+        const int count = S.count, count_far = kLocal ? S.count_far : 0;
         const long long gen = S.gen, gen_end = S.gen_end;
         const int pending = S.pending_pose;
         const int exhausted = S.exhausted;
@@ -299,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             continue;
         }
 
-        if (gen < gen_end && count <= queue_threshold) {
+        if (gen < gen_end && count + count_far <= queue_threshold) {
             // ---------------- GENERATE ----------------
             if (tid == 0) {
                 S.gen = min(gen + (long long)kThreads, gen_end);
@@ -308,7 +350,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             // the stage's samples gen + [0, n), ordered by primary cell: thread t traces
             // sample gen + S.order[t]
             const int n_stage = int(min((long long)kThreads, gen_end - gen));
-            if (p.coherent_order) {
+            const bool ordered = !kLocal && p.coherent_order;
+            if (ordered) {
                 int key = kPrimaryCells;
                 if (tid < n_stage) {
                     const uint64_t h0 = uint64_t(pc.offset + gen + tid);
@@ -317,7 +360,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                 }
                 order_by_key(S, key);
             }
-            const long long s = gen + (p.coherent_order && tid < n_stage ? S.order[tid] : tid);
+            const long long s = gen + (ordered && tid < n_stage ? S.order[tid] : tid);
+            const bool local = kLocal && L.planes > 0;  // the sensor lies in the cube
             bool has_item = false;
             float4 item = make_float4(0.f, 0.f, 0.f, 0.f);
             if (s < gen_end) {
@@ -346,7 +390,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                     NeeOut ne;
                     if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, 0, o, d,
                                                      mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f), H, H, 0.f, 0.0, 0.f,
-                                                     1.f, freq, pc.weight, ne, nullptr, nullptr, &S.ff[1]) &&
+                                                     1.f, freq, pc.weight, ne, nullptr, nullptr, &S.ff[1],
+                                                     local ? &L : nullptr) &&
                         ne.splat) {
                         if (pc.fine_row) {
                             splat_fine(pc.fine_row, p.fine_bins, ne.sample, ne.value);
@@ -361,12 +406,22 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                     float time = 0.f, r = 0.f, cosT;
                     double plen = 0.0;
                     f3 hp, n;
-                    if (walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n, cosT)) {
+                    bool hit, pending = false;
+                    if (local) {
+                        const int slot = closest_local(L, HSR_TRIS, o, d, cosT);
+                        pending = slot < 0;
+                        hit = !pending && arrive(HSR_TRIS, slot, cosT, o, d, time, r, plen, hp, n, cosT);
+                    } else {
+                        hit = walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n, cosT);
+                    }
+                    if (hit || pending) {
                         // deferred: the field now (the same operations as antenna_sample); a
                         // zero field ends the path as the reference's test before tracing would
                         if (deferred) H = c3_scl(antenna_field(pc.tx, ldir), 1.f / g.pdf);
                         if (!deferred || !c3_is_zero(H)) {
-                            push_path<kPhase, kCap>(S, gst, hp, d, H, n, time, r, cosT, freq, 1, plen, g);
+                            push_path<kPhase, kLocal, kCap>(S, gst, pending ? o : hp, d, H, n, time, r, cosT, freq,
+                                                            pending ? kRayPending : 1, plen, g,
+                                                            pending || (kLocal && !(local && local_holds(L, hp))));
                             alive = true;
                         }
                     }
@@ -378,9 +433,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             continue;
         }
 
-        if (count > 0) {
+        if (count + count_far > 0) {
             // ---------------- EXTEND ----------------
-            const int n = min(count, kThreads);
+            // kLocal: the fuller end of the stack; the lower one asks the pose's list
+            const bool local = kLocal && count > count_far;
+            const bool upper = kLocal && !local;
+            const int n = min(upper ? count_far : count, kThreads);
             const bool mine = tid < n;
             f3 o, din, nrm;
             c3 Hin;
@@ -390,7 +448,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             Guided g{0.f, 0.f, 1.f, cf{0.f, 0.f}};
             // the popped paths, ordered by the octant of their reflected direction: thread t
             // continues stack entry count - 1 - S.order[t]
-            if (p.coherent_order) {
+            const bool ordered = !kLocal && p.coherent_order;
+            if (ordered) {
                 int key = kPrimaryCells;
                 if (mine) {
                     const int e = count - 1 - tid;
@@ -402,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                 order_by_key(S, key);
             }
             if (mine) {
-                const int slot = count - 1 - (p.coherent_order ? S.order[tid] : tid);
+                const int slot = upper ? kCap - count_far + tid : count - 1 - (ordered ? S.order[tid] : tid);
                 if (gst)
                     g = Guided{gst[slot], gst[kCap + slot], gst[2 * kCap + slot],
                                cf{gst[3 * kCap + slot], gst[4 * kCap + slot]}};
@@ -421,34 +480,56 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                 depth = S.depth[slot];
             }
             __syncthreads();  // all pops read before the stack shrinks
-            if (tid == 0) S.count = count - n;
+            if (tid == 0) {
+                if (upper)
+                    S.count_far = count_far - n;
+                else
+                    S.count = count - n;
+            }
             __syncthreads();
             bool has_item = false;
             float4 item = make_float4(0.f, 0.f, 0.f, 0.f);
             if (mine) {
                 f3 d = din;
                 c3 H = Hin;
-                reflect(nrm, d, H);
-                NeeOut ne;
-                if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, depth, o, d, din,
-                                                 nrm, Hin, H, time, plen, r, cosT, freq, pc.weight, ne, nullptr,
-                                                 nullptr, &S.ff[1])) {
-                    g.gw = cadd(g.gw, ne.gw_add);
-                    if (ne.splat) {
-                        if (pc.fine_row) {
-                            splat_fine(pc.fine_row, p.fine_bins, ne.sample, ne.value);
-                        } else {
-                            item = splat_item(ne.sample, ne.value);
-                            has_item = true;
+                const bool resumed = kLocal && (depth & kRayPending);  // its estimate is done
+                if (kLocal) depth &= kRayPending - 1;
+                bool onward = resumed;
+                if (!resumed) {
+                    reflect(nrm, d, H);
+                    NeeOut ne;
+                    if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, depth, o, d, din,
+                                                     nrm, Hin, H, time, plen, r, cosT, freq, pc.weight, ne, nullptr,
+                                                     nullptr, &S.ff[1], local ? &L : nullptr)) {
+                        g.gw = cadd(g.gw, ne.gw_add);
+                        if (ne.splat) {
+                            if (pc.fine_row) {
+                                splat_fine(pc.fine_row, p.fine_bins, ne.sample, ne.value);
+                            } else {
+                                item = splat_item(ne.sample, ne.value);
+                                has_item = true;
+                            }
                         }
                     }
+                    onward = !(depth >= fl.maxDepth || r >= HSR_MAXDIST) && !c3_is_zero(H);
                 }
                 bool alive = false;
-                if (!(depth >= fl.maxDepth || r >= HSR_MAXDIST) && !c3_is_zero(H)) {
+                if (onward) {
                     f3 hp, n2;
                     float cosT2;
-                    if (walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n2, cosT2)) {
-                        push_path<kPhase, kCap>(S, gst, hp, d, H, n2, time, r, cosT2, freq, depth + 1, plen, g);
+                    bool hit, unsettled = false;
+                    if (local) {
+                        const int slot = closest_local(L, HSR_TRIS, o, d, cosT2);
+                        unsettled = slot < 0;
+                        hit = !unsettled && arrive(HSR_TRIS, slot, cosT2, o, d, time, r, plen, hp, n2, cosT2);
+                    } else {
+                        hit = walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n2, cosT2);
+                    }
+                    if (hit || unsettled) {
+                        push_path<kPhase, kLocal, kCap>(S, gst, unsettled ? o : hp, d, H, n2, time, r, cosT2, freq,
+                                                        unsettled ? depth | kRayPending : depth + 1, plen, g,
+                                                        unsettled ||
+                                                            (kLocal && !(L.planes > 0 && local_holds(L, hp))));
                         alive = true;
                     }
                 }
@@ -467,7 +548,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             }
             cur_pose = pending;
             pc = load_pose(p, cur_pose);
-            __syncthreads();  // every thread is done with the old pose's job
+            __syncthreads();  // every thread is done with the old pose's job and list
+            if (kLocal) {
+                const int4 *src = reinterpret_cast<const int4 *>(p.local + pending);
+                int4 *dst = reinterpret_cast<int4 *>(&L);
+                for (int k = tid; k < int(sizeof(LocalList) / sizeof(int4)); k += kThreads) dst[k] = __ldg(src + k);
+            }
             if (tid == 0) {
                 if (kMixed) {
                     S.job = p.jobs[pending];
@@ -501,14 +587,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
 #undef HSR_BANDWIDTH
 }
 
-// Dynamic shared memory of a launch: the stack, the range row of N bins and, guided, the
-// CTA's training sums and the guiding part of the stacked paths.
-template <int kQueue> size_t wave_smem_for(int samples, bool guided) {
-    constexpr int kCap = kThreads + kQueue;
-    return sizeof(WaveShared<kCap>) + 2 * size_t(samples) * sizeof(float) +
-           (guided ? (kGuideMaxNodes + kGuideStackFields * kCap) * sizeof(float) : 0);
-}
-
 // The stack capacity (as its GENERATE threshold) a launch with threshold q runs: 64 for
 // 1..64, 256 above 128, else (0 = the default, or 65..128) 128.
 inline int wave_capacity(int32_t q) {
@@ -517,12 +595,12 @@ inline int wave_capacity(int32_t q) {
 }
 
 // The launch of one instantiation.
-template <int kPhase, bool kMixed, int kQueue, bool kFF = false, bool kLazy = false>
+template <int kPhase, bool kMixed, int kQueue, bool kFF = false, bool kLazy = false, bool kLocal = false>
 void wave_instance(const TraceParams &p, int grid, cudaStream_t st) {
-    const size_t smem = wave_smem_for<kQueue>(p.samples, p.do_guide != 0);
-    cudaFuncSetAttribute(k_wave<kPhase, kMixed, kQueue, kFF, kLazy>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(smem));
-    k_wave<kPhase, kMixed, kQueue, kFF, kLazy><<<grid, kThreads, smem, st>>>(p);
+    const size_t smem = wave_smem_for<kQueue>(p.samples, p.do_guide != 0, kLocal);
+    auto *kernel = k_wave<kPhase, kMixed, kQueue, kFF, kLazy, kLocal>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    kernel<<<grid, kThreads, smem, st>>>(p);
 }
 
 // The uniform form at one capacity, with the primary field formed eagerly or on a hit.
@@ -541,6 +619,11 @@ template <int kPhase> void wave_dispatch(const TraceParams &p, int grid, cudaStr
     const int cap = wave_capacity(p.queue_threshold);
     if (p.ff_tx) {  // far-field runs: the uniform form at the default capacity
         wave_instance<kPhase, false, kWaveDefaultQueue, true>(p, grid, st);
+    } else if (p.local) {
+        if (p.jobs)
+            wave_instance<kPhase, true, kWaveLocalQueue, false, false, true>(p, grid, st);
+        else
+            wave_instance<kPhase, false, kWaveLocalQueue, false, false, true>(p, grid, st);
     } else if (p.jobs) {  // the mixed form is built at the two smaller capacities
         if (p.queue_threshold > kWaveSmallQueue)
             wave_instance<kPhase, true, kWaveDefaultQueue>(p, grid, st);
