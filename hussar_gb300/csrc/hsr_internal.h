@@ -83,8 +83,8 @@ struct SceneDev {
     void *frame_buf = nullptr;  // MIMO radar cube (hsr_simulate_frame), grown as needed
     size_t frame_bytes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // the radius of a neighbourhood list in this scene where it is dense enough for the
-    // poses to have one (hsr_local.cuh), else 0
+    // the first radius of the search for a pose's neighbourhood list where this scene is
+    // dense enough for the poses to have one (hsr_local.cuh), else 0
     float local_radius = 0.f;
     LaunchConfig tuned;  // set by hsr_autotune_batch / hsr_set_launch_config
     float last_kernel_ms = 0.f;

@@ -9,8 +9,9 @@ namespace hsr {
 
 namespace {
 
-constexpr int kFrontier = 512;   // nodes of one tree level a search holds
-constexpr int kCandidates = 192;  // triangles a search holds
+constexpr int kFrontier = 1024;    // nodes of one tree level a search holds
+constexpr int kCandidates = 1024;  // triangles a search holds
+constexpr int kNearest = 192;      // triangles that are ranked
 constexpr int kSearchSteps = 14;
 
 // A scene whose point queries visit fewer nodes than this keeps to the BVH: the list's
@@ -22,6 +23,8 @@ struct Search {
     int frontier[2][kFrontier];
     int slot[kCandidates];
     float dist[kCandidates];
+    int near_slot[kNearest];
+    float near_dist[kNearest];
     int next, found;
 };
 
@@ -85,22 +88,66 @@ __device__ int collect(Search &S, const DNode *__restrict__ nodes, const DTri *_
     return S.found;
 }
 
-// A radius within which between kLocalTris + 1 and kCandidates triangles lie (their number
-// is returned, the search holds them), or 0 where the scene has no such radius.
-__device__ int find_radius(Search &S, const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 c, float &h) {
+// The more than kLocalTris and at most kNearest triangles nearest c (S.near_slot,
+// S.near_dist; their number is returned), or 0 where there are no such. A search down the
+// tree costs 20 us, most of it latency (25 levels of dependent loads), so it takes in up to 1024
+// triangles around a first radius `h` and the radius is then narrowed on their distances:
+// one or two searches for most poses. Searching again until 65 to 192 triangles were in
+// reach, the lists of 96 poses (1 M triangles) took 220 us, now 129; those of 1999 poses
+// (20 k triangles) 228, now 188.
+__device__ int find_nearest(Search &S, const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 c, float h) {
+    const int lane = threadIdx.x;
     float lo = 0.f, hi = 0.f;  // too few within lo, too many within hi (0: not known)
-    for (int step = 0; step < kSearchSteps; ++step) {
+    int n = 0;
+    for (int step = 0; step < kSearchSteps && n <= kLocalTris; ++step) {
         int visited;
-        const int n = collect(S, nodes, tris, c, h, visited);
-        if (n > kLocalTris) return n;
+        n = collect(S, nodes, tris, c, h, visited);
         if (n < 0)
             hi = h;
         else
             lo = h;
-        h = lo == 0.f ? 0.4f * hi : hi == 0.f ? 2.5f * lo : sqrtf(lo * hi);
+        if (n <= kLocalTris) h = lo == 0.f ? 0.4f * hi : hi == 0.f ? 2.5f * lo : sqrtf(lo * hi);
         __syncwarp();
     }
-    return 0;
+    if (n <= kLocalTris) return 0;
+    // bisection for a distance that at most kNearest and more than kLocalTris are within
+    auto within = [&](float t) {
+        int m = 0;
+        for (int i = lane; i < n; i += 32) m += S.dist[i] <= t;
+        return __reduce_add_sync(0xffffffffu, m);
+    };
+    float below = 0.f, t = h;
+    int m = n;
+    for (int step = 0; step < 24 && (m > kNearest || m <= kLocalTris); ++step) {
+        const float mid = 0.5f * (below + h);
+        m = within(mid);
+        if (m > kNearest) h = mid;
+        if (m <= kLocalTris) below = mid;
+        t = mid;
+    }
+    if (m > kNearest || m <= kLocalTris) return 0;  // too many at one distance
+    int at = 0;
+    for (int i = lane; i - lane < n; i += 32) {
+        const bool in = i < n && S.dist[i] <= t;
+        const unsigned mask = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            const int k = at + __popc(mask & ((1u << lane) - 1u));
+            S.near_slot[k] = S.slot[i];
+            S.near_dist[k] = S.dist[i];
+        }
+        at += __popc(mask);
+    }
+    __syncwarp();
+    return m;
+}
+
+// The rank of one of the n nearest.
+__device__ __forceinline__ int rank_of(const Search &S, int n, int i) {
+    const float di = S.near_dist[i];
+    const int si = S.near_slot[i];
+    int rank = 0;
+    for (int k = 0; k < n; ++k) rank += S.near_dist[k] < di || (S.near_dist[k] == di && S.near_slot[k] < si);
+    return rank;
 }
 
 // One warp per pose. The list is left empty (planes 0: the pose's queries all go to the
@@ -123,19 +170,16 @@ __global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ 
     }
     const f3 c = mk3(rx[pose].position[0], rx[pose].position[1], rx[pose].position[2]);
     const f3 s = mk3(tx[pose].position[0], tx[pose].position[1], tx[pose].position[2]);
-    float h = guess;
-    const int n = guess > 0.f ? find_radius(S, nodes, tris, c, h) : 0;
+    const int n = guess > 0.f ? find_nearest(S, nodes, tris, c, guess) : 0;
     if (n <= kLocalTris) {
         if (lane == 0) out[pose].planes = 0;
         return;
     }
     // the kLocalTris nearest in order, and the cube up to the next triangle's box
     for (int i = lane; i < n; i += 32) {
-        const float di = S.dist[i];
-        int rank = 0;
-        for (int k = 0; k < n; ++k) rank += S.dist[k] < di || (S.dist[k] == di && S.slot[k] < S.slot[i]);
-        if (rank < kLocalTris) near_slot[rank] = S.slot[i];
-        if (rank == kLocalTris) L.h = local_half_edge(di, c);
+        const int rank = rank_of(S, n, i);
+        if (rank < kLocalTris) near_slot[rank] = S.near_slot[i];
+        if (rank == kLocalTris) L.h = local_half_edge(S.near_dist[i], c);
     }
     __syncwarp();
     const float half = L.h;
@@ -209,7 +253,7 @@ __global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ 
 }
 
 // At kDensityPoints triangle centroids spread over the scene: the nodes a point query
-// visits and the radius of a neighbourhood.
+// visits and the distance of the first triangle that a list there would not hold.
 constexpr int kDensityPoints = 128;
 
 __global__ void __launch_bounds__(32) k_density(const DNode *__restrict__ nodes, const DTri *__restrict__ tris,
@@ -221,9 +265,10 @@ __global__ void __launch_bounds__(32) k_density(const DNode *__restrict__ nodes,
     int visited;
     collect(S, nodes, tris, c, 0.f, visited);
     __syncwarp();
-    float h = guess;
-    const int n = float(visited) >= 0.5f * kDenseNodes ? find_radius(S, nodes, tris, c, h) : 0;
-    if (threadIdx.x == 0) out[blockIdx.x] = make_float2(float(visited), n > 0 ? h : 0.f);
+    const int n = float(visited) >= 0.5f * kDenseNodes ? find_nearest(S, nodes, tris, c, guess) : 0;
+    for (int i = threadIdx.x; i < n; i += 32)
+        if (rank_of(S, n, i) == kLocalTris) out[blockIdx.x] = make_float2(float(visited), S.near_dist[i]);
+    if (n == 0 && threadIdx.x == 0) out[blockIdx.x] = make_float2(float(visited), 0.f);
 }
 
 }  // namespace
@@ -261,9 +306,10 @@ int measure_density(SceneDev &s, cudaStream_t st, std::string &err) {
         visited += x.x / kDensityPoints;
         if (x.y > 0.f) radius.push_back(x.y);
     }
-    if (visited < kDenseNodes || radius.size() < kDensityPoints / 2) return 0;
+    if (visited < kDenseNodes || radius.size() < kDensityPoints / 4) return 0;
     std::nth_element(radius.begin(), radius.begin() + radius.size() / 2, radius.end());
-    s.local_radius = radius[radius.size() / 2];
+    // twice the usual distance: some 200 to 500 triangles in reach, a single search mostly
+    s.local_radius = 2.f * radius[radius.size() / 2];
     return 0;
 }
 

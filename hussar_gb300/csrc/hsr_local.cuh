@@ -22,7 +22,8 @@
 // 33 poses on 100 k triangles (reference phase) 17 -> 5.1 ms, 1999 short poses on 20 k
 // triangles 19.9 -> 12.8 ms (of which 10 on the host). With 32, 48, 64 and 96 triangles, one
 // plane each, the first of these took 28.5, 22.1, 19.3 and 20.5 ms; grouping by plane
-// took 64 to 17.1. The lists take one warp per pose and 0.22 ms before the launch.
+// took 64 to 17.1. The lists take one warp per pose and 0.13 ms before the launch. Served
+// mix (24 requests, two of three scenes dense) 31 -> 12 ms.
 #pragma once
 #include <math_constants.h>
 
@@ -35,40 +36,38 @@ namespace hsr {
 // Half the cube's edge where the nearest triangle that is not listed has its bounding box
 // at Chebyshev distance `next` from the centre: less a margin for the rounding of hit points
 // and of box corners formed from v0 + e.
-__host__ __device__ __forceinline__ float local_half_edge(float next, f3 c) {
+__device__ __forceinline__ float local_half_edge(float next, f3 c) {
     return next - 1e-5f * (next + fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)))) - 1e-6f;
 }
 
 // A triangle's plane relative to the centre, and the margin its test needs: tri_test's
 // distance comes from products of edges and of vertex differences with a few roundings
 // each, so in terms of the distance to the plane its error is at most some 2^-22 of the
-// lengths involved, magnified by how acute the triangle is. A degenerate triangle gets the
+// lengths involved, magnified by how acute the triangle is; so is the error of the plane
+// formed here in single precision. The margin is 2^-19 of them. A degenerate triangle gets the
 // plane 0 = 0, which is always tested. The normal's largest component is positive.
-__host__ __device__ __forceinline__ float4 local_plane(const DTri &T, f3 c, float h, float &eps) {
-    const double e1[3] = {T.e1.x, T.e1.y, T.e1.z}, e2[3] = {T.e2.x, T.e2.y, T.e2.z};
-    const double v[3] = {double(T.v0.x) - c.x, double(T.v0.y) - c.y, double(T.v0.z) - c.z};
-    double n[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]};
-    const double len = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    const double l1 = sqrt(e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
-    const double l2 = sqrt(e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
-    const double lv = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-    double big = n[0];
-    if (fabs(n[1]) > fabs(big)) big = n[1];
-    if (fabs(n[2]) > fabs(big)) big = n[2];
-    const double inv = len > 0.0 ? (big < 0.0 ? -1.0 : 1.0) / len : 0.0;
-    for (int a = 0; a < 3; ++a) n[a] *= inv;
-    const double acute = fmin(fmax(l1 * l2 * fabs(inv), 1.0), 1e6);
-    eps = float(2e-6 * (lv + l1 + l2 + double(h)) * acute);
-    return make_float4(float(n[0]), float(n[1]), float(n[2]), float(n[0] * v[0] + n[1] * v[1] + n[2] * v[2]));
+__device__ __forceinline__ float4 local_plane(const DTri &T, f3 c, float h, float &eps) {
+    const f3 e1 = mk3(T.e1.x, T.e1.y, T.e1.z), e2 = mk3(T.e2.x, T.e2.y, T.e2.z);
+    const f3 v = mk3(T.v0.x - c.x, T.v0.y - c.y, T.v0.z - c.z);
+    const f3 n = crs3(e1, e2);
+    const float len = nrm3(n), l1 = nrm3(e1), l2 = nrm3(e2);
+    float big = n.x;
+    if (fabsf(n.y) > fabsf(big)) big = n.y;
+    if (fabsf(n.z) > fabsf(big)) big = n.z;
+    const float inv = len > 0.f ? (big < 0.f ? -1.f : 1.f) / len : 0.f;
+    const f3 u = scl3(inv, n);
+    const float acute = fminf(fmaxf(l1 * l2 * fabsf(inv), 1.f), 1e6f);
+    eps = 2e-6f * (nrm3(v) + l1 + l2 + h) * acute;
+    return make_float4(u.x, u.y, u.z, dot3(u, v));
 }
 
 // Whether two planes share a group: they are apart by less than local_merge_margin anywhere
 // in the cube, which the pose's eps takes in.
-__host__ __device__ __forceinline__ bool local_same_plane(float4 a, float4 b, float h) {
+__device__ __forceinline__ bool local_same_plane(float4 a, float4 b, float h) {
     return fabsf(a.x - b.x) <= 1e-6f && fabsf(a.y - b.y) <= 1e-6f && fabsf(a.z - b.z) <= 1e-6f &&
            fabsf(a.w - b.w) <= 1e-6f * h;
 }
-__host__ __device__ __forceinline__ float local_merge_margin(float h) { return 4e-6f * h; }
+__device__ __forceinline__ float local_merge_margin(float h) { return 4e-6f * h; }
 
 // Whether a point lies in the list's cube.
 __device__ __forceinline__ bool local_holds(const LocalList &L, f3 p) {

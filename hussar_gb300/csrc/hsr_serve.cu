@@ -208,6 +208,7 @@ struct TickSlot {
     int64_t seq = -1;  // tick number
     unsigned char *h_in = nullptr, *d_in = nullptr;
     float *h_out = nullptr, *d_out = nullptr;
+    LocalList *d_local = nullptr;  // neighbourhood lists of the tick's poses
     unsigned *h_status = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<ReqPtr> members;                         // requests with a segment in the tick
@@ -313,6 +314,7 @@ hsr_server::~hsr_server() {
         if (t.h_status) cudaFreeHost(t.h_status);
         if (t.d_in) cudaFree(t.d_in);
         if (t.d_out) cudaFree(t.d_out);
+        if (t.d_local) cudaFree(t.d_local);
         if (t.ev0) cudaEventDestroy(t.ev0);
         if (t.ev1) cudaEventDestroy(t.ev1);
     }
@@ -431,6 +433,8 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
     bool coherent = true;
     // a tick whose requests share one scene, chirp and N runs the uniform kernel
     bool uniform = true;
+    // a scene of the tick gives its poses neighbourhood lists
+    bool dense = false;
     const ReqPtr *first = nullptr;
     int64_t out_off = 0;
     tile[0] = 0;
@@ -456,7 +460,8 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
             j.tris = q->scene->tris;
             j.rf = q->r.rf;
             j.samples = q->r.samples_per_chirp;
-            j.local_radius = 0.f;
+            j.local_radius = q->scene->local_radius;
+            dense = dense || j.local_radius > 0.f;
             j.acc_offset = q->arena_off / int64_t(sizeof(double));
             acc_row[P] = j.acc_offset;
             if (!first) {
@@ -570,6 +575,11 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
             p.acc_row = reinterpret_cast<const int64_t *>(t.d_in + layout.acc_row);
             p.field_on_hit = q0->scene->tuned.field_on_hit;
             p.coherent_order = q0->scene->tuned.coherent_order;
+        }
+        if (dense) {
+            if (launch_local_build(p, (*first)->scene->local_radius, t.d_local, stream) != 0)
+                e = cudaErrorLaunchFailure;
+            p.local = t.d_local;
         }
         auto it = blocks_cache.find(maxN);
         if (it == blocks_cache.end()) it = blocks_cache.emplace(maxN, wave_blocks_per_sm(maxN, true, guided)).first;
@@ -824,7 +834,8 @@ hsr_status hsr_server_create(const hsr_server_config *cfg, hsr_server **out) {
             return serve_fail(HSR_ERR_OUT_OF_MEMORY, "pinned host buffers for the tick slots");
         }
         if (!dev_alloc(&t.d_in, s->layout.bytes, err) ||
-            !dev_alloc(&t.d_out, sizeof(float) * size_t(s->out_floats_cap), err))
+            !dev_alloc(&t.d_out, sizeof(float) * size_t(s->out_floats_cap), err) ||
+            !dev_alloc(&t.d_local, sizeof(LocalList) * size_t(cfg->max_slots), err))
             return serve_fail(HSR_ERR_OUT_OF_MEMORY, err);
         if (cudaEventCreate(&t.ev0) != cudaSuccess || cudaEventCreate(&t.ev1) != cudaSuccess) {
             cudaGetLastError();
