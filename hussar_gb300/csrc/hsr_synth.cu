@@ -431,6 +431,9 @@ __global__ void k_synth_finalize(const float *__restrict__ c, int slices, int64_
     if (i >= int64_t(P) * N) return;
     const int p = int(i / N), m = int(i % N);
     float re = 0.f, im = 0.f;
+    // one thread adds a bin's slices in order; 16 of them in flight, as few poses mean many
+    // slices and few threads (96 poses x 256 bins: 80 -> 32 us)
+#pragma unroll 16
     for (int z = 0; z < slices; ++z) {
         re += c[size_t(z) * slice + size_t(p) * ldc + m];
         im += c[size_t(z) * slice + size_t(p) * ldc + N + m];
