@@ -465,8 +465,8 @@ __global__ void k_relink(int64_t n_nodes, DNode *nodes, const int32_t *__restric
 // never removed). The build's DNodes are written back only when the result passes its
 // checks (every node's parent chain ends at node 0; leaves at most 60 deep).
 constexpr int kReinsPath = 96;       // deepest parent chain a search handles
-constexpr int kReinsHeap = 384;      // search frontier (a fuller frontier drops entries)
-constexpr int kReinsPops = 4096;
+constexpr int kReinsStack = 96;      // a search's deferred subtrees
+constexpr int kReinsVisits = 8192;   // most subtrees it opens
 constexpr int kReinsMaxDepth = 60;   // the traversal stack holds 64 entries
 
 __device__ __forceinline__ Box box_union(const Box &a, const Box &b) {
@@ -479,8 +479,36 @@ __device__ __forceinline__ Box box_union(const Box &a, const Box &b) {
     return u;
 }
 
+// A node of the tree under optimisation: box and children (leaf: kx = -1), one sector.
+struct __align__(32) ReinsNode {
+    float lo[3];
+    int kx;
+    float hi[3];
+    int ky;
+};
+
+__device__ __forceinline__ ReinsNode reins_load(const ReinsNode *__restrict__ t, int i) {
+    const float4 *p = reinterpret_cast<const float4 *>(t + i);
+    const float4 a = __ldg(p), b = __ldg(p + 1);
+    return ReinsNode{{a.x, a.y, a.z}, __float_as_int(a.w), {b.x, b.y, b.z}, __float_as_int(b.w)};
+}
+
+__device__ __forceinline__ ReinsNode reins_node(const Box &b, int kx, int ky) {
+    return ReinsNode{{b.lo[0], b.lo[1], b.lo[2]}, kx, {b.hi[0], b.hi[1], b.hi[2]}, ky};
+}
+
+__device__ __forceinline__ Box box_of(const ReinsNode &n) {
+    Box b;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        b.lo[k] = n.lo[k];
+        b.hi[k] = n.hi[k];
+    }
+    return b;
+}
+
 __global__ void k_reins_init(int m, const DNode *__restrict__ nodes, const int32_t *__restrict__ par_i, int *rpar,
-                             int2 *rkid, Box *rbox) {
+                             ReinsNode *tree) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const DNode nd = nodes[i];
@@ -489,13 +517,12 @@ __global__ void k_reins_init(int m, const DNode *__restrict__ nodes, const int32
     for (int w = 0; w < 2; ++w) {
         k[w] = c[w] >= 0 ? c[w] : m + ~c[w];
         if (c[w] < 0) {
-            rbox[k[w]] = child_box(nd, w);
+            tree[k[w]] = reins_node(child_box(nd, w), -1, -1);
             rpar[k[w]] = i;
         }
     }
-    rkid[i] = make_int2(k[0], k[1]);
     rpar[i] = par_i[i];
-    rbox[i] = box_union(child_box(nd, 0), child_box(nd, 1));
+    tree[i] = reins_node(box_union(child_box(nd, 0), child_box(nd, 1)), k[0], k[1]);
 }
 
 // Depth of every node (the root 0) and the deepest leaf; bad: a parent chain that does not
@@ -515,10 +542,19 @@ __global__ void k_reins_depth(int total, int m, const int *__restrict__ rpar, in
 }
 
 // The best place for subtree n: mv_x[n] (-1: none lowers the cost by min_gain) and the
-// cost it saves, mv_gain[n].
-__global__ void __launch_bounds__(128) k_reins_search(int total, int m, const int *__restrict__ rpar,
-                                                      const int2 *__restrict__ rkid, const Box *__restrict__ rbox,
-                                                      const int *__restrict__ depth, float min_gain, int *mv_x,
+// cost it saves, mv_gain[n]. Taking n out removes its parent P and shrinks the ancestors
+// below the one, y, whose other child's subtree (or which itself) receives it; from y up
+// nothing changes. So the search climbs from n: `saved` is what the removal saves up to
+// here, and each subtree hanging off the path is searched depth first, the child that grows
+// less first, with the best place so far as the bound (Meister and Bittner 2018). An open
+// subtree is a node and the growth of its ancestors; it is left where even a new parent no
+// larger than n would not pay.
+// A best-first search of the same space from the root, with the removal's shrunk boxes and
+// a 384-entry heap in local memory (5.8 KB per thread), visited fewer nodes but took 2.4 ms
+// per pass on 250 k triangles; this one 0.39 (0.65 with the descent as a loop inside the
+// climb), to trees of the same node visits per ray (boxes 126, urban 18.6).
+__global__ void __launch_bounds__(128) k_reins_search(int total, const int *__restrict__ rpar,
+                                                      const ReinsNode *__restrict__ tree, float min_gain, int *mv_x,
                                                       float *mv_gain) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= total) return;
@@ -527,117 +563,112 @@ __global__ void __launch_bounds__(128) k_reins_search(int total, int m, const in
     if (P < 0) return;
     const int G = rpar[P];
     if (G < 0) return;
-    const int dp = depth[P];
-    if (dp >= kReinsPath) return;
-    const int2 pk = rkid[P];
-    const int S = pk.x == n ? pk.y : pk.x;
-    // the tree with n taken out: P disappears, S takes its place, P's ancestors shrink
-    int pnode[kReinsPath];
-    Box pbox[kReinsPath];
-    float drem = -box_area(rbox[P]);
-    Box cur = rbox[S];
-    int child = P;
-    for (int y = G, steps = 0; y >= 0; child = y, y = rpar[y], ++steps) {
-        const int dy = depth[y];
-        if (steps >= kReinsPath || dy < 0 || dy >= dp) return;  // an inconsistent snapshot: no move
-        const int2 yk = rkid[y];
-        const Box nb = box_union(cur, rbox[yk.x == child ? yk.y : yk.x]);
-        drem += box_area(nb) - box_area(rbox[y]);
-        pnode[dy] = y;
-        pbox[dy] = nb;
-        cur = nb;
-    }
-    const Box bn = rbox[n];
+    const Box bn = box_of(reins_load(tree, n));
     const float an = box_area(bn);
-    // best-first branch and bound over the detached tree; a node's key is the area its
-    // ancestors grow by when n goes below them (the induced cost). Only a place whose
-    // insertion cost is below -drem - min_gain saves more than min_gain: that is the
-    // starting bound, so a subtree already well placed ends its search at once.
-    float hk[kReinsHeap];
-    int hv[kReinsHeap];
-    int hs = 1;
-    hk[0] = 0.f;
-    hv[0] = 0;
-    float best = -drem - min_gain;
-    int bx = -1;
-    for (int pops = 0; hs > 0 && pops < kReinsPops; ++pops) {
-        const float ic0 = hk[0];
-        int x = hv[0];
-        --hs;
-        if (hs > 0) {  // sift the last entry down from the top
-            const float k = hk[hs];
-            const int v = hv[hs];
-            int i = 0;
-            while (true) {
-                int c = 2 * i + 1;
-                if (c >= hs) break;
-                if (c + 1 < hs && hk[c + 1] < hk[c]) ++c;
-                if (hk[c] >= k) break;
-                hk[i] = hk[c];
-                hv[i] = hv[c];
-                i = c;
-            }
-            hk[i] = k;
-            hv[i] = v;
-        }
-        if (ic0 + an >= best) break;
-        if (x == P) x = S;
-        const int dx = depth[x];
-        const Box bxx = (dx < dp && pnode[dx] == x) ? pbox[dx] : rbox[x];
-        const float au = box_area(box_union(bxx, bn));
-        if (x != S && x != 0 && ic0 + au < best) {
-            best = ic0 + au;
+    const ReinsNode pn = reins_load(tree, P);
+    const int S = pn.kx == n ? pn.ky : pn.kx;
+    float saved = box_area(box_of(pn)), best = min_gain;
+    int bx = -1, visits = 0;
+    int stack[kReinsStack];
+    float grown[kReinsStack];
+    int sp = 0;
+    // node x as a place under ancestors that grow by d; its own growth added to d tells
+    // whether its subtree is opened
+    auto consider = [&](int x, const ReinsNode &t, float &d) {
+        const Box b = box_of(t);
+        const float au = box_area(box_union(b, bn));
+        const float gain = saved - (d + au);
+        if (gain > best) {
+            best = gain;
             bx = x;
         }
-        const float ic = ic0 + au - box_area(bxx);
-        if (x < m && ic + an < best) {
-            const int2 xk = rkid[x];
-            for (int w = 0; w < 2; ++w) {
-                if (hs >= kReinsHeap) break;
-                int i = hs++;
-                while (i > 0 && hk[(i - 1) / 2] > ic) {
-                    hk[i] = hk[(i - 1) / 2];
-                    hv[i] = hv[(i - 1) / 2];
-                    i = (i - 1) / 2;
-                }
-                hk[i] = ic;
-                hv[i] = w ? xk.y : xk.x;
+        d += au - box_area(b);
+        return t.kx >= 0;
+    };
+    auto open = [&](int x, float d) {
+        if (sp < kReinsStack && saved - d - an > best) {
+            stack[sp] = x;
+            grown[sp++] = d;
+        }
+    };
+    const ReinsNode sn = reins_load(tree, S);
+    Box cur = box_of(sn);  // the path's box without n
+    if (sn.kx >= 0) open(S, saved - box_area(cur));  // below the sibling (beside it is where n is)
+    int child = P, y = G, steps = 0;
+    float saved_next = saved;  // `saved` once the open subtrees are done
+    // one loop for both kinds of step, so that a lane that climbs does not wait for one that
+    // descends
+    while (true) {
+        if (sp > 0 && visits < kReinsVisits) {
+            const int x = stack[--sp];
+            const float d = grown[sp];
+            if (!(saved - d - an > best)) continue;
+            ++visits;
+            const ReinsNode t = reins_load(tree, x);
+            const ReinsNode l = reins_load(tree, t.kx), r = reins_load(tree, t.ky);
+            float dl = d, dr = d;
+            const bool kl = consider(t.kx, l, dl), kr = consider(t.ky, r, dr);
+            if (dl < dr) {
+                if (kr) open(t.ky, dr);
+                if (kl) open(t.kx, dl);
+            } else {
+                if (kl) open(t.kx, dl);
+                if (kr) open(t.ky, dr);
+            }
+            continue;
+        }
+        sp = 0;
+        saved = saved_next;
+        if (steps > 0 && child != 0) {  // beside the ancestor passed last
+            const float gain = saved - box_area(box_union(cur, bn));
+            if (gain > best) {
+                best = gain;
+                bx = child;
             }
         }
+        if (y < 0) break;
+        if (++steps > kReinsPath) return;
+        const ReinsNode yn = reins_load(tree, y);
+        const int c = yn.kx == child ? yn.ky : yn.kx;
+        const ReinsNode cn = reins_load(tree, c);
+        float d = 0.f;
+        if (consider(c, cn, d)) open(c, d);
+        cur = box_union(cur, box_of(cn));
+        saved_next = saved + (box_area(box_of(yn)) - box_area(cur));
+        child = y;
+        y = rpar[y];
     }
-    const float gain = -(drem + best);
-    if (bx >= 0 && gain > min_gain) {  // bx >= 0 already means gain > min_gain, up to rounding
+    if (bx >= 0) {
         mv_x[n] = bx;
-        mv_gain[n] = gain;
+        mv_gain[n] = best;
     }
 }
 
 // The nodes a move rewires: n, P, S, G, X, X's parent.
-__device__ __forceinline__ void reins_touched(int n, int x, const int *rpar, const int2 *rkid, int *t) {
+__device__ __forceinline__ void reins_touched(int n, int x, const int *rpar, const ReinsNode *tree, int *t) {
     const int P = rpar[n];
-    const int2 pk = rkid[P];
     t[0] = n;
     t[1] = P;
-    t[2] = pk.x == n ? pk.y : pk.x;
+    t[2] = tree[P].kx == n ? tree[P].ky : tree[P].kx;
     t[3] = rpar[P];
     t[4] = x;
     t[5] = rpar[x];
 }
 
-__global__ void k_reins_lock(int total, const int *__restrict__ rpar, const int2 *__restrict__ rkid,
+__global__ void k_reins_lock(int total, const int *__restrict__ rpar, const ReinsNode *__restrict__ tree,
                              const int *__restrict__ mv_x, const float *__restrict__ mv_gain,
                              unsigned long long *lock) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= total || mv_x[n] < 0) return;
     int t[6];
-    reins_touched(n, mv_x[n], rpar, rkid, t);
+    reins_touched(n, mv_x[n], rpar, tree, t);
     for (int k = 0; k < 6; ++k)
         if (t[k] < 0 || t[k] >= total) return;
     const unsigned long long key = (static_cast<unsigned long long>(__float_as_uint(mv_gain[n])) << 32) | unsigned(n);
     for (int k = 0; k < 6; ++k) atomicMax(&lock[t[k]], key);
 }
 
-__global__ void k_reins_claim(int total, const int *__restrict__ rpar, const int2 *__restrict__ rkid,
+__global__ void k_reins_claim(int total, const int *__restrict__ rpar, const ReinsNode *__restrict__ tree,
                               const int *__restrict__ mv_x, const float *__restrict__ mv_gain,
                               const unsigned long long *__restrict__ lock, char *moving) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -645,7 +676,7 @@ __global__ void k_reins_claim(int total, const int *__restrict__ rpar, const int
     moving[n] = 0;
     if (mv_x[n] < 0) return;
     int t[6];
-    reins_touched(n, mv_x[n], rpar, rkid, t);
+    reins_touched(n, mv_x[n], rpar, tree, t);
     const unsigned long long key = (static_cast<unsigned long long>(__float_as_uint(mv_gain[n])) << 32) | unsigned(n);
     for (int k = 0; k < 6; ++k)
         if (t[k] < 0 || t[k] >= total || lock[t[k]] != key) return;
@@ -665,34 +696,37 @@ __global__ void k_reins_keep(int total, const int *__restrict__ rpar, const int 
     keep[n] = 1;
 }
 
-__global__ void k_reins_apply(int total, int *rpar, int2 *rkid, const int *__restrict__ mv_x,
+__global__ void k_reins_apply(int total, int *rpar, ReinsNode *tree, const int *__restrict__ mv_x,
                               const char *__restrict__ keep, int *applied) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= total || !keep[n]) return;
+    auto replace = [&](int parent, int from, int to) {
+        if (tree[parent].kx == from)
+            tree[parent].kx = to;
+        else
+            tree[parent].ky = to;
+    };
     const int X = mv_x[n];
     const int P = rpar[n], G = rpar[P];
-    const int2 pk = rkid[P];
-    const int S = pk.x == n ? pk.y : pk.x;
+    const int S = tree[P].kx == n ? tree[P].ky : tree[P].kx;
     // take n out: S replaces P below G
-    int2 gk = rkid[G];
-    if (gk.x == P) gk.x = S; else gk.y = S;
-    rkid[G] = gk;
+    replace(G, P, S);
     rpar[S] = G;
     // P becomes the parent of X and n, in X's place
     const int XP = rpar[X];
-    int2 xk = rkid[XP];
-    if (xk.x == X) xk.x = P; else xk.y = P;
-    rkid[XP] = xk;
+    replace(XP, X, P);
     rpar[P] = XP;
-    rkid[P] = make_int2(X, n);
+    tree[P].kx = X;
+    tree[P].ky = n;
     rpar[X] = P;
     rpar[n] = P;
     atomicAdd(applied, 1);
 }
 
 // Boxes from the leaves up: a leaf's thread climbs while it is the second child to arrive.
-__global__ void k_reins_refit(int total, int m, const int *__restrict__ rpar, const int2 *__restrict__ rkid,
-                              Box *rbox, int *counters, int *bad) {
+// A child's box comes from another SM: read and written in the L2.
+__global__ void k_reins_refit(int total, int m, const int *__restrict__ rpar, ReinsNode *tree, int *counters,
+                              int *bad) {
     const int leaf = m + blockIdx.x * blockDim.x + threadIdx.x;
     if (leaf >= total) return;
     int p = rpar[leaf];
@@ -704,36 +738,33 @@ __global__ void k_reins_refit(int total, int m, const int *__restrict__ rpar, co
         __threadfence();
         if (atomicAdd(&counters[p], 1) == 0) return;
         __threadfence();
-        const int2 k = rkid[p];
-        const volatile Box *vb = rbox;
-        Box a, b;
-        for (int j = 0; j < 3; ++j) {
-            a.lo[j] = vb[k.x].lo[j];
-            a.hi[j] = vb[k.x].hi[j];
-            b.lo[j] = vb[k.y].lo[j];
-            b.hi[j] = vb[k.y].hi[j];
-        }
-        rbox[p] = box_union(a, b);
+        float4 *t = reinterpret_cast<float4 *>(tree);
+        const float4 w0 = __ldcg(t + 2 * p), w1 = __ldcg(t + 2 * p + 1);
+        const int kx = __float_as_int(w0.w), ky = __float_as_int(w1.w);
+        const float4 a0 = __ldcg(t + 2 * kx), a1 = __ldcg(t + 2 * kx + 1);
+        const float4 b0 = __ldcg(t + 2 * ky), b1 = __ldcg(t + 2 * ky + 1);
+        __stcg(t + 2 * p, make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), w0.w));
+        __stcg(t + 2 * p + 1, make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), w1.w));
     }
 }
 
 // Back to the build's layout: DNodes with child boxes and references (leaf: ~slot),
 // internal and leaf parent links.
-__global__ void k_reins_write(int m, const int *__restrict__ rpar, const int2 *__restrict__ rkid,
-                              const Box *__restrict__ rbox, DNode *nodes, int32_t *par_i, int32_t *par_l) {
+__global__ void k_reins_write(int m, const int *__restrict__ rpar, const ReinsNode *__restrict__ tree, DNode *nodes,
+                              int32_t *par_i, int32_t *par_l) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    const int2 k = rkid[i];
-    const Box l = rbox[k.x], r = rbox[k.y];
+    const int kx = tree[i].kx, ky = tree[i].ky;
+    const Box l = box_of(tree[kx]), r = box_of(tree[ky]);
     DNode nd;
     nd.a = make_float4(l.lo[0], l.hi[0], l.lo[1], l.hi[1]);
     nd.b = make_float4(r.lo[0], r.hi[0], r.lo[1], r.hi[1]);
     nd.c = make_float4(l.lo[2], l.hi[2], r.lo[2], r.hi[2]);
-    nd.d = make_int4(k.x < m ? k.x : ~(k.x - m), k.y < m ? k.y : ~(k.y - m), 0, 0);
+    nd.d = make_int4(kx < m ? kx : ~(kx - m), ky < m ? ky : ~(ky - m), 0, 0);
     nodes[i] = nd;
     par_i[i] = rpar[i];
-    if (k.x >= m) par_l[k.x - m] = i;
-    if (k.y >= m) par_l[k.y - m] = i;
+    if (kx >= m) par_l[kx - m] = i;
+    if (ky >= m) par_l[ky - m] = i;
 }
 
 }  // namespace
@@ -751,8 +782,7 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
     if (g_bvh_optimize <= 0 || nt < 4 || nt >= (int64_t(1) << 30)) return 0;
     const int m = int(nt - 1), total = int(2 * nt - 1);
     int *rpar = nullptr, *depth = nullptr, *mv_x = nullptr, *counters = nullptr, *scal = nullptr;
-    int2 *rkid = nullptr;
-    Box *rbox = nullptr;
+    ReinsNode *tree = nullptr;
     float *mv_gain = nullptr;
     unsigned long long *lock = nullptr;
     char *moving = nullptr, *keep = nullptr;
@@ -760,18 +790,18 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
     do {
         if (!dev_alloc(&rpar, sizeof(int) * total, err) || !dev_alloc(&depth, sizeof(int) * total, err) ||
             !dev_alloc(&mv_x, sizeof(int) * total, err) || !dev_alloc(&counters, sizeof(int) * m, err) ||
-            !dev_alloc(&scal, sizeof(int) * 4, err) || !dev_alloc(&rkid, sizeof(int2) * m, err) ||
-            !dev_alloc(&rbox, sizeof(Box) * total, err) || !dev_alloc(&mv_gain, sizeof(float) * total, err) ||
+            !dev_alloc(&scal, sizeof(int) * 4, err) || !dev_alloc(&tree, sizeof(ReinsNode) * total, err) ||
+            !dev_alloc(&mv_gain, sizeof(float) * total, err) ||
             !dev_alloc(&lock, sizeof(unsigned long long) * total, err) || !dev_alloc(&moving, size_t(total), err) ||
             !dev_alloc(&keep, size_t(total), err)) {
             rc = 3;
             break;
         }
         const int T = 256;
-        k_reins_init<<<blocks_for(m, T), T, 0, st>>>(m, s.nodes, par_i, rpar, rkid, rbox);
+        k_reins_init<<<blocks_for(m, T), T, 0, st>>>(m, s.nodes, par_i, rpar, tree);
         note_launches(1);
-        Box root;
-        if (cudaMemcpyAsync(&root, rbox, sizeof(Box), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        ReinsNode root;
+        if (cudaMemcpyAsync(&root, tree, sizeof(root), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             err = "BVH optimisation: reading the root box failed";
             rc = 2;
@@ -785,13 +815,12 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
             cudaMemsetAsync(lock, 0, sizeof(unsigned long long) * total, st);
             cudaMemsetAsync(counters, 0, sizeof(int) * m, st);
             k_reins_depth<<<blocks_for(total, T), T, 0, st>>>(total, m, rpar, depth, scal + 2, scal + 1);
-            k_reins_search<<<blocks_for(total, 128), 128, 0, st>>>(total, m, rpar, rkid, rbox, depth, min_gain, mv_x,
-                                                                   mv_gain);
-            k_reins_lock<<<blocks_for(total, T), T, 0, st>>>(total, rpar, rkid, mv_x, mv_gain, lock);
-            k_reins_claim<<<blocks_for(total, T), T, 0, st>>>(total, rpar, rkid, mv_x, mv_gain, lock, moving);
+            k_reins_search<<<blocks_for(total, 128), 128, 0, st>>>(total, rpar, tree, min_gain, mv_x, mv_gain);
+            k_reins_lock<<<blocks_for(total, T), T, 0, st>>>(total, rpar, tree, mv_x, mv_gain, lock);
+            k_reins_claim<<<blocks_for(total, T), T, 0, st>>>(total, rpar, tree, mv_x, mv_gain, lock, moving);
             k_reins_keep<<<blocks_for(total, T), T, 0, st>>>(total, rpar, mv_x, moving, keep);
-            k_reins_apply<<<blocks_for(total, T), T, 0, st>>>(total, rpar, rkid, mv_x, keep, scal);
-            k_reins_refit<<<blocks_for(nt, T), T, 0, st>>>(total, m, rpar, rkid, rbox, counters, scal + 1);
+            k_reins_apply<<<blocks_for(total, T), T, 0, st>>>(total, rpar, tree, mv_x, keep, scal);
+            k_reins_refit<<<blocks_for(nt, T), T, 0, st>>>(total, m, rpar, tree, counters, scal + 1);
             note_launches(7);
             if (cudaMemcpyAsync(h, scal, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess) {
@@ -812,7 +841,7 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
             break;
         }
         if (h[1] || h[2] > kReinsMaxDepth) break;
-        k_reins_write<<<blocks_for(m, T), T, 0, st>>>(m, rpar, rkid, rbox, s.nodes, par_i, par_l);
+        k_reins_write<<<blocks_for(m, T), T, 0, st>>>(m, rpar, tree, s.nodes, par_i, par_l);
         note_launches(1);
         if (cudaStreamSynchronize(st) != cudaSuccess) {
             err = "BVH optimisation write-back failed";
@@ -824,8 +853,7 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
     cudaFree(mv_x);
     cudaFree(counters);
     cudaFree(scal);
-    cudaFree(rkid);
-    cudaFree(rbox);
+    cudaFree(tree);
     cudaFree(mv_gain);
     cudaFree(lock);
     cudaFree(moving);
@@ -984,51 +1012,104 @@ static int build_ploc(SceneDev &s, int64_t nt, const int32_t *ids2, const float 
     return rc;
 }
 
+namespace {
+
+// Nodes of every subtree, from the nodes with two leaves up: the second of two internal
+// children to arrive goes on. Climbs out of a collapsed leaf end where the parent no longer
+// refers to the node.
+__global__ void k_tree_sizes(int64_t n, const DNode *__restrict__ nodes, const int32_t *__restrict__ par_i, int *size,
+                             int *arrived) {
+    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (t >= n || nodes[t].d.x >= 0 || nodes[t].d.y >= 0) return;
+    int i = int(t), s = 1;
+    for (int steps = 0; steps < 1024; ++steps) {
+        __stcg(&size[i], s);
+        if (i == 0) return;
+        const int p = par_i[i];
+        if (p < 0) return;
+        const int4 d = nodes[p].d;
+        if (d.x != i && d.y != i) return;
+        if (d.x >= 0 && d.y >= 0) {
+            __threadfence();
+            if (atomicAdd(&arrived[p], 1) == 0) return;
+            __threadfence();
+        }
+        s = 1 + (d.x >= 0 ? __ldcg(&size[d.x]) : 0) + (d.y >= 0 ? __ldcg(&size[d.y]) : 0);
+        i = p;
+    }
+}
+
+// A reachable node's place in depth-first order: a first child follows its parent, a second
+// one its sibling's subtree; summed over the path to the root. placed: how many there were.
+__global__ void k_tree_place(int64_t n, const DNode *__restrict__ nodes, const int32_t *__restrict__ par_i,
+                             const int *__restrict__ size, int64_t out_count, DNode *__restrict__ out, int *placed) {
+    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (t >= n) return;
+    auto first = [&](const int4 &d) { return d.x >= 0 ? size[d.x] : 0; };
+    int64_t id = 0;
+    int c = int(t);
+    for (int steps = 0; c != 0; ++steps) {
+        const int p = par_i[c];
+        if (p < 0 || steps >= 1024) return;
+        const int4 d = nodes[p].d;
+        if (d.x == c)
+            id += 1;
+        else if (d.y == c)
+            id += 1 + first(d);
+        else
+            return;
+        c = p;
+    }
+    if (id >= out_count) return;
+    DNode nd = nodes[t];
+    const int skip = first(nd.d);
+    if (nd.d.x >= 0) nd.d.x = int(id) + 1;
+    if (nd.d.y >= 0) nd.d.y = int(id) + 1 + skip;
+    out[id] = nd;
+    atomicAdd(placed, 1);
+}
+
+}  // namespace
+
 // The reachable nodes renumbered in depth-first order from the root (each node's first
 // child follows it in memory, so a descent reads neighbouring nodes), the nodes inside
-// collapsed leaves dropped: the node array shrinks to the reachable nodes. On the host:
-// one download and one upload of the node array.
-static int renumber_depth_first(SceneDev &s, cudaStream_t st, std::string &err) {
+// collapsed leaves dropped: the node array shrinks to the reachable nodes. `counters` holds
+// one int per node. (The host's walk over a downloaded copy took 15 ms of the 49 of a
+// build of 250 k triangles.)
+static int renumber_depth_first(SceneDev &s, const int32_t *par_i, int *counters, cudaStream_t st, std::string &err) {
     const int64_t n = s.node_count;
     if (n < 2) return 0;
-    std::vector<DNode> h(static_cast<size_t>(n));
-    if (cudaMemcpyAsync(h.data(), s.nodes, sizeof(DNode) * h.size(), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
-        err = "BVH layout: node download failed";
-        return 2;
-    }
-    std::vector<int32_t> newid(static_cast<size_t>(n), -1), order, stack{0};
-    order.reserve(size_t(n));
-    while (!stack.empty()) {
-        const int32_t i = stack.back();
-        stack.pop_back();
-        if (i >= n || newid[i] >= 0 || int64_t(order.size()) >= n) {
-            err = "BVH layout: the tree is not a tree";
-            return 2;
-        }
-        newid[i] = int32_t(order.size());
-        order.push_back(i);
-        if (h[i].d.y >= 0) stack.push_back(h[i].d.y);
-        if (h[i].d.x >= 0) stack.push_back(h[i].d.x);
-    }
-    std::vector<DNode> out(order.size());
-    for (size_t k = 0; k < order.size(); ++k) {
-        DNode d = h[order[k]];
-        if (d.d.x >= 0) d.d.x = newid[d.d.x];
-        if (d.d.y >= 0) d.d.y = newid[d.d.y];
-        out[k] = d;
-    }
-    DNode *compact = nullptr;  // the array shrinks to the reachable nodes
-    if (!dev_alloc(&compact, sizeof(DNode) * out.size(), err)) return 3;
-    if (cudaMemcpyAsync(compact, out.data(), sizeof(DNode) * out.size(), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
+    int *size = nullptr;
+    DNode *compact = nullptr;
+    if (!dev_alloc(&size, sizeof(int) * size_t(n + 1), err)) return 3;
+    auto fail = [&](int rc, const char *what) {
+        if (rc == 2) err = what;
+        cudaFree(size);
         cudaFree(compact);
-        err = "BVH layout: node upload failed";
-        return 2;
-    }
+        return rc;
+    };
+    const int T = 256;
+    cudaMemsetAsync(counters, 0, sizeof(int) * size_t(n), st);
+    cudaMemsetAsync(size, 0, sizeof(int) * size_t(n + 1), st);
+    k_tree_sizes<<<blocks_for(n, T), T, 0, st>>>(n, s.nodes, par_i, size, counters);
+    note_launches(1);
+    int count = 0, placed = 0;
+    if (cudaMemcpyAsync(&count, size, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return fail(2, "BVH layout: subtree sizes failed");
+    if (count < 1 || count > n) return fail(2, "BVH layout: the tree is not a tree");
+    // the array shrinks to the reachable nodes
+    if (!dev_alloc(&compact, sizeof(DNode) * size_t(count), err)) return fail(3, "");
+    k_tree_place<<<blocks_for(n, T), T, 0, st>>>(n, s.nodes, par_i, size, count, compact, size + n);
+    note_launches(1);
+    if (cudaMemcpyAsync(&placed, size + n, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return fail(2, "BVH layout failed");
+    if (placed != count) return fail(2, "BVH layout: the tree is not a tree");
+    cudaFree(size);
     cudaFree(s.nodes);
     s.nodes = compact;
-    s.node_count = int64_t(out.size());
+    s.node_count = count;
     return 0;
 }
 
@@ -1173,7 +1254,7 @@ int bvh_build(SceneDev &s, const float *d_v, int64_t nv, const int32_t *d_idx, i
             fail(lrc);
             break;
         }
-        const int drc = renumber_depth_first(s, st, err);
+        const int drc = renumber_depth_first(s, par_i, counters, st, err);
         if (drc) {
             fail(drc);
             break;
