@@ -71,12 +71,12 @@ struct Scratch {
     int64_t *budget, *offset, *tile_start;
     float *weights;
     int *train, *active, *clear;
-    double *tw;
     double *acc;
     double *fine;  // fine-histogram rows (HSR_SPLAT_FINE_SYNTH), P x kFineRowPerBin N FP64 sums
     float *rows;
     LocalList *local;    // neighbourhood lists (dense scenes)
     unsigned *counters;  // [0] status word, [2..3] 64-bit work counter
+    bool fresh = false;  // the next pass clears the status word
     size_t bytes;
 };
 
@@ -91,31 +91,31 @@ static Scratch carve(void *base, int32_t P, int32_t N, bool fine, bool local) {
         off += align256(bytes);
         return r;
     };
+    // status word and rows together (one download), then what a call uploads together
     s.counters = reinterpret_cast<unsigned *>(take(64));
+    s.rows = reinterpret_cast<float *>(take(sizeof(float) * 2 * size_t(P) * N));
     s.tx = reinterpret_cast<hsr_antenna *>(take(sizeof(hsr_antenna) * P));
     s.rx = reinterpret_cast<hsr_antenna *>(take(sizeof(hsr_antenna) * P));
-    s.ff_tx = reinterpret_cast<hsr_ff_antenna *>(take(sizeof(hsr_ff_antenna) * P));
-    s.ff_rx = reinterpret_cast<hsr_ff_antenna *>(take(sizeof(hsr_ff_antenna) * P));
     s.budget = reinterpret_cast<int64_t *>(take(sizeof(int64_t) * P));
     s.offset = reinterpret_cast<int64_t *>(take(sizeof(int64_t) * P));
+    s.ff_tx = reinterpret_cast<hsr_ff_antenna *>(take(sizeof(hsr_ff_antenna) * P));
+    s.ff_rx = reinterpret_cast<hsr_ff_antenna *>(take(sizeof(hsr_ff_antenna) * P));
     s.tile_start = reinterpret_cast<int64_t *>(take(sizeof(int64_t) * (P + 1)));
     s.weights = reinterpret_cast<float *>(take(sizeof(float) * P));
     s.train = reinterpret_cast<int *>(take(sizeof(int) * P));
     s.active = reinterpret_cast<int *>(take(sizeof(int) * P));
     s.clear = reinterpret_cast<int *>(take(sizeof(int) * P));
-    s.tw = reinterpret_cast<double *>(take(sizeof(double) * P));
     s.acc = reinterpret_cast<double *>(take(sizeof(double) * 2 * size_t(P) * N));
     s.fine = fine ? reinterpret_cast<double *>(take(sizeof(double) * kFineRowPerBin * size_t(P) * N)) : nullptr;
-    s.rows = reinterpret_cast<float *>(take(sizeof(float) * 2 * size_t(P) * N));
     s.local = local ? reinterpret_cast<LocalList *>(take(sizeof(LocalList) * size_t(P))) : nullptr;
     s.bytes = off;
     return s;
 }
 
-// Carves the scene's scratch for P poses with N bins (growing it when needed) and clears
-// the status word on `st`: every call reports the device status of its own work only.
-static hsr_status ensure_scratch(SceneDev &sc, int32_t P, int32_t N, Scratch &out, cudaStream_t st,
-                                 bool fine = false) {
+// Carves the scene's scratch for P poses with N bins (growing it when needed). The call's
+// first pass clears the status word: every call reports the device status of its own work
+// only.
+static hsr_status ensure_scratch(SceneDev &sc, int32_t P, int32_t N, Scratch &out, bool fine = false) {
     const bool local = sc.local_radius > 0.f;
     Scratch need = carve(nullptr, P, N, fine, local);
     if (need.bytes > sc.scratch_bytes) {
@@ -133,8 +133,7 @@ static hsr_status ensure_scratch(SceneDev &sc, int32_t P, int32_t N, Scratch &ou
         sc.scratch_bytes = need.bytes;
     }
     out = carve(sc.scratch, P, N, fine, local);
-    cudaError_t e = cudaMemsetAsync(out.counters, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return cuda_fail(e, "status clear");
+    out.fresh = true;
     return HSR_OK;
 }
 
@@ -191,20 +190,34 @@ static hsr_status ensure_guide(SceneDev &sc, int P, GuideMem &out) {
 
 static constexpr int32_t kTile = 4096;  // most samples a CTA takes at once
 
+// The accumulator rows a pass starts from zero: none, all (poses null), or those flagged.
+struct PassClear {
+    double *rows = nullptr;
+    const int *poses = nullptr;
+};
+
 // One trace launch over the poses' current budgets/offsets/weights in scratch.
 // The autotuned tile, CTAs per SM and queue threshold apply to plain passes.
 static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_config *rf, int32_t N,
                                const hsr_tracer_flags *fl, int32_t P, float sample_weight, bool per_pose_weights,
                                int32_t phase_mode, int32_t splat_mode, cudaStream_t st, const GuideMem *g,
-                               void *records = nullptr, int max_rec = 0, unsigned long long *counters = nullptr) {
+                               const PassClear &clr, void *records = nullptr, int max_rec = 0,
+                               unsigned long long *counters = nullptr) {
     const bool wave = g_path_kernel == 0 && fl->useGeometricalOptics && !records && !counters;
     const bool tuned = !fl->doGuiding;
     const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile : kTile;
     const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(s.counters + 2, 0, 8, st)) != cudaSuccess) return cuda_fail(e, "memset counter");
-    if (launch_tile_prefix(s.budget, P, items.samples, s.tile_start, st) != 0)
-        return cuda_fail(cudaGetLastError(), "tile prefix launch");
+    PrepareParams q{};
+    q.budget = s.budget;
+    q.pose_count = P;
+    q.tile = items.samples;
+    q.tile_start = s.tile_start;
+    q.work_counter = reinterpret_cast<unsigned long long *>(s.counters + 2);
+    q.status = s.fresh ? s.counters : nullptr;
+    q.rows = clr.rows;
+    q.row_len = 2 * int64_t(N);
+    q.clear = clr.poses;
+    if (launch_prepare(q, st) != 0) return cuda_fail(cudaGetLastError(), "pass set-up launch");
     TraceParams p{};
     p.nodes = sc.nodes;
     p.tris = sc.tris;
@@ -287,13 +300,11 @@ static hsr_status run_plain(SceneDev &sc, const Scratch &s, const hsr_rf_config 
         if (r != HSR_OK) return r;
         if ((e = cudaMemsetAsync(s.fine, 0, sizeof(double) * kFineRowPerBin * size_t(P) * N, st)) != cudaSuccess)
             return cuda_fail(e, "memset fine histogram");
-    } else if ((e = cudaMemsetAsync(s.acc, 0, sizeof(double) * 2 * size_t(P) * N, st)) != cudaSuccess) {
-        return cuda_fail(e, "memset accumulators");
     }
     hsr_tracer_flags plain = *fl;
     plain.doGuiding = 0;
     hsr_status r = enqueue_pass(sc, s, rf, N, &plain, P, sample_weight, false, phase_mode, splat_mode, st, nullptr,
-                                records, max_rec, counters);
+                                PassClear{fine ? nullptr : s.acc, nullptr}, records, max_rec, counters);
     if (r != HSR_OK) return r;
     if (fine) return synthesise(sc, s, P, sample_weight, nullptr, normalise, d_out_rows, st);
     if (launch_finalize(s.acc, P, N, s.budget, sample_weight, nullptr, normalise, d_out_rows, st) != 0)
@@ -351,15 +362,13 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
         if (r != HSR_OK) return r;
         if ((e = cudaMemsetAsync(s.fine, 0, sizeof(double) * kFineRowPerBin * size_t(P) * N, st)) != cudaSuccess)
             return cuda_fail(e, "memset fine histogram");
-    } else if ((e = cudaMemsetAsync(s.acc, 0, sizeof(double) * 2 * size_t(P) * N, st)) != cudaSuccess) {
-        return cuda_fail(e, "memset accumulators");
     }
     if (launch_guide_reset(P, g.samp_child, g.samp_p, g.train_child, g.train_acc, g.train_count, st) != 0)
         return cuda_fail(cudaGetLastError(), "guide reset");
     if (K > size_t(kGuideMaxIters)) return fail(HSR_ERR_INVALID_ARGUMENT, "guided budget needs too many iterations");
     // every iteration's schedule, uploaded once: the iterations then run back to back
     const size_t it_bytes = 32 * size_t(P);
-    std::vector<unsigned char> blk(K * it_bytes);
+    std::vector<unsigned char> blk(K * it_bytes + 8 * size_t(P));
     std::vector<double> tw(P, 0.0);
     std::vector<char> any_clear(K, 0), any_active(K, 0);
     for (size_t k = 0; k < K; ++k) {
@@ -392,6 +401,8 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
             any_active[k] |= active[p] != 0;
         }
     }
+    std::memcpy(blk.data() + K * it_bytes, tw.data(), 8 * size_t(P));
+    const double *d_tw = reinterpret_cast<const double *>(g.sched + K * it_bytes);
     if ((e = cudaMemcpyAsync(g.sched, blk.data(), blk.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return cuda_fail(e, "schedule upload");
     for (size_t k = 0; k < K; ++k) {
@@ -409,26 +420,26 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
         si.train = reinterpret_cast<int *>(si.weights + P);
         si.clear = si.train + P;
         si.active = si.clear + P;
-        if (any_clear[k]) {
-            const int rc = fine ? launch_clear_rows_f(s.fine, P, kFineRowPerBin * N, si.clear, st)
-                                : launch_clear_rows(s.acc, P, N, si.clear, st);
-            if (rc != 0) return cuda_fail(cudaGetLastError(), "clear rows");
+        si.fresh = s.fresh && k == 0;
+        PassClear clr;
+        if (fine) {
+            if (any_clear[k] && launch_clear_rows_f(s.fine, P, kFineRowPerBin * N, si.clear, st) != 0)
+                return cuda_fail(cudaGetLastError(), "clear rows");
+        } else if (k == 0 || any_clear[k]) {
+            clr = PassClear{s.acc, k == 0 ? nullptr : si.clear};
         }
-        r = enqueue_pass(sc, si, rf, N, fl, P, 1.f, true, phase_mode, splat_mode, st, &g);
+        r = enqueue_pass(sc, si, rf, N, fl, P, 1.f, true, phase_mode, splat_mode, st, &g, clr);
         if (r != HSR_OK) return r;
         if (any_active[k] &&
             launch_guide_step(P, si.active, g.samp_child, g.samp_p, g.train_child, g.train_acc, g.train_count, st) != 0)
             return cuda_fail(cudaGetLastError(), "guide step");
     }
-    if ((e = cudaMemcpyAsync(s.tw, tw.data(), 8 * P, cudaMemcpyHostToDevice, st)) != cudaSuccess)
-        return cuda_fail(e, "weight upload");
     if (fine) {
-        r = synthesise(sc, s, P, 1.f, s.tw, normalise, d_out_rows, st);
+        r = synthesise(sc, s, P, 1.f, d_tw, normalise, d_out_rows, st);
         if (r != HSR_OK) return r;
-    } else if (launch_finalize(s.acc, P, N, s.budget, 1.f, s.tw, normalise, d_out_rows, st) != 0) {
+    } else if (launch_finalize(s.acc, P, N, s.budget, 1.f, d_tw, normalise, d_out_rows, st) != 0) {
         return cuda_fail(cudaGetLastError(), "finalize launch");
     }
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "guided finalize");
     if (h_total_weight)
         for (int p = 0; p < P; ++p) h_total_weight[p] = tw[p];
     return HSR_OK;
@@ -457,15 +468,66 @@ static hsr_status read_status(const Scratch &s, cudaStream_t st) {
     return HSR_OK;
 }
 
-static hsr_status upload_poses(const Scratch &s, int32_t P, const hsr_antenna *tx, const hsr_antenna *rx,
-                               const int64_t *budget, const int64_t *offset, cudaMemcpyKind kind, cudaStream_t st) {
+// A host call's poses, budgets and offsets in one upload (tx .. offset, or budget .. ff_rx
+// for far-field antennas, lie together in the scratch). The copy has left the staging
+// block when it returns (pageable memory).
+static hsr_status upload_block(SceneDev &sc, char *first, char *last,
+                               std::initializer_list<std::pair<void *, std::pair<const void *, size_t>>> parts,
+                               cudaStream_t st) {
+    const size_t bytes = size_t(last - first);
+    if (sc.stage.size() < bytes) sc.stage.resize(bytes);
+    for (const auto &p : parts)
+        std::memcpy(sc.stage.data() + (static_cast<char *>(p.first) - first), p.second.first, p.second.second);
+    const cudaError_t e = cudaMemcpyAsync(first, sc.stage.data(), bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? HSR_OK : cuda_fail(e, "pose upload");
+}
+
+static hsr_status upload_poses(SceneDev &sc, const Scratch &s, int32_t P, const hsr_antenna *tx, const hsr_antenna *rx,
+                               const int64_t *budget, const int64_t *offset, cudaStream_t st) {
+    const size_t a = sizeof(hsr_antenna) * size_t(P), n = sizeof(int64_t) * size_t(P);
+    return upload_block(sc, reinterpret_cast<char *>(s.tx), reinterpret_cast<char *>(s.offset) + n,
+                        {{s.tx, {tx, a}}, {s.rx, {rx, a}}, {s.budget, {budget, n}}, {s.offset, {offset, n}}}, st);
+}
+
+static hsr_status upload_poses_ff(SceneDev &sc, const Scratch &s, int32_t P, const hsr_ff_antenna *tx,
+                                  const hsr_ff_antenna *rx, const int64_t *budget, const int64_t *offset,
+                                  cudaStream_t st) {
+    const size_t a = sizeof(hsr_ff_antenna) * size_t(P), n = sizeof(int64_t) * size_t(P);
+    return upload_block(sc, reinterpret_cast<char *>(s.budget), reinterpret_cast<char *>(s.ff_rx) + a,
+                        {{s.budget, {budget, n}}, {s.offset, {offset, n}}, {s.ff_tx, {tx, a}}, {s.ff_rx, {rx, a}}}, st);
+}
+
+// Poses that are on the device already are read where they are.
+static void use_device_poses(Scratch &s, const hsr_antenna *tx, const hsr_antenna *rx, const int64_t *budget,
+                             const int64_t *offset) {
+    s.tx = const_cast<hsr_antenna *>(tx);
+    s.rx = const_cast<hsr_antenna *>(rx);
+    s.budget = const_cast<int64_t *>(budget);
+    s.offset = const_cast<int64_t *>(offset);
+}
+
+// Ends a host call: `floats` of the rows (or of `src`) to the host, then the status. Small
+// rows come with the status word before them in one download.
+static hsr_status fetch_rows(const Scratch &s, float *out, size_t floats, cudaStream_t st,
+                             const float *src = nullptr) {
+    constexpr size_t kTogether = 256 << 10;
+    const size_t bytes = sizeof(float) * floats;
     cudaError_t e;
-    if ((e = cudaMemcpyAsync(s.tx, tx, sizeof(hsr_antenna) * P, kind, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(s.rx, rx, sizeof(hsr_antenna) * P, kind, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(s.budget, budget, sizeof(int64_t) * P, kind, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(s.offset, offset, sizeof(int64_t) * P, kind, st)) != cudaSuccess)
-        return cuda_fail(e, "pose upload");
-    return HSR_OK;
+    if (!src && bytes <= kTogether) {
+        const size_t head = size_t(reinterpret_cast<char *>(s.rows) - reinterpret_cast<char *>(s.counters));
+        std::vector<char> host(head + bytes);
+        if ((e = cudaMemcpyAsync(host.data(), s.counters, head + bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(st)) != cudaSuccess)
+            return cuda_fail(e, "row download");
+        unsigned bits;
+        std::memcpy(&bits, host.data(), sizeof(bits));
+        std::memcpy(out, host.data() + head, bytes);
+        return bits ? fail(HSR_ERR_DEVICE, status_text(bits)) : HSR_OK;
+    }
+    if ((e = cudaMemcpyAsync(out, src ? src : s.rows, bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+        return cuda_fail(e, "row download");
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "run");
+    return read_status(s, st);
 }
 
 }  // namespace hsr
@@ -803,7 +865,7 @@ hsr_status hsr_debug_records(hsr_scene *s, const hsr_rf_config *rf, int32_t samp
         return fail(HSR_ERR_INVALID_ARGUMENT, "bad record request");
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
-    if ((st = ensure_scratch(s->dev, 1, samples, sc, 0)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, 1, samples, sc)) != HSR_OK) return st;
     const size_t rec_bytes = size_t(budget) * max_rec * 36;
     void *d_rec = nullptr;
     std::string err;
@@ -811,7 +873,7 @@ hsr_status hsr_debug_records(hsr_scene *s, const hsr_rf_config *rf, int32_t samp
     std::vector<int32_t> init(rec_bytes / 4, 0);  // unused slots: depth = -1
     for (size_t i = 0; i < init.size(); i += 9) init[i] = -1;
     cudaMemcpy(d_rec, init.data(), rec_bytes, cudaMemcpyHostToDevice);
-    if ((st = upload_poses(sc, 1, tx, rx, &budget, &index_offset, cudaMemcpyHostToDevice, 0)) != HSR_OK) {
+    if ((st = upload_poses(s->dev, sc, 1, tx, rx, &budget, &index_offset, 0)) != HSR_OK) {
         cudaFree(d_rec);
         return st;
     }
@@ -849,17 +911,12 @@ hsr_status hsr_backend_run(const hsr_scene *cs, const hsr_rf_config *rf, const h
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = 0;
-    if ((st = ensure_scratch(s->dev, 1, N, sc, strm)) != HSR_OK) return st;
-    if ((st = upload_poses(sc, 1, tx, rx, &budget, &index_offset, cudaMemcpyHostToDevice, strm)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, 1, N, sc)) != HSR_OK) return st;
+    if ((st = upload_poses(s->dev, sc, 1, tx, rx, &budget, &index_offset, strm)) != HSR_OK) return st;
     st = run_plain(s->dev, sc, rf, N, fl, 1, sample_weight, phase_mode, HSR_SPLAT_DIRICHLET16, 0, sc.rows, strm);
     if (st != HSR_OK) return st;
     std::vector<float> row(2 * size_t(N));
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(row.data(), sc.rows, sizeof(float) * 2 * N, cudaMemcpyDeviceToHost, strm)) !=
-        cudaSuccess)
-        return cuda_fail(e, "row download");
-    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "backend run");
-    if ((st = read_status(sc, strm)) != HSR_OK) return st;
+    if ((st = fetch_rows(sc, row.data(), row.size(), strm)) != HSR_OK) return st;
     // the reference writes only chirp 0 / channel 0 (path.h:130, 291-292)
     const int C = frame->channelCount;
     for (int32_t k = 0; k < N; ++k) {
@@ -1001,26 +1058,20 @@ hsr_status hsr_backend_run_guided(hsr_scene *s, const hsr_rf_config *rf, const h
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = 0;
-    if ((st = ensure_scratch(s->dev, 1, N, sc, strm)) != HSR_OK) return st;
-    if ((st = upload_poses(sc, 1, tx, rx, &budget, &index_offset, cudaMemcpyHostToDevice, strm)) != HSR_OK) return st;
-    cudaError_t e;
+    if ((st = ensure_scratch(s->dev, 1, N, sc)) != HSR_OK) return st;
+    if ((st = upload_poses(s->dev, sc, 1, tx, rx, &budget, &index_offset, strm)) != HSR_OK) return st;
     const int tr = train ? 1 : 0;
-    if ((e = cudaMemcpyAsync(sc.train, &tr, sizeof(int), cudaMemcpyHostToDevice, strm)) != cudaSuccess ||
-        (e = cudaMemsetAsync(sc.acc, 0, sizeof(double) * 2 * size_t(N), strm)) != cudaSuccess)
-        return cuda_fail(e, "guided run set-up");
+    const cudaError_t e = cudaMemcpyAsync(sc.train, &tr, sizeof(int), cudaMemcpyHostToDevice, strm);
+    if (e != cudaSuccess) return cuda_fail(e, "guided run set-up");
     hsr_tracer_flags g = *fl;
     g.doGuiding = 1;
     if ((st = enqueue_pass(s->dev, sc, rf, N, &g, 1, sample_weight, false, phase_mode, HSR_SPLAT_DIRICHLET16, strm,
-                           &guide->g)) != HSR_OK)
+                           &guide->g, PassClear{sc.acc, nullptr})) != HSR_OK)
         return st;
     if (launch_finalize(sc.acc, 1, N, sc.budget, sample_weight, nullptr, 0, sc.rows, strm) != 0)
         return cuda_fail(cudaGetLastError(), "finalize launch");
     std::vector<float> row(2 * size_t(N));
-    if ((e = cudaMemcpyAsync(row.data(), sc.rows, sizeof(float) * 2 * N, cudaMemcpyDeviceToHost, strm)) !=
-        cudaSuccess)
-        return cuda_fail(e, "row download");
-    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "guided backend run");
-    if ((st = read_status(sc, strm)) != HSR_OK) return st;
+    if ((st = fetch_rows(sc, row.data(), row.size(), strm)) != HSR_OK) return st;
     const int C = frame->channelCount;
     for (int32_t k = 0; k < N; ++k) {
         size_t id = size_t(k) * C;
@@ -1057,20 +1108,15 @@ hsr_status hsr_path_tracer_run(hsr_scene *s, const hsr_rf_config *rf, const hsr_
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = 0;
-    if ((st = ensure_scratch(s->dev, 1, N, sc, strm)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, 1, N, sc)) != HSR_OK) return st;
     int64_t zero = 0;
-    if ((st = upload_poses(sc, 1, tx, rx, &samples, &zero, cudaMemcpyHostToDevice, strm)) != HSR_OK) return st;
+    if ((st = upload_poses(s->dev, sc, 1, tx, rx, &samples, &zero, strm)) != HSR_OK) return st;
     double tw = 0.0;
     st = run_guided(s->dev, sc, rf, N, fl, 1, std::vector<int64_t>{samples}, std::vector<int64_t>{0}, phase_mode,
                     HSR_SPLAT_DIRICHLET16, 0, sc.rows, strm, &tw, interrupt_flag);
     if (st != HSR_OK) return st;
     std::vector<float> row(2 * size_t(N));
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(row.data(), sc.rows, sizeof(float) * 2 * N, cudaMemcpyDeviceToHost, strm)) !=
-        cudaSuccess)
-        return cuda_fail(e, "row download");
-    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "guided run");
-    if ((st = read_status(sc, strm)) != HSR_OK) return st;
+    if ((st = fetch_rows(sc, row.data(), row.size(), strm)) != HSR_OK) return st;
     const int C = frame->channelCount;
     for (int32_t k = 0; k < N; ++k) {
         size_t id = size_t(k) * C;
@@ -1093,9 +1139,8 @@ hsr_status hsr_simulate_batch_device(hsr_scene *s, const hsr_rf_config *rf, int3
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
-    if ((st = ensure_scratch(s->dev, P, N, sc, strm, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
-    if ((st = upload_poses(sc, P, d_tx, d_rx, d_budget, d_offset, cudaMemcpyDeviceToDevice, strm)) != HSR_OK)
-        return st;
+    if ((st = ensure_scratch(s->dev, P, N, sc, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
+    use_device_poses(sc, d_tx, d_rx, d_budget, d_offset);
     if (!fl->doGuiding)
         return run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, d_out_rows, strm);
     // the guided schedule is planned on the host: it reads the budgets back (synchronising)
@@ -1105,7 +1150,9 @@ hsr_status hsr_simulate_batch_device(hsr_scene *s, const hsr_rf_config *rf, int3
         (e = cudaMemcpyAsync(o.data(), d_offset, 8 * P, cudaMemcpyDeviceToHost, strm)) != cudaSuccess ||
         (e = cudaStreamSynchronize(strm)) != cudaSuccess)
         return cuda_fail(e, "budget read-back");
-    return run_guided(s->dev, sc, rf, N, fl, P, b, o, phase_mode, splat_mode, 1, d_out_rows, strm, nullptr, nullptr);
+    st = run_guided(s->dev, sc, rf, N, fl, P, b, o, phase_mode, splat_mode, 1, d_out_rows, strm, nullptr, nullptr);
+    if (st == HSR_OK && (e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "guided batch");
+    return st;
 }
 
 hsr_status hsr_simulate_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, const hsr_tracer_flags *fl, int32_t P,
@@ -1122,8 +1169,8 @@ hsr_status hsr_simulate_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
-    if ((st = ensure_scratch(s->dev, P, N, sc, strm, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
-    if ((st = upload_poses(sc, P, tx, rx, budget, offset, cudaMemcpyHostToDevice, strm)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, P, N, sc, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
+    if ((st = upload_poses(s->dev, sc, P, tx, rx, budget, offset, strm)) != HSR_OK) return st;
     if (!fl->doGuiding) {
         st = run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, sc.rows, strm);
     } else {
@@ -1132,12 +1179,7 @@ hsr_status hsr_simulate_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
                         nullptr);
     }
     if (st != HSR_OK) return st;
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(out_rows, sc.rows, sizeof(float) * 2 * size_t(P) * N, cudaMemcpyDeviceToHost, strm)) !=
-        cudaSuccess)
-        return cuda_fail(e, "row download");
-    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "batch run");
-    return read_status(sc, strm);
+    return fetch_rows(sc, out_rows, 2 * size_t(P) * N, strm);
 }
 
 hsr_status hsr_simulate_frame(hsr_scene *s, const hsr_rf_config *rf, const hsr_frame_config *frame,
@@ -1163,7 +1205,7 @@ hsr_status hsr_simulate_frame(hsr_scene *s, const hsr_rf_config *rf, const hsr_f
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
-    if ((st = ensure_scratch(s->dev, C, N, sc, strm, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, C, N, sc, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
     const size_t bytes = sizeof(float) * 2 * size_t(frame->chirpCount) * N * C;
     if (bytes > s->dev.frame_bytes) {
         cudaStreamSynchronize(strm);
@@ -1174,9 +1216,7 @@ hsr_status hsr_simulate_frame(hsr_scene *s, const hsr_rf_config *rf, const hsr_f
         if (!dev_alloc(&s->dev.frame_buf, bytes, err)) return fail(HSR_ERR_OUT_OF_MEMORY, "frame buffer: " + err);
         s->dev.frame_bytes = bytes;
     }
-    if ((st = upload_poses(sc, C, ctx.data(), crx.data(), b.data(), o.data(), cudaMemcpyHostToDevice, strm)) !=
-        HSR_OK)
-        return st;
+    if ((st = upload_poses(s->dev, sc, C, ctx.data(), crx.data(), b.data(), o.data(), strm)) != HSR_OK) return st;
     st = fl->doGuiding ? run_guided(s->dev, sc, rf, N, fl, C, b, o, phase_mode, splat_mode, 1, sc.rows, strm,
                                     nullptr, nullptr)
                        : run_plain(s->dev, sc, rf, N, fl, C, 1.f, phase_mode, splat_mode, 1, sc.rows, strm);
@@ -1184,11 +1224,7 @@ hsr_status hsr_simulate_frame(hsr_scene *s, const hsr_rf_config *rf, const hsr_f
     float *d_frame = static_cast<float *>(s->dev.frame_buf);
     if (launch_assemble_frame(sc.rows, frame->chirpCount, N, C, d_frame, strm) != 0)
         return cuda_fail(cudaGetLastError(), "frame assembly");
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(frame_out, d_frame, bytes, cudaMemcpyDeviceToHost, strm)) != cudaSuccess)
-        return cuda_fail(e, "frame download");
-    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "frame simulation");
-    return read_status(sc, strm);
+    return fetch_rows(sc, frame_out, bytes / sizeof(float), strm, d_frame);
 }
 
 hsr_status hsr_simulate_batch_ff(hsr_scene *s, const hsr_rf_config *rf, int32_t N, const hsr_tracer_flags *fl,
@@ -1208,21 +1244,12 @@ hsr_status hsr_simulate_batch_ff(hsr_scene *s, const hsr_rf_config *rf, int32_t 
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
     cudaStream_t strm = nullptr;
-    if ((st = ensure_scratch(s->dev, P, N, sc, strm)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, P, N, sc)) != HSR_OK) return st;
     sc.far_field = true;
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(sc.ff_tx, tx, sizeof(hsr_ff_antenna) * P, cudaMemcpyHostToDevice, strm)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(sc.ff_rx, rx, sizeof(hsr_ff_antenna) * P, cudaMemcpyHostToDevice, strm)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(sc.budget, budget, sizeof(int64_t) * P, cudaMemcpyHostToDevice, strm)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(sc.offset, offset, sizeof(int64_t) * P, cudaMemcpyHostToDevice, strm)) != cudaSuccess)
-        return cuda_fail(e, "far-field pose upload");
+    if ((st = upload_poses_ff(s->dev, sc, P, tx, rx, budget, offset, strm)) != HSR_OK) return st;
     st = run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, HSR_SPLAT_DIRICHLET16, 1, sc.rows, strm);
     if (st != HSR_OK) return st;
-    if ((e = cudaMemcpyAsync(out_rows, sc.rows, sizeof(float) * 2 * size_t(P) * N, cudaMemcpyDeviceToHost, strm)) !=
-        cudaSuccess)
-        return cuda_fail(e, "row download");
-    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "far-field batch run");
-    return read_status(sc, strm);
+    return fetch_rows(sc, out_rows, 2 * size_t(P) * N, strm);
 }
 
 // ---- autotuning of the plain wavefront launch --------------------------------------
@@ -1247,13 +1274,14 @@ hsr_status hsr_autotune_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
     std::lock_guard<std::mutex> lk(s->mu);
     SceneDev &d = s->dev;
     Scratch sc;
-    if ((st = ensure_scratch(d, P, N, sc, nullptr, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
-    if ((st = upload_poses(sc, P, tx, rx, budget, offset, cudaMemcpyHostToDevice, nullptr)) != HSR_OK) return st;
+    if ((st = ensure_scratch(d, P, N, sc, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
+    if ((st = upload_poses(d, sc, P, tx, rx, budget, offset, nullptr)) != HSR_OK) return st;
     const LaunchConfig saved = d.tuned;
     auto trial = [&](const LaunchConfig &c, float &ms) -> hsr_status {
         d.tuned = c;
         ms = 1e30f;
-        for (int r = 0; r < 2; ++r) {
+        sc.fresh = true;
+        for (int r = 0; r < 2; ++r, sc.fresh = false) {
             hsr_status rs = run_plain(d, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, sc.rows, nullptr);
             if (rs != HSR_OK) return rs;
             cudaError_t e = cudaEventSynchronize(d.ev1);
@@ -1360,12 +1388,12 @@ hsr_status hsr_debug_traversal_counts(hsr_scene *s, const hsr_rf_config *rf, int
     if (st != HSR_OK) return st;
     std::lock_guard<std::mutex> lk(s->mu);
     Scratch sc;
-    if ((st = ensure_scratch(s->dev, P, N, sc, nullptr)) != HSR_OK) return st;
+    if ((st = ensure_scratch(s->dev, P, N, sc)) != HSR_OK) return st;
     unsigned long long *d_cnt = nullptr;
     std::string err;
     if (!dev_alloc(&d_cnt, 4 * sizeof(unsigned long long), err)) return fail(HSR_ERR_OUT_OF_MEMORY, err);
     cudaMemset(d_cnt, 0, 4 * sizeof(unsigned long long));
-    if ((st = upload_poses(sc, P, tx, rx, budget, offset, cudaMemcpyHostToDevice, 0)) != HSR_OK) {
+    if ((st = upload_poses(s->dev, sc, P, tx, rx, budget, offset, 0)) != HSR_OK) {
         cudaFree(d_cnt);
         return st;
     }
@@ -1539,7 +1567,8 @@ hsr_status hsr_batch_graph_create(hsr_scene *s, const hsr_rf_config *rf, int32_t
             return st != HSR_OK ? st : cuda_fail(e, "graph synthesis operand");
         }
     }
-    const Scratch sc = carve(g->scratch, P, N, fine, local);
+    Scratch sc = carve(g->scratch, P, N, fine, local);
+    use_device_poses(sc, d_tx, d_rx, d_budget, d_offset);
     g->status = sc.counters;
     cudaStream_t cs = nullptr;
     if ((e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking)) != cudaSuccess) {
@@ -1550,8 +1579,7 @@ hsr_status hsr_batch_graph_create(hsr_scene *s, const hsr_rf_config *rf, int32_t
     if ((e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) {
         rst = cuda_fail(e, "begin capture");
     } else {
-        rst = upload_poses(sc, P, d_tx, d_rx, d_budget, d_offset, cudaMemcpyDeviceToDevice, cs);
-        if (rst == HSR_OK) rst = run_plain(gdev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, d_out_rows, cs);
+        rst = run_plain(gdev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, d_out_rows, cs);
         cudaGraph_t graph = nullptr;
         e = cudaStreamEndCapture(cs, &graph);
         g->graph = graph;

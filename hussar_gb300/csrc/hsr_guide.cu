@@ -284,8 +284,8 @@ __global__ void __launch_bounds__(256) k_guide_step(const int *__restrict__ acti
 
 size_t guide_bytes_per_pose() {
     // samp child + p, train child + 3 acc, count, and the guided schedule (kGuideMaxIters
-    // iterations x 32 B)
-    return size_t(kGuideMaxNodes) * (4 + 4 + 4 + 12) + size_t(kGuideMaxIters) * 32 + 16;
+    // iterations x 32 B) with the total weight
+    return size_t(kGuideMaxNodes) * (4 + 4 + 4 + 12) + size_t(kGuideMaxIters) * 32 + 8 + 16;
 }
 
 int launch_guide_reset(int P, int *samp_child, float *samp_p, int *train_child, float *train_acc, int *train_count,

@@ -74,7 +74,7 @@ struct SceneDev {
     // scratch
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
-    unsigned *status = nullptr;  // device status word + work counter
+    std::vector<char> stage;     // host copy of a call's poses and budgets (one upload)
     void *guide = nullptr;       // guiding trees + step scratch, sized for guide_cap poses
     int guide_cap = 0;
     SynthOperand synth;          // cached twiddle operand (fine-histogram synthesis)
@@ -247,7 +247,8 @@ struct GuideMem {
     float *train_acc;
     int *train_count;
     // the whole schedule of a guided call, iteration-major: per iteration budget and
-    // Halton offset (int64), sample weight (float), train, clear and active flags (int)
+    // Halton offset (int64), sample weight (float), train, clear and active flags (int);
+    // then the poses' total weights (double)
     unsigned char *sched;
 };
 
@@ -266,7 +267,7 @@ inline GuideMem carve_guide(void *base, int P) {
     g.train_child = reinterpret_cast<int *>(take(4 * M));
     g.train_acc = reinterpret_cast<float *>(take(12 * M));
     g.train_count = reinterpret_cast<int *>(take(4 * size_t(P)));
-    g.sched = reinterpret_cast<unsigned char *>(take(size_t(kGuideMaxIters) * 32 * size_t(P)));
+    g.sched = reinterpret_cast<unsigned char *>(take((size_t(kGuideMaxIters) * 32 + 8) * size_t(P)));
     return g;
 }
 
@@ -283,10 +284,21 @@ extern int g_synth_engine;
 
 // Launches (all asynchronous on `st`).
 int launch_trace(const TraceParams &p, int phase_mode, int splat_mode, int grid, cudaStream_t st, std::string &err);
-int launch_tile_prefix(const int64_t *budget, int32_t pose_count, int32_t tile, int64_t *tile_start, cudaStream_t st);
+// What k_prepare sets up before a pass.
+struct PrepareParams {
+    const int64_t *budget;  // [pose_count]
+    int32_t pose_count;
+    int32_t tile;           // samples per work item
+    int64_t *tile_start;    // [pose_count + 1]
+    unsigned long long *work_counter;
+    unsigned *status;       // nullptr: kept
+    double *rows;           // [pose_count][row_len] accumulators to clear; nullptr: none
+    int64_t row_len;
+    const int *clear;       // per pose; nullptr: every row
+};
+int launch_prepare(const PrepareParams &q, cudaStream_t st);
 int launch_finalize(const double *acc, int32_t pose_count, int32_t samples, const int64_t *budget, float sample_weight,
                     const double *total_weight, int normalise, float *out_rows, cudaStream_t st);
-int launch_clear_rows(double *acc, int32_t pose_count, int32_t samples, const int *clear, cudaStream_t st);
 // A MIMO radar cube [chirp][sample][channel] from per-channel rows (hsr_simulate_frame).
 int launch_assemble_frame(const float *rows, int32_t chirps, int32_t samples, int32_t channels, float *frame,
                           cudaStream_t st);

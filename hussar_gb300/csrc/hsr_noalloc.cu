@@ -130,22 +130,23 @@ extern "C" hsr_status hsr_simulate_batch_device_noalloc(hsr_scene *scene, const 
     // must not be destroyed while this call's work is in flight
     std::lock_guard<std::mutex> lk(*scene_mutex(scene));
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
-    // what must start at zero: status word, work counter, this call's accumulators
-    cudaError_t e = cudaMemsetAsync(s->counters, 0, sizeof(s->counters), strm);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->acc, 0, sizeof(double) * 2 * size_t(P) * N, strm);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        set_last_error(std::string("clearing the static scratch: ") + cudaGetErrorString(e));
-        return HSR_ERR_CUDA;
-    }
     // the scene's tuned tile where it has one, else 4096 samples (the prefix holds
     // pose_count + 1 entries whatever the tile)
     const bool wave = g_path_kernel == 0 && flags->useGeometricalOptics != 0;
     const int32_t tile = sc->tuned.tile > 0 ? sc->tuned.tile : 4096;
     const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     int64_t *tile_start = reinterpret_cast<int64_t *>(s->tile_start);
-    if (launch_tile_prefix(d_budget, P, items.samples, tile_start, strm) != 0) {
-        set_last_error("tile prefix launch failed");
+    PrepareParams q{};
+    q.budget = d_budget;
+    q.pose_count = P;
+    q.tile = items.samples;
+    q.tile_start = tile_start;
+    q.work_counter = reinterpret_cast<unsigned long long *>(s->counters + 2);
+    q.status = s->counters;
+    q.rows = s->acc;
+    q.row_len = 2 * int64_t(N);
+    if (launch_prepare(q, strm) != 0) {
+        set_last_error("pass set-up launch failed");
         return HSR_ERR_CUDA;
     }
     TraceParams p{};

@@ -39,3 +39,23 @@ def test_every_sample_is_traced_once(setup, tile, poses):
         if b:
             ref = np.asarray(ref, np.complex128)
             assert np.linalg.norm(row - ref) <= 1e-4 * np.linalg.norm(ref), (tile, b)
+
+
+@pytest.mark.parametrize("poses", [1023, 1024, 1025, 2049])
+def test_prefix_over_many_poses(setup, oracle_lib, poses):
+    """The items' prefix is formed 1024 poses at a time; poses without samples lie between.
+    Every 97th pose and the ones around a chunk's end against the oracle."""
+    be, rf, t, _, _, _ = setup
+    be.set_launch_config(default=True)
+    rng = np.random.default_rng(poses)
+    budget = rng.integers(0, 700, poses) * (rng.random(poses) < 0.8)
+    budget[-1] = 300
+    offset = rng.integers(0, 1 << 20, poses)
+    ants = scenes.plane_poses(poses, 9, 10.0)
+    rows = be.simulate_batch(rf, N, t, ants, ants, budget, offset)
+    ora = oracle_lib.Scene(scenes.boxes_mesh(5, 40, 10.0))
+    for k in sorted({*range(0, poses, 97), 1022, min(1023, poses - 1), min(1024, poses - 1), poses - 1}):
+        if budget[k]:
+            ref = np.asarray(ora.fetch_row(rf, N, ants[k], ants[k], t, int(budget[k]), offset=int(offset[k])),
+                             np.complex128)
+            assert np.linalg.norm(rows[k] - ref) <= 1e-4 * np.linalg.norm(ref), k
