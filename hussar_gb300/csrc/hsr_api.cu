@@ -889,6 +889,26 @@ hsr_status hsr_debug_records(hsr_scene *s, const hsr_rf_config *rf, int32_t samp
     return st;
 }
 
+// The sum of n additions of a sample's weight (path.h:445). While the partial sums fit the
+// 53 bits of a double (the weight's significant bits and the count's together) every
+// addition is exact and the sum is the product; the loop it replaces took 2.6 ms of the
+// 3.4 of a run of 2^22 samples. Any additions after that are made one by one.
+static double weight_sum(float weight, int64_t n) {
+    if (n <= 0) return 0.0;
+    unsigned bits;
+    std::memcpy(&bits, &weight, sizeof(bits));
+    unsigned mantissa = (bits & 0x7fffffu) | 0x800000u;
+    int significant = 24;
+    while (!(mantissa & 1u)) {
+        mantissa >>= 1;
+        --significant;
+    }
+    const int64_t exact = std::min(n, int64_t(1) << (53 - significant));
+    double sum = double(exact) * double(weight);
+    for (int64_t i = exact; i < n; ++i) sum += double(weight);
+    return sum;
+}
+
 hsr_status hsr_backend_run(const hsr_scene *cs, const hsr_rf_config *rf, const hsr_frame_config *frame,
                            const hsr_antenna *tx, const hsr_antenna *rx, const hsr_tracer_flags *fl, int64_t budget,
                            int64_t index_offset, float sample_weight, int32_t phase_mode, float *frame_inout,
@@ -924,9 +944,7 @@ hsr_status hsr_backend_run(const hsr_scene *cs, const hsr_rf_config *rf, const h
         frame_inout[2 * id] += row[2 * k];
         frame_inout[2 * id + 1] += row[2 * k + 1];
     }
-    double w = 0;
-    for (int64_t i = 0; i < budget; ++i) w += double(sample_weight);
-    *total_weight_inout += w;
+    *total_weight_inout += weight_sum(sample_weight, budget);
     return HSR_OK;
 }
 
@@ -1078,9 +1096,7 @@ hsr_status hsr_backend_run_guided(hsr_scene *s, const hsr_rf_config *rf, const h
         frame_inout[2 * id] += row[2 * k];
         frame_inout[2 * id + 1] += row[2 * k + 1];
     }
-    double w = 0;
-    for (int64_t i = 0; i < budget; ++i) w += double(sample_weight);
-    *total_weight_inout += w;
+    *total_weight_inout += weight_sum(sample_weight, budget);
     return HSR_OK;
 }
 

@@ -59,3 +59,19 @@ def test_prefix_over_many_poses(setup, oracle_lib, poses):
             ref = np.asarray(ora.fetch_row(rf, N, ants[k], ants[k], t, int(budget[k]), offset=int(offset[k])),
                              np.complex128)
             assert np.linalg.norm(rows[k] - ref) <= 1e-4 * np.linalg.norm(ref), k
+
+
+@pytest.mark.parametrize("weight", [1.0, 0.1, 3.0, 1e-3, 0.0, 1e30])
+def test_total_weight_is_the_sum_of_additions(product_lib, weight):
+    """hsr_backend_run's total weight against adding the float weight sample by sample."""
+    mesh = scenes.dihedral_mesh()
+    from hussar_gb300 import FrameConfig, Scene
+    t = PathTracer()
+    t.doGuiding = False
+    t.configureFrame(FrameConfig(1, 8, 1))
+    rf, _ = scenes.rf_77ghz(8, 5e6)
+    a = scenes.dihedral_workload(poses=2).tx[0]
+    budget = 70001
+    t.currentSampleWeight = weight
+    gb300.Backend(mesh, t).run(Scene(rf, a, a), budget)
+    assert t.totalWeight == np.cumsum(np.full(budget, np.float64(np.float32(weight))))[-1]
