@@ -385,10 +385,10 @@ class _GB300:
             d = np.ascontiguousarray(directions, np.float32).reshape(-1, 3)
             n = len(o)
             tf = np.full(n, np.inf, np.float32) if tfar is None else np.ascontiguousarray(tfar, np.float32)
-            t = np.zeros(n, np.float32)
-            p = np.zeros((n, 3), np.float32)
-            nn = np.zeros((n, 3), np.float32)
-            prim = np.zeros(n, np.int32)
+            t = np.empty(n, np.float32)
+            p = np.empty((n, 3), np.float32)
+            nn = np.empty((n, 3), np.float32)
+            prim = np.empty(n, np.int32)
             _lib.check(_lib.lib().hsr_intersect(self._scene, n, _lib.ptr(o), _lib.ptr(d), _lib.ptr(tf),
                                                  _lib.ptr(t), _lib.ptr(p), _lib.ptr(nn), _lib.ptr(prim)))
             return t, p, nn, prim
@@ -398,7 +398,7 @@ class _GB300:
             o = np.ascontiguousarray(origins, np.float32).reshape(-1, 3)
             d = np.ascontiguousarray(directions, np.float32).reshape(-1, 3)
             tf = np.ascontiguousarray(tfar, np.float32).reshape(-1)
-            vis = np.zeros(len(o), np.int32)
+            vis = np.empty(len(o), np.int32)
             _lib.check(_lib.lib().hsr_visible(self._scene, len(o), _lib.ptr(o), _lib.ptr(d), _lib.ptr(tf),
                                                _lib.ptr(vis)))
             return vis

@@ -305,9 +305,18 @@ int launch_assemble_frame(const float *rows, int32_t chirps, int32_t samples, in
 // The device Halton sampler at host-chosen indices (hsr_debug_halton).
 int launch_debug_halton(const uint64_t *d_index, int64_t count, int dim, float *d_out);
 int launch_debug_sincos_sweep(unsigned lo_bits, unsigned hi_bits, unsigned long long *d_counts);
-int launch_ray_queries(const DNode *nodes, const DTri *tris, int64_t count, const float *o, const float *d,
-                       const float *tfar, float *t, float *p, float *n, int32_t *prim, int32_t *vis, unsigned *status,
-                       cudaStream_t st);
+// Ray queries: origins and directions [count][3], limits [count]; closest hits
+// to t, p, n, prim (any may be null), or occlusion to vis. Device-readable arrays.
+struct RayQueries {
+    const DNode *nodes;
+    const DTri *tris;
+    int64_t count;
+    const float *o, *d, *tfar;
+    float *t, *p, *n;
+    int32_t *prim, *vis;
+    unsigned *status;
+};
+int launch_ray_queries(const RayQueries &q, cudaStream_t st);
 int trace_smem_bytes(int samples, int splat_mode, int fine_bins);
 size_t wave_smem_bytes(int samples, bool guided);
 // The split-phase instantiations of the wavefront kernel (hsr_wave_split.cu).

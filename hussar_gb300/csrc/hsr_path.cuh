@@ -315,7 +315,8 @@ __device__ __forceinline__ void ff_sample(const FfAnt &a, float u0, float u1, f3
 // RX (`ff_rx` the receiver): FFAntenna::nee replaces NFAntenna::nee, and the direct term
 // is zero (FFAntenna::evaluate zeroes the ray, emitter.h:253-255). `local`: the pose's
 // neighbourhood list where `o` lies in its cube, which then answers the occlusion query.
-template <int kPhase, bool kCount, bool kFF = false, bool kEvery = false>
+// kStep: the BVH's answer comes with the warp's lanes in step.
+template <int kPhase, bool kCount, bool kFF = false, bool kEvery = false, bool kStep = false>
 __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *nodes, const DTri *tris,
                                          const hsr_rf_config &rf, int samples, const Ant &tx, const Ant &rx, int depth,
                                          f3 o, f3 d, f3 tmpd, f3 hit_n, const c3 &inc_H, const c3 &H, float time,
@@ -431,8 +432,9 @@ __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *node
     const bool trains = p.do_guide && !(gw.re == 0.f && gw.im == 0.f);
     if (!fl.poDiffraction && (kEvery || splats || trains)) {
         if (kCount) (*rays)++;
-        if (local ? any_local(*local, tris, o, nd, tMax)
-                  : any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt))
+        if (local   ? any_local(*local, tris, o, nd, tMax)
+            : kStep ? any_hit_in_step(nodes, tris, o, nd, kEpsilon, tMax, p.status)
+                    : any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt))
             return false;
     }
     if (!splats) return true;

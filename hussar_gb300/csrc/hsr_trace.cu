@@ -273,40 +273,45 @@ __global__ void k_finalize(const double *__restrict__ acc, int32_t pose_count, i
     out[2 * i + 1] = im;
 }
 
-__global__ void k_ray_queries(const DNode *__restrict__ nodes, const DTri *__restrict__ tris, int64_t count,
-                              const float *__restrict__ o, const float *__restrict__ d, const float *__restrict__ tfar,
-                              float *t, float *pp, float *nn, int32_t *prim, int32_t *vis, unsigned *status) {
-    int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (i >= count) return;
-    f3 oo = mk3(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
-    f3 dd = mk3(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
-    if (vis) {
-        vis[i] = any_hit<false>(nodes, tris, oo, dd, kEpsilon, tfar[i], status, nullptr) ? 0 : 1;
+__global__ void k_ray_queries(RayQueries q) {
+    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= q.count) return;
+    const f3 o = mk3(q.o[3 * i], q.o[3 * i + 1], q.o[3 * i + 2]);
+    const f3 d = mk3(q.d[3 * i], q.d[3 * i + 1], q.d[3 * i + 2]);
+    if (q.vis) {
+        q.vis[i] = any_hit_in_step(q.nodes, q.tris, o, d, kEpsilon, q.tfar[i], q.status) ? 0 : 1;
         return;
     }
     float th;
-    int pr;
-    int slot = closest_hit<false>(nodes, tris, oo, dd, kEpsilon, tfar[i], th, pr, status, nullptr);
+    int prim;
+    const int slot = closest_hit_in_step(q.nodes, q.tris, o, d, kEpsilon, q.tfar[i], th, prim, q.status);
+    f3 n = mk3(0.f, 0.f, 0.f), p = n;
     if (slot >= 0) {
-        DTri T = load_tri(tris, slot);
-        f3 n = hit_normal(T, dd);
-        f3 hp = add3(oo, scl3(th, dd));
-        t[i] = th;
-        prim[i] = pr;
-        pp[3 * i] = hp.x;
-        pp[3 * i + 1] = hp.y;
-        pp[3 * i + 2] = hp.z;
-        nn[3 * i] = n.x;
-        nn[3 * i + 1] = n.y;
-        nn[3 * i + 2] = n.z;
-    } else {
-        t[i] = CUDART_INF_F;
-        prim[i] = -1;
-        for (int k = 0; k < 3; ++k) pp[3 * i + k] = nn[3 * i + k] = 0.f;
+        n = hit_normal(load_tri(q.tris, slot), d);
+        p = add3(o, scl3(th, d));
+    }
+    if (q.t) q.t[i] = slot >= 0 ? th : CUDART_INF_F;
+    if (q.prim) q.prim[i] = slot >= 0 ? prim : -1;
+    if (q.p) {
+        q.p[3 * i] = p.x;
+        q.p[3 * i + 1] = p.y;
+        q.p[3 * i + 2] = p.z;
+    }
+    if (q.n) {
+        q.n[3 * i] = n.x;
+        q.n[3 * i + 1] = n.y;
+        q.n[3 * i + 2] = n.z;
     }
 }
 
 }  // namespace
+
+int launch_ray_queries(const RayQueries &q, cudaStream_t st) {
+    if (q.count <= 0) return 0;
+    k_ray_queries<<<unsigned((q.count + 255) / 256), 256, 0, st>>>(q);
+    note_launches(1);
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
 
 int trace_smem_bytes(int samples, int splat_mode, int fine_bins) {
     (void)splat_mode;
@@ -460,16 +465,6 @@ int launch_debug_halton(const uint64_t *d_index, int64_t count, int dim, float *
 
 int launch_debug_sincos_sweep(unsigned lo_bits, unsigned hi_bits, unsigned long long *d_counts) {
     k_debug_sincos_sweep<<<152 * 16, 256>>>(lo_bits, hi_bits, d_counts);
-    note_launches(1);
-    return cudaGetLastError() == cudaSuccess ? 0 : 2;
-}
-
-int launch_ray_queries(const DNode *nodes, const DTri *tris, int64_t count, const float *o, const float *d,
-                       const float *tfar, float *t, float *p, float *n, int32_t *prim, int32_t *vis, unsigned *status,
-                       cudaStream_t st) {
-    if (count <= 0) return 0;
-    k_ray_queries<<<unsigned((count + 255) / 256), 256, 0, st>>>(nodes, tris, count, o, d, tfar, t, p, n, prim, vis,
-                                                                  status);
     note_launches(1);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }

@@ -177,11 +177,14 @@ __device__ __forceinline__ bool arrive(const DTri *tris, int slot, float th, f3 
 // when the path continues with a stored hit. The reference's zero-field test (path.h:413,
 // 439) is the caller's: in GO mode the field does not change across the hit, so testing it
 // before or after is the same.
+template <bool kStep>
 __device__ __forceinline__ bool walk(const TraceParams &p, const DNode *nodes, const DTri *tris, f3 o, f3 d,
                                      float &time, float &r, double &plen, f3 &hp, f3 &n, float &cosT) {
     float th;
     int primh;
-    const int slot = closest_hit<false>(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status, nullptr);
+    const int slot =
+        kStep ? closest_hit_in_step(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status)
+              : closest_hit<false>(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status, nullptr);
     return slot >= 0 && arrive(tris, slot, th, o, d, time, r, plen, hp, n, cosT);
 }
 
@@ -388,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                 }
                 if (!fl.onlyIndirect) {
                     NeeOut ne;
-                    if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, 0, o, d,
+                    if (nee_eval<kPhase, false, kFF, false, kLocal>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, 0, o, d,
                                                      mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f), H, H, 0.f, 0.0, 0.f,
                                                      1.f, freq, pc.weight, ne, nullptr, nullptr, &S.ff[1],
                                                      local ? &L : nullptr) &&
@@ -412,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                         pending = slot < 0;
                         hit = !pending && arrive(HSR_TRIS, slot, cosT, o, d, time, r, plen, hp, n, cosT);
                     } else {
-                        hit = walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n, cosT);
+                        hit = walk<kLocal>(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n, cosT);
                     }
                     if (hit || pending) {
                         // deferred: the field now (the same operations as antenna_sample); a
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                 if (!resumed) {
                     reflect(nrm, d, H);
                     NeeOut ne;
-                    if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, depth, o, d, din,
+                    if (nee_eval<kPhase, false, kFF, false, kLocal>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, depth, o, d, din,
                                                      nrm, Hin, H, time, plen, r, cosT, freq, pc.weight, ne, nullptr,
                                                      nullptr, &S.ff[1], local ? &L : nullptr)) {
                         g.gw = cadd(g.gw, ne.gw_add);
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                         unsettled = slot < 0;
                         hit = !unsettled && arrive(HSR_TRIS, slot, cosT2, o, d, time, r, plen, hp, n2, cosT2);
                     } else {
-                        hit = walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n2, cosT2);
+                        hit = walk<kLocal>(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n2, cosT2);
                     }
                     if (hit || unsettled) {
                         push_path<kPhase, kLocal, kCap>(S, gst, unsettled ? o : hp, d, H, n2, time, r, cosT2, freq,
