@@ -40,7 +40,7 @@ struct LaunchConfig {
 constexpr int kWaveMaxQueueThreshold = 256;  // thresholds above 128: the 512-entry stack
 constexpr int kWaveDefaultQueue = 128;       // threshold 0 (the default) and up to 128: 384 entries
 constexpr int kWaveSmallQueue = 64;          // thresholds up to this run with a 320-entry stack
-constexpr int kWaveLocalQueue = 256;         // launches with neighbourhood lists: 512 entries
+constexpr int kWaveLocalQueue = 128;         // launches with neighbourhood lists: 384 entries
 // The work items of a wavefront launch whose tile (the most samples a CTA takes at once;
 // 4096 where none was chosen) is `tile`: one GENERATE stage each, pulled in runs of up to a
 // tile that shrink towards the end of the launch (pull_items in hsr_wave.cuh). A tile that
@@ -145,18 +145,23 @@ struct PoseJob {
 };
 
 // A pose's neighbourhood list (hsr_local.cuh): the triangles nearest its receiver, grouped
-// by plane, and the cube around the receiver that only they reach. planes 0: the pose has
+// by plane (nearest group first), and the cube around the receiver that only they reach. planes 0: the pose has
 // none.
-constexpr int kLocalTris = 64;
+constexpr int kLocalTris = 96;
 struct LocalList {
     float4 plane[kLocalTris];  // n . (p - centre) = w
-    int slot[kLocalTris];      // plane j's triangles: slot[start[j]] .. slot[start[j + 1] - 1]
+    float4 u[kLocalTris];      // a triangle's barycentric coordinates of a point of its plane:
+    float4 v[kLocalTris];      // xyz . (p - centre) - w
+    // x: margin of a plane's distances; y: Chebyshev distance from the centre of the nearest
+    // bounding box of its triangles, less a margin (ascending)
+    float2 range[kLocalTris];
+    float uv_eps[kLocalTris];     // margin of a triangle's coordinates
+    int slot[kLocalTris];      // plane j's triangles: start[j] .. start[j + 1] - 1
     unsigned char start[kLocalTris + 4];
     float cx, cy, cz;          // the receiver
     float h;                   // half the cube's edge
-    float eps;                 // margin of the plane test
     int planes;
-    int pad;
+    int pad[2];
 };
 static_assert(sizeof(LocalList) % 16 == 0, "copied in 16-byte words");
 

@@ -11,7 +11,7 @@ namespace {
 
 constexpr int kFrontier = 1024;    // nodes of one tree level a search holds
 constexpr int kCandidates = 1024;  // triangles a search holds
-constexpr int kNearest = 192;      // triangles that are ranked
+constexpr int kNearest = 3 * kLocalTris;  // triangles that are ranked
 constexpr int kSearchSteps = 14;
 
 // A scene whose point queries visit fewer nodes than this keeps to the BVH: the list's
@@ -160,8 +160,9 @@ __global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ 
     __shared__ Search S;
     __shared__ LocalList L;
     __shared__ int near_slot[kLocalTris];
+    __shared__ float near_dist[kLocalTris];
     __shared__ float4 near_plane[kLocalTris];
-    __shared__ unsigned char near_group[kLocalTris];
+    __shared__ unsigned char near_group[kLocalTris], next[kLocalTris];
     const int pose = blockIdx.x, lane = threadIdx.x;
     if (jobs) {
         nodes = jobs[pose].nodes;
@@ -178,60 +179,78 @@ __global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ 
     // the kLocalTris nearest in order, and the cube up to the next triangle's box
     for (int i = lane; i < n; i += 32) {
         const int rank = rank_of(S, n, i);
-        if (rank < kLocalTris) near_slot[rank] = S.near_slot[i];
-        if (rank == kLocalTris) L.h = local_half_edge(S.near_dist[i], c);
+        if (rank < kLocalTris) {
+            near_slot[rank] = S.near_slot[i];
+            near_dist[rank] = S.near_dist[i];
+        }
+        if (rank == kLocalTris) L.h = local_clear(S.near_dist[i], c);
     }
     __syncwarp();
     const float half = L.h;
-    float eps = 0.f;
-    for (int j = lane; j < kLocalTris; j += 32) {
-        float e;
-        near_plane[j] = local_plane(load_tri(tris, near_slot[j]), c, half, e);
-        eps = fmaxf(eps, e);
-    }
-    for (int off = 16; off; off >>= 1) eps = fmaxf(eps, __shfl_xor_sync(0xffffffffu, eps, off));
-    eps += local_merge_margin(half);
+    for (int j = lane; j < kLocalTris; j += 32) near_plane[j] = local_tri(load_tri(tris, near_slot[j]), c, half).plane;
     __syncwarp();
     // the planes in order of their nearest triangle: each triangle joins the first group
-    // whose plane it shares (lane l compares with groups l and l + 32)
-    static_assert(kLocalTris == 64, "two groups per lane");
-    int groups = 0, size[2] = {0, 0};
+    // whose plane it shares (a lane compares with the groups l, l + 32, ...)
+    constexpr int kPerLane = kLocalTris / 32;
+    static_assert(kLocalTris % 32 == 0 && kLocalTris < 256, "whole lanes of groups, offsets in a byte");
+    int groups = 0, size[kPerLane] = {};
     for (int j = 0; j < kLocalTris; ++j) {
         const float4 pl = near_plane[j];
-        const unsigned lo = __ballot_sync(0xffffffffu, lane < groups && local_same_plane(L.plane[lane], pl, half));
-        const unsigned hi =
-            __ballot_sync(0xffffffffu, lane + 32 < groups && local_same_plane(L.plane[lane + 32], pl, half));
-        const int g = lo ? __ffs(int(lo)) - 1 : hi ? 31 + __ffs(int(hi)) : groups;
+        int g = groups;
+#pragma unroll
+        for (int w = kPerLane - 1; w >= 0; --w) {
+            const unsigned same = __ballot_sync(
+                0xffffffffu, lane + 32 * w < groups && local_same_plane(L.plane[lane + 32 * w], pl, half));
+            if (same) g = 32 * w + __ffs(int(same)) - 1;
+        }
         if (g == groups) {
-            if (lane == 0) L.plane[g] = pl;
+            if (lane == 0) {
+                L.plane[g] = pl;
+                L.range[g].y = local_clear(near_dist[j], c);
+            }
             ++groups;
         }
         if (lane == 0) near_group[j] = (unsigned char)g;
-        if (lane == (g & 31)) ++size[g >> 5];
+#pragma unroll
+        for (int w = 0; w < kPerLane; ++w)
+            if (lane + 32 * w == g) ++size[w];
         __syncwarp();
     }
     // where each group starts, then its triangles
-    int first[2], total = 0;
-    for (int k = 0; k < 2; ++k) {
-        int sum = size[k];
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kPerLane; ++w) {
+        int sum = size[w];
         for (int off = 1; off < 32; off <<= 1) {
             const int v = __shfl_up_sync(0xffffffffu, sum, off);
             if (lane >= off) sum += v;
         }
-        first[k] = total + sum - size[k];
+        const int before = total + sum - size[w];
         total += __shfl_sync(0xffffffffu, sum, 31);
-        L.start[lane + 32 * k] = (unsigned char)first[k];
+        L.start[lane + 32 * w] = (unsigned char)before;
+        next[lane + 32 * w] = (unsigned char)before;
     }
     if (lane == 0) L.start[kLocalTris] = (unsigned char)kLocalTris;
     for (int j = 0; j < kLocalTris; ++j) {
         const int g = near_group[j];
-        if (lane == (g & 31)) L.slot[first[g >> 5]++] = near_slot[j];
+        if (lane == (g & 31)) L.slot[next[g]++] = near_slot[j];
+    }
+    __syncwarp();
+    for (int j = lane; j < groups; j += 32) {
+        float eps = 0.f;
+        for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
+            const LocalTri t = local_tri(load_tri(tris, L.slot[k]), c, half);
+            L.u[k] = t.u;
+            L.v[k] = t.v;
+            L.uv_eps[k] = t.uv_eps;
+            eps = fmaxf(eps, t.plane_eps);
+        }
+        L.range[j].x = eps + local_merge_margin(half);
     }
     if (lane == 0) {
         L.cx = c.x;
         L.cy = c.y;
         L.cz = c.z;
-        L.eps = eps;
         L.planes = groups;
     }
     __syncwarp();

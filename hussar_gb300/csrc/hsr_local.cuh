@@ -4,26 +4,31 @@
 // In a dense scene most of a path's traversal finds the same place again: on the boxes
 // workload (1 M triangles, about 57 overlapping boxes over any point) a segment is 5 cm long on
 // average, yet a query descends through the 110-130 nodes whose boxes hold that point. All
-// queries of a pose start there. So each pose gets the list of the 64 triangles whose bounding
+// queries of a pose start there. So each pose gets the list of the 96 triangles whose bounding
 // boxes are nearest its receiver, and the largest cube around the receiver that no other
 // triangle's box reaches (with a margin). A segment inside the cube can only meet listed
 // triangles: an occlusion query between two of its points, and a closest-hit query whose
-// hit lies inside, are settled by the list; 96-98 % of them on the boxes scene with 64
-// triangles (48: 95 %, 32: 91 %, 128: 98 %). A query that leaves the cube unanswered goes
-// to the BVH as before. Every lane of a warp tests the same triangle at the same time
-// (broadcast loads, no divergence), where a warp's lanes each walk the tree by themselves (14 of 32
-// active).
+// hit lies inside, are settled by the list; 98-99 % of them on the boxes scene (64 triangles:
+// 97 %, 32: 91 %). A query that leaves the cube unanswered goes to the BVH as before. Every
+// lane of a warp tests the same triangle at the same time (broadcast loads, no divergence),
+// where a warp's lanes each walk the tree by themselves (14 of 32 active).
 //
-// The list is grouped by plane, and a plane is tested first: the segment's end points on one
-// side of it, both further than `eps`, and none of its triangles can be met. `eps` covers
-// the rounding of tri_test, so that whatever tri_test would accept reaches it.
+// The list is grouped by plane, nearest group first, and a query ends at the first group
+// further out than its segment reaches, which shrinks with every hit found. A plane is
+// tested first: the segment's end points on one side of it, both further than its margin,
+// and none of its triangles can be met. Where the plane is crossed, the crossing's
+// barycentric coordinates in its triangles, from two more dot products each, tell hits from
+// misses, again with margins that cover the rounding of tri_test. Only what lies within the
+// margins, and a ray's final candidate, goes through tri_test itself, whose distance is the
+// answer.
 //
-// Whole calls before -> after: 96 poses on 1 M triangles (14 M paths, 4 bounces) 91 -> 17.1 ms,
-// 33 poses on 100 k triangles (reference phase) 17 -> 5.1 ms, 1999 short poses on 20 k
-// triangles 19.9 -> 12.8 ms (of which 10 on the host). With 32, 48, 64 and 96 triangles, one
-// plane each, the first of these took 28.5, 22.1, 19.3 and 20.5 ms; grouping by plane
-// took 64 to 17.1. The lists take one warp per pose and 0.13 ms before the launch. Served
-// mix (24 requests, two of three scenes dense) 31 -> 12 ms.
+// Whole calls without and with the lists: 96 poses on 1 M triangles (14 M paths, 4 bounces) 91
+// and 14.4 ms, 33 poses on 100 k triangles (reference phase) 17 and 3.9 ms, 1999 short poses on
+// 20 k triangles 19.9 (9 of it on the host) and 4.4 ms, served mix of 24 requests (two of three
+// scenes dense) 31 and 9.3 ms. On the first two: 64 triangles 15.3 and 4.4, 128 triangles
+// 14.4 and 3.9; every triangle of 64 through tri_test 19.3 and 5.6, grouped by plane 17.1 and
+// 5.1, 16.2 and 5.0 with the queries by the BVH in step. The lists take one warp per pose
+// and 0.13 ms before the launch.
 #pragma once
 #include <math_constants.h>
 
@@ -33,20 +38,29 @@
 
 namespace hsr {
 
-// Half the cube's edge where the nearest triangle that is not listed has its bounding box
-// at Chebyshev distance `next` from the centre: less a margin for the rounding of hit points
-// and of box corners formed from v0 + e.
-__device__ __forceinline__ float local_half_edge(float next, f3 c) {
-    return next - 1e-5f * (next + fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)))) - 1e-6f;
+// How far from the centre a point can lie and surely be outside a bounding box at Chebyshev
+// distance `dist` from it: less a margin for the rounding of hit points and of box corners
+// formed from v0 + e. With the nearest triangle that is not listed, half the cube's edge.
+__device__ __forceinline__ float local_clear(float dist, f3 c) {
+    return dist - 1e-5f * (dist + fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)))) - 1e-6f;
 }
 
-// A triangle's plane relative to the centre, and the margin its test needs: tri_test's
-// distance comes from products of edges and of vertex differences with a few roundings
-// each, so in terms of the distance to the plane its error is at most some 2^-22 of the
-// lengths involved, magnified by how acute the triangle is; so is the error of the plane
-// formed here in single precision. The margin is 2^-19 of them. A degenerate triangle gets the
-// plane 0 = 0, which is always tested. The normal's largest component is positive.
-__device__ __forceinline__ float4 local_plane(const DTri &T, f3 c, float h, float &eps) {
+// Chebyshev distance from the centre.
+__device__ __forceinline__ float local_radius(f3 q) { return fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))); }
+
+// A triangle's plane and coordinates relative to the centre, and their margins: tri_test's
+// distance comes from products of edges and of vertex differences with a few roundings each,
+// so in terms of the distance to the plane its error is at most some 2^-22 of the lengths
+// involved, magnified by how acute the triangle is; so is the error of what is formed here
+// in single precision. The margin is 2^-19 of them, and that distance over the triangle's
+// heights for its coordinates. A degenerate triangle gets the plane 0 = 0, which is always
+// crossed, at no number. The normal's largest component is positive.
+struct LocalTri {
+    float4 plane, u, v;
+    float plane_eps, uv_eps;
+};
+
+__device__ __forceinline__ LocalTri local_tri(const DTri &T, f3 c, float h) {
     const f3 e1 = mk3(T.e1.x, T.e1.y, T.e1.z), e2 = mk3(T.e2.x, T.e2.y, T.e2.z);
     const f3 v = mk3(T.v0.x - c.x, T.v0.y - c.y, T.v0.z - c.z);
     const f3 n = crs3(e1, e2);
@@ -54,15 +68,23 @@ __device__ __forceinline__ float4 local_plane(const DTri &T, f3 c, float h, floa
     float big = n.x;
     if (fabsf(n.y) > fabsf(big)) big = n.y;
     if (fabsf(n.z) > fabsf(big)) big = n.z;
-    const float inv = len > 0.f ? (big < 0.f ? -1.f : 1.f) / len : 0.f;
-    const f3 u = scl3(inv, n);
-    const float acute = fminf(fmaxf(l1 * l2 * fabsf(inv), 1.f), 1e6f);
-    eps = 2e-6f * (nrm3(v) + l1 + l2 + h) * acute;
-    return make_float4(u.x, u.y, u.z, dot3(u, v));
+    const float size = len > 0.f ? 1.f / len : 0.f;
+    const f3 unit = scl3(size, n);
+    // u = (p - v0) . (e2 x n) / |n|^2, v = (p - v0) . (n x e1) / |n|^2
+    const f3 nu = scl3(size, crs3(e2, unit)), nv = scl3(size, crs3(unit, e1));
+    const f3 facing = scl3(big < 0.f ? -1.f : 1.f, unit);
+    const float acute = fminf(fmaxf(l1 * l2 * size, 1.f), 1e6f);
+    LocalTri t;
+    t.plane = make_float4(facing.x, facing.y, facing.z, dot3(facing, v));
+    t.u = make_float4(nu.x, nu.y, nu.z, dot3(nu, v));
+    t.v = make_float4(nv.x, nv.y, nv.z, dot3(nv, v));
+    t.plane_eps = 2e-6f * (nrm3(v) + l1 + l2 + h) * acute;
+    t.uv_eps = 2.f * fmaxf(nrm3(nu), nrm3(nv)) * t.plane_eps + 1e-6f;
+    return t;
 }
 
 // Whether two planes share a group: they are apart by less than local_merge_margin anywhere
-// in the cube, which the pose's eps takes in.
+// in the cube, which the margins take in.
 __device__ __forceinline__ bool local_same_plane(float4 a, float4 b, float h) {
     return fabsf(a.x - b.x) <= 1e-6f && fabsf(a.y - b.y) <= 1e-6f && fabsf(a.z - b.z) <= 1e-6f &&
            fabsf(a.w - b.w) <= 1e-6f * h;
@@ -74,6 +96,28 @@ __device__ __forceinline__ bool local_holds(const LocalList &L, f3 p) {
     return fmaxf(fabsf(p.x - L.cx), fmaxf(fabsf(p.y - L.cy), fabsf(p.z - L.cz))) <= L.h;
 }
 
+// 1 / x within 2 ulps (0: infinite).
+__device__ __forceinline__ float local_inverse(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.f / x;
+#endif
+}
+
+// Where a point of its plane lies in triangle k: -1 outside, 1 inside, 0 too near an edge (or
+// no number) to tell. `scale`: the coordinates' margin in units of the list's.
+__device__ __forceinline__ int local_inside(const LocalList &L, int k, f3 p, float scale) {
+    const float4 a = L.u[k], b = L.v[k];
+    const float u = __fmaf_rn(a.x, p.x, __fmaf_rn(a.y, p.y, __fmaf_rn(a.z, p.z, -a.w)));
+    const float v = __fmaf_rn(b.x, p.x, __fmaf_rn(b.y, p.y, __fmaf_rn(b.z, p.z, -b.w)));
+    const float m = L.uv_eps[k] * scale;
+    const float least = fminf(u, fminf(v, 1.f - (u + v)));
+    return least < -m ? -1 : least > m ? 1 : 0;
+}
+
 // Closest hit of a ray that starts in the cube: the slot and its distance, or -1 where the
 // list does not settle it (no listed triangle is hit before the ray leaves the cube).
 __device__ __forceinline__ int closest_local(const LocalList &L, const DTri *__restrict__ tris, f3 o, f3 d,
@@ -83,30 +127,56 @@ __device__ __forceinline__ int closest_local(const LocalList &L, const DTri *__r
     const float ey = (L.h - copysignf(1.f, d.y) * q.y) * fabsf(safe_inv(d.y));
     const float ez = (L.h - copysignf(1.f, d.z) * q.z) * fabsf(safe_inv(d.z));
     const float t_exit = fminf(ex, fminf(ey, ez)) * 0.999999f;
-    const float eps = L.eps;
     t_best = t_exit;
     int best = -1, prim_best = 0x7fffffff;
-#pragma unroll 4
+    auto verify = [&](int slot) {
+        const DTri T = load_tri(tris, slot);
+        float t;
+        if (tri_test(T, o, d, kEpsilon, CUDART_INF_F, t) && t <= t_best) {
+            const int prim = __float_as_int(T.v0.w);
+            if (t < t_best || prim < prim_best) {
+                t_best = t;
+                prim_best = prim;
+                best = slot;
+            }
+        }
+    };
+    // The candidate: a sure hit at about `near` (within `slack`), nearer than any sure hit
+    // before it. What cannot be told from it, or is no sure hit, is verified at once.
+    int cand = -1;
+    float near = t_exit, slack = 0.f;
+    const float from = local_radius(q);
+    float reach = L.h;  // of the segment up to `near`: what lies further out cannot be met
     for (int j = 0; j < L.planes; ++j) {
         const float4 n = L.plane[j];
+        const float eps = L.range[j].x;
+        if (L.range[j].y > reach) break;
         const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
         const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
-        const float se = __fmaf_rn(s1, t_best, s0);
+        const float se = __fmaf_rn(s1, near + slack, s0);
         if (fminf(s0, se) > eps || fmaxf(s0, se) < -eps) continue;
+        const float inv = local_inverse(s1), steep = fabsf(inv);
+        const float t = -s0 * inv, tol = 2.f * eps * steep;
+        if (t < kEpsilon - tol || t > near + slack + tol) continue;
+        const f3 p = mk3(__fmaf_rn(t, d.x, q.x), __fmaf_rn(t, d.y, q.y), __fmaf_rn(t, d.z, q.z));
         for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
-            const int slot = L.slot[k];
-            const DTri T = load_tri(tris, slot);
-            float t;
-            if (tri_test(T, o, d, kEpsilon, CUDART_INF_F, t) && t <= t_best) {
-                const int prim = __float_as_int(T.v0.w);
-                if (t < t_best || prim < prim_best) {
-                    t_best = t;
-                    prim_best = prim;
-                    best = slot;
+            const int in = local_inside(L, k, p, 1.f + steep);
+            if (in < 0) continue;
+            if (in > 0 && t > kEpsilon + tol && t + tol < near - slack) {
+                cand = L.slot[k];
+                near = t;
+                slack = tol;
+                reach = fmaxf(from, local_radius(p)) + tol;
+            } else {
+                verify(L.slot[k]);
+                if (t_best < near) {
+                    near = t_best;
+                    slack = 0.f;
                 }
             }
         }
     }
+    if (cand >= 0) verify(cand);
     return best;
 }
 
@@ -114,16 +184,24 @@ __device__ __forceinline__ int closest_local(const LocalList &L, const DTri *__r
 // cube's centre.
 __device__ __forceinline__ bool any_local(const LocalList &L, const DTri *__restrict__ tris, f3 o, f3 d, float dist) {
     const f3 q = mk3(o.x - L.cx, o.y - L.cy, o.z - L.cz);
-    const float eps = L.eps;
-#pragma unroll 4
+    const float reach = local_radius(q);
     for (int j = 0; j < L.planes; ++j) {
         const float4 n = L.plane[j];
+        const float eps = L.range[j].x;
+        if (L.range[j].y > reach) break;
         const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
         if (fminf(s0, -n.w) > eps || fmaxf(s0, -n.w) < -eps) continue;
+        const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
+        const float inv = local_inverse(s1), steep = fabsf(inv);
+        const float t = -s0 * inv, tol = 2.f * eps * steep;
+        if (t < kEpsilon - tol || t > dist + tol) continue;
+        const f3 p = mk3(__fmaf_rn(t, d.x, q.x), __fmaf_rn(t, d.y, q.y), __fmaf_rn(t, d.z, q.z));
         for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
-            const DTri T = load_tri(tris, L.slot[k]);
-            float t;
-            if (tri_test(T, o, d, kEpsilon, dist, t)) return true;
+            const int in = local_inside(L, k, p, 1.f + steep);
+            if (in < 0) continue;
+            if (in > 0 && t > kEpsilon + tol && t < dist - tol) return true;
+            float th;
+            if (tri_test(load_tri(tris, L.slot[k]), o, d, kEpsilon, dist, th)) return true;
         }
     }
     return false;

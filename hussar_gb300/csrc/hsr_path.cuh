@@ -299,30 +299,37 @@ __device__ __forceinline__ void ff_sample(const FfAnt &a, float u0, float u1, f3
     H = c3_div(a.pol, a.pdf);
 }
 
-// Returns false when the estimate is occluded or skipped (no record, no splat).
+// A next-event estimate between its two halves: what it is worth if the path sees the
+// receiver, and the occlusion query that decides that.
+struct NeeState {
+    f3 nd;        // direction and distance to the receiver
+    float dist;
+    float ntime;  // time of flight and path length at the receiver
+    double nlen;
+    cf v, gw;
+    float dphase;
+    bool ask;     // whether the query's answer matters
+    bool splats;
+};
+
+// The first half. Returns false when the estimate is skipped.
 // The occlusion query comes last, and only where its answer matters: an estimate that is
 // exactly zero (the receiver behind the surface, the reflected ray further from the
 // receiver than the filter's taper reaches, 3.7 m at 77 GHz) adds the same nothing either
 // way. Urban canyon (1 M triangles, 5 bounces): 3.02 -> 2.16 rays and 59 -> 40 nodes per
 // path, a 12 x 2^19-sample frame 6.6-7.3 -> 5.6 ms; sphere + ground 1.86 -> 1.83 rays; the
 // dense boxes, whose paths stay within metres of the sensor, skip none and run the same
-// (sweep of 96 poses 91 ms either way). kEvery (the recording
-// kernel) asks for every estimate, so that a record exists exactly where the path sees
-// the receiver.
-// depth == 0: direct TX->RX connection (only with onlyIndirect = false).
-// `nodes`/`tris` are the scene the pose traces, `rf`/`samples` its chirp and range bins
+// (sweep of 96 poses 91 ms either way). kEvery (the recording kernel) asks for every
+// estimate, so that a record exists exactly where the path sees the receiver.
+// depth == 0: direct TX->RX connection (only with onlyIndirect = false). `rf`: the chirp
 // (uniform over a launch, or the pose's PoseJob in a mixed batch). kFF: far-field TX and
 // RX (`ff_rx` the receiver): FFAntenna::nee replaces NFAntenna::nee, and the direct term
-// is zero (FFAntenna::evaluate zeroes the ray, emitter.h:253-255). `local`: the pose's
-// neighbourhood list where `o` lies in its cube, which then answers the occlusion query.
-// kStep: the BVH's answer comes with the warp's lanes in step.
-template <int kPhase, bool kCount, bool kFF = false, bool kEvery = false, bool kStep = false>
-__device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *nodes, const DTri *tris,
-                                         const hsr_rf_config &rf, int samples, const Ant &tx, const Ant &rx, int depth,
-                                         f3 o, f3 d, f3 tmpd, f3 hit_n, const c3 &inc_H, const c3 &H, float time,
-                                         double plen, float r, float cosTheta, float freq, float sampleWeight,
-                                         NeeOut &out, TraversalCounters *cnt, unsigned *rays,
-                                         const FfAnt *ff_rx = nullptr, const LocalList *local = nullptr) {
+// is zero (FFAntenna::evaluate zeroes the ray, emitter.h:253-255).
+template <bool kFF, bool kEvery>
+__device__ __forceinline__ bool nee_begin(const TraceParams &p, const Ant &tx, const Ant &rx, int depth, f3 o, f3 d,
+                                          f3 tmpd, f3 hit_n, const c3 &inc_H, const c3 &H, float time, double plen,
+                                          float r, float cosTheta, float freq, float sampleWeight, const FfAnt *ff_rx,
+                                          NeeState &st) {
     const hsr_tracer_flags &fl = p.flags;
     f3 nd;
     float rr;
@@ -420,24 +427,36 @@ __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *node
         }
     }
     if (depth > 0) gw = cadd(gw, v);
+    st.nd = nd;
+    st.dist = tMax;
+    st.ntime = ntime;
+    st.nlen = nlen;
+    st.v = v;
+    st.gw = gw;
+    st.dphase = dphase;
+    // Integrator::splat's early-out (integrator.h:113-135)
+    st.splats = fl.produceDebugImage || !(sampleWeight == 0.f || v.re == 0.f || v.im == 0.f);
+    const bool trains = p.do_guide && !(gw.re == 0.f && gw.im == 0.f);
+    st.ask = !fl.poDiffraction && (kEvery || st.splats || trains);
+    return true;
+}
+
+// The second half, for an estimate whose path sees the receiver: where and with what phase it
+// adds to the frame. `samples`: the range bins.
+template <int kPhase>
+__device__ __forceinline__ void nee_end(const hsr_rf_config &rf, int samples, const NeeState &st, float sampleWeight,
+                                        NeeOut &out) {
+    const float ntime = st.ntime;
+    const double nlen = st.nlen;
+    const cf v = st.v;
     out.time = ntime;
     out.v = v;
-    out.dphase = dphase;
-    out.gw_add = gw;
+    out.dphase = st.dphase;
+    out.gw_add = st.gw;
     out.splat = false;
     out.sample = 0.f;
     out.value = cf{0.f, 0.f};
-    // Integrator::splat's early-out (integrator.h:113-135)
-    const bool splats = fl.produceDebugImage || !(sampleWeight == 0.f || v.re == 0.f || v.im == 0.f);
-    const bool trains = p.do_guide && !(gw.re == 0.f && gw.im == 0.f);
-    if (!fl.poDiffraction && (kEvery || splats || trains)) {
-        if (kCount) (*rays)++;
-        if (local   ? any_local(*local, tris, o, nd, tMax)
-            : kStep ? any_hit_in_step(nodes, tris, o, nd, kEpsilon, tMax, p.status)
-                    : any_hit<kCount>(nodes, tris, o, nd, kEpsilon, tMax, p.status, cnt))
-            return false;
-    }
-    if (!splats) return true;
+    if (!st.splats) return;
     float sample;
     cf ph;
     if (kPhase == HSR_PHASE_REFERENCE_FP32) {
@@ -472,6 +491,29 @@ __device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *node
     out.sample = sample;
     out.value = cscl(cmul(v, ph), sampleWeight);
     out.splat = true;
+}
+
+// Both halves and the query, by one thread: false when the estimate is occluded or skipped (no
+// record, no splat). `local`: the pose's neighbourhood list where `o` lies in its cube,
+// which then answers the query.
+template <int kPhase, bool kCount, bool kFF = false, bool kEvery = false>
+__device__ __forceinline__ bool nee_eval(const TraceParams &p, const DNode *nodes, const DTri *tris,
+                                         const hsr_rf_config &rf, int samples, const Ant &tx, const Ant &rx, int depth,
+                                         f3 o, f3 d, f3 tmpd, f3 hit_n, const c3 &inc_H, const c3 &H, float time,
+                                         double plen, float r, float cosTheta, float freq, float sampleWeight,
+                                         NeeOut &out, TraversalCounters *cnt, unsigned *rays,
+                                         const FfAnt *ff_rx = nullptr, const LocalList *local = nullptr) {
+    NeeState st;
+    if (!nee_begin<kFF, kEvery>(p, tx, rx, depth, o, d, tmpd, hit_n, inc_H, H, time, plen, r, cosTheta, freq,
+                                sampleWeight, ff_rx, st))
+        return false;
+    if (st.ask) {
+        if (kCount) (*rays)++;
+        if (local ? any_local(*local, tris, o, st.nd, st.dist)
+                  : any_hit<kCount>(nodes, tris, o, st.nd, kEpsilon, st.dist, p.status, cnt))
+            return false;
+    }
+    nee_end<kPhase>(rf, samples, st, sampleWeight, out);
     return true;
 }
 

@@ -275,16 +275,23 @@ __global__ void k_finalize(const double *__restrict__ acc, int32_t pose_count, i
 
 __global__ void k_ray_queries(RayQueries q) {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (i >= q.count) return;
-    const f3 o = mk3(q.o[3 * i], q.o[3 * i + 1], q.o[3 * i + 2]);
-    const f3 d = mk3(q.d[3 * i], q.d[3 * i + 1], q.d[3 * i + 2]);
+    const bool active = i < q.count;
+    f3 o = mk3(0.f, 0.f, 0.f), d = mk3(0.f, 0.f, 1.f);
+    float tfar = 0.f;
+    if (active) {
+        o = mk3(q.o[3 * i], q.o[3 * i + 1], q.o[3 * i + 2]);
+        d = mk3(q.d[3 * i], q.d[3 * i + 1], q.d[3 * i + 2]);
+        tfar = q.tfar[i];
+    }
     if (q.vis) {
-        q.vis[i] = any_hit_in_step(q.nodes, q.tris, o, d, kEpsilon, q.tfar[i], q.status) ? 0 : 1;
+        const bool hidden = any_hit_in_step(active, q.nodes, q.tris, o, d, kEpsilon, tfar, q.status);
+        if (active) q.vis[i] = hidden ? 0 : 1;
         return;
     }
     float th;
     int prim;
-    const int slot = closest_hit_in_step(q.nodes, q.tris, o, d, kEpsilon, q.tfar[i], th, prim, q.status);
+    const int slot = closest_hit_in_step(active, q.nodes, q.tris, o, d, kEpsilon, tfar, th, prim, q.status);
+    if (!active) return;
     f3 n = mk3(0.f, 0.f, 0.f), p = n;
     if (slot >= 0) {
         n = hit_normal(load_tri(q.tris, slot), d);

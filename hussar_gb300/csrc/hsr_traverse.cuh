@@ -240,7 +240,8 @@ __device__ __forceinline__ bool any_hit(const DNode *__restrict__ nodes, const D
 // ---- the same queries, a warp's lanes kept in step ----
 // The loops above leave it to the compiler where lanes that took different branches meet
 // again, which in the ray-query kernel is late: 6.6 of 32 lanes were active. Here the
-// calling lanes go together: each walks up to kInStep nodes, then those that stand at a
+// whole warp goes together (every lane calls, those without a ray with active = false): each
+// walks up to kInStep nodes, then those that stand at a
 // leaf test it, until none has work left. Closest hits of 1 M rays, whole calls, loops above ->
 // here: urban canyon (1 M triangles) 1496 -> 580 us, boxes of 3000 triangles 1674 -> 740, of
 // 1 M 2544 -> 1725, sphere + ground 445 either way (1, 2 and 8 nodes per turn: 2000, 1870
@@ -249,16 +250,10 @@ __device__ __forceinline__ bool any_hit(const DNode *__restrict__ nodes, const D
 constexpr int kInStep = 4;
 constexpr int kNoNode = 0x7fffffff;
 
-__device__ __forceinline__ unsigned lanes_here() {
+// Whether any lane of the warp has work left.
+__device__ __forceinline__ bool any_lane(bool p) {
 #ifdef __CUDA_ARCH__
-    return __activemask();
-#else
-    return 1u;
-#endif
-}
-__device__ __forceinline__ bool any_of(unsigned lanes, bool p) {
-#ifdef __CUDA_ARCH__
-    return __any_sync(lanes, p) != 0;
+    return __any_sync(0xffffffffu, p) != 0;
 #else
     return p;
 #endif
@@ -267,8 +262,9 @@ __device__ __forceinline__ bool any_of(unsigned lanes, bool p) {
 struct Walk {
     int stack[kTraversalStack];
     int sp = 0;
-    int node = 0;
+    int node;
 
+    __device__ __forceinline__ explicit Walk(bool active) : node(active ? 0 : kNoNode) {}
     __device__ __forceinline__ bool inside() const { return node >= 0 && node != kNoNode; }
     __device__ __forceinline__ void pop() { node = sp == 0 ? kNoNode : stack[--sp]; }
     // one node: to the nearer child hit, the other one deferred
@@ -293,12 +289,11 @@ struct Walk {
 };
 
 // closest_hit's answer.
-__device__ __forceinline__ int closest_hit_in_step(const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 o,
-                                                   f3 d, float tnear, float tfar, float &t_best, int &prim_best,
+__device__ __forceinline__ int closest_hit_in_step(bool active, const DNode *__restrict__ nodes,
+                                                   const DTri *__restrict__ tris, f3 o, f3 d, float tnear, float tfar, float &t_best, int &prim_best,
                                                    unsigned *status) {
     const RayPre rp = ray_pre(o, d);
-    const unsigned lanes = lanes_here();
-    Walk w;
+    Walk w(active);
     int best = -1;
     prim_best = 0x7fffffff;
     t_best = tfar;
@@ -306,7 +301,7 @@ __device__ __forceinline__ int closest_hit_in_step(const DNode *__restrict__ nod
 #pragma unroll 1
         for (int k = 0; k < kInStep; ++k)
             if (w.inside()) w.down(nodes, rp, tnear, t_best, status);
-        if (!any_of(lanes, w.node != kNoNode)) return best;
+        if (!any_lane(w.node != kNoNode)) return best;
         if (w.node < 0) {
             const int ref = ~w.node;
             const int last = (ref >> 3) + (ref & 7);
@@ -328,17 +323,17 @@ __device__ __forceinline__ int closest_hit_in_step(const DNode *__restrict__ nod
 }
 
 // any_hit's answer.
-__device__ __forceinline__ bool any_hit_in_step(const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 o,
-                                                f3 d, float tnear, float tfar, unsigned *status) {
+__device__ __forceinline__ bool any_hit_in_step(bool active, const DNode *__restrict__ nodes,
+                                                const DTri *__restrict__ tris, f3 o, f3 d, float tnear, float tfar,
+                                                unsigned *status) {
     const RayPre rp = ray_pre(o, d);
-    const unsigned lanes = lanes_here();
-    Walk w;
+    Walk w(active);
     bool hit = false;
     while (true) {
 #pragma unroll 1
         for (int k = 0; k < kInStep; ++k)
             if (w.inside()) w.down(nodes, rp, tnear, tfar, status);
-        if (!any_of(lanes, w.node != kNoNode)) return hit;
+        if (!any_lane(w.node != kNoNode)) return hit;
         if (w.node < 0) {
             const int ref = ~w.node;
             const int last = (ref >> 3) + (ref & 7);

@@ -84,21 +84,25 @@ constexpr int kGuideStackFields = 5;
 // field are those of a ray the list did not settle; without it they are a hit's.
 constexpr int kRayPending = 1 << 30;
 
-// `far`: onto the upper end of the stack (kLocal).
-template <int kPhase, bool kLocal, int kCap>
-__device__ __forceinline__ void push_path(WaveShared<kCap> &S, float *gst, f3 o, f3 d, const c3 &H, f3 n, float time,
-                                          float r, float cosT, float freq, int depth, double plen, const Guided &g,
-                                          bool far = false) {
-    // one shared atomic per warp and end: the lanes pushing there take consecutive slots
-    const unsigned active = __activemask();
+// The slots of the lanes that push a path at the lower or (`far`) the upper end: one shared
+// atomic per warp and end. The whole warp calls.
+template <int kCap> __device__ __forceinline__ int claim_slot(WaveShared<kCap> &S, bool push, bool far) {
     const int lane = threadIdx.x & 31;
-    const unsigned mine = kLocal ? __match_any_sync(active, far) : active;
-    const int leader = __ffs(mine) - 1;
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned lower = __ballot_sync(0xffffffffu, push && !far);
+    const unsigned upper = __ballot_sync(0xffffffffu, push && far);
     int base = 0;
-    if (lane == leader) base = atomicAdd(kLocal && far ? &S.count_far : &S.count, __popc(mine));
-    base = __shfl_sync(active, base, leader);
-    int slot = base + __popc(mine & ((1u << lane) - 1u));  // < kCap by construction (see k_wave)
-    if (kLocal && far) slot = kCap - 1 - slot;
+    if (lane == 0 && lower) base = atomicAdd(&S.count, __popc(lower));
+    if (lane == 1 && upper) base = atomicAdd(&S.count_far, __popc(upper));
+    const int low = __shfl_sync(0xffffffffu, base, 0) + __popc(lower & below);  // < kCap by construction (see k_wave)
+    const int up = __shfl_sync(0xffffffffu, base, 1) + __popc(upper & below);
+    return far ? kCap - 1 - up : low;
+}
+
+template <int kPhase, int kCap>
+__device__ __forceinline__ void store_path(WaveShared<kCap> &S, float *gst, int slot, f3 o, f3 d, const c3 &H, f3 n,
+                                           float time, float r, float cosT, float freq, int depth, double plen,
+                                           const Guided &g) {
     S.ox[slot] = o.x;
     S.oy[slot] = o.y;
     S.oz[slot] = o.z;
@@ -128,6 +132,21 @@ __device__ __forceinline__ void push_path(WaveShared<kCap> &S, float *gst, f3 o,
         gst[3 * kCap + slot] = g.gw.re;
         gst[4 * kCap + slot] = g.gw.im;
     }
+}
+
+// The lanes that call push a path each.
+template <int kPhase, int kCap>
+__device__ __forceinline__ void push_path(WaveShared<kCap> &S, float *gst, f3 o, f3 d, const c3 &H, f3 n, float time,
+                                          float r, float cosT, float freq, int depth, double plen, const Guided &g) {
+    // one shared atomic per warp: the lanes pushing here take consecutive slots
+    const unsigned active = __activemask();
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(active) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(&S.count, __popc(active));
+    base = __shfl_sync(active, base, leader);
+    const int slot = base + __popc(active & ((1u << lane) - 1u));  // < kCap by construction (see k_wave)
+    store_path<kPhase>(S, gst, slot, o, d, H, n, time, r, cosT, freq, depth, plen, g);
 }
 
 // A stable counting sort of the stage's items by key (< kPrimaryCells; the items
@@ -177,15 +196,40 @@ __device__ __forceinline__ bool arrive(const DTri *tris, int slot, float th, f3 
 // when the path continues with a stored hit. The reference's zero-field test (path.h:413,
 // 439) is the caller's: in GO mode the field does not change across the hit, so testing it
 // before or after is the same.
-template <bool kStep>
 __device__ __forceinline__ bool walk(const TraceParams &p, const DNode *nodes, const DTri *tris, f3 o, f3 d,
                                      float &time, float &r, double &plen, f3 &hp, f3 &n, float &cosT) {
     float th;
     int primh;
-    const int slot =
-        kStep ? closest_hit_in_step(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status)
-              : closest_hit<false>(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status, nullptr);
+    const int slot = closest_hit<false>(nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, primh, p.status, nullptr);
     return slot >= 0 && arrive(tris, slot, th, o, d, time, r, plen, hp, n, cosT);
+}
+
+// Dense scenes: the closest hit of each lane's segment (o, d), or -1, from the pose's list
+// (`local`) or the BVH. The whole warp calls, lanes without a segment with active = false,
+// and leaves together: run by the lanes that have one, what follows the query ran once for each
+// group of lanes that left it together (14 of 32 lanes active on the boxes; sweep of 96
+// poses 16.1 ms against 14.3).
+__device__ __forceinline__ int warp_closest(bool active, bool local, const LocalList &L, const TraceParams &p,
+                                            const DNode *nodes, const DTri *tris, f3 o, f3 d, float &th) {
+    int slot = -1, prim;
+    if (!local)
+        slot = closest_hit_in_step(active, nodes, tris, o, d, kEpsilon, CUDART_INF_F, th, prim, p.status);
+    else if (active)
+        slot = closest_local(L, tris, o, d, th);
+    __syncwarp();
+    return slot;
+}
+
+// Whether each lane's segment from o along d meets anything up to `dist`, in the same manner.
+__device__ __forceinline__ bool warp_occluded(bool active, bool local, const LocalList &L, const TraceParams &p,
+                                              const DNode *nodes, const DTri *tris, f3 o, f3 d, float dist) {
+    bool hit = false;
+    if (!local)
+        hit = any_hit_in_step(active, nodes, tris, o, d, kEpsilon, dist, p.status);
+    else if (active)
+        hit = any_local(L, tris, o, d, dist);
+    __syncwarp();
+    return hit;
 }
 
 // PathTracer::run's derived chirp quantities (path.h:240, radar.h:128-130).
@@ -249,13 +293,15 @@ template <int kQueue> size_t wave_smem_for(int samples, bool guided, bool local 
 // kLazy (the field_on_hit launch shape): with indirect-only paths, a primary ray's
 // antenna field is formed only once the ray has hit something.
 // kLocal (dense scenes): each pose has a neighbourhood list (p.local, hsr_local.cuh). The
-// stack (512 entries: 384 ran 2 % slower) then has two ends. Paths whose hit point lies in the list's cube are at the lower
-// end; their EXTEND asks the list alone: the occlusion query is settled by it, and a
-// closest-hit query that is not becomes a pending ray at the upper end. The upper end holds
-// those and the paths outside the cube; its EXTEND asks the BVH. A stage works on one end
-// (the fuller one), so a warp never waits for one lane's tree traversal among 31 list
-// lookups. Active lanes 14 -> 26 of 32, instructions per path a fifth (boxes, 1 M triangles).
-// field_on_hit and coherent_order don't apply here.
+// stack (384 entries; 512 leave the L1 too little beside the list: 0-5 % slower) then has two
+// ends. Paths whose hit point lies in the list's cube are at the lower end; their EXTEND
+// asks the list alone: the occlusion query is settled by it, and a closest-hit query that is
+// not becomes a pending ray at the upper end. The upper end holds those and the paths
+// outside the cube; its EXTEND asks the BVH. A stage works on one end (the fuller one), so a
+// warp never waits for one lane's tree traversal among 31 list lookups. The stages' parts
+// run by the whole warp, which meets after each query; in this manner the other forms lose
+// 4 % (urban) to 29 % (sphere, whose rays mostly miss at the root) and keep theirs.
+// field_on_hit and coherent_order don't apply here (the coherent order costs 7 to 20 %).
 template <int kPhase, bool kMixed, int kQueue, bool kFF = false, bool kLazy = false, bool kLocal = false>
 __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
     constexpr int kCap = kThreads + kQueue;
@@ -367,69 +413,107 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             const bool local = kLocal && L.planes > 0;  // the sensor lies in the cube
             bool has_item = false;
             float4 item = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (s < gen_end) {
-                const uint64_t hindex = uint64_t(pc.offset + s);
-                const float freq = rf.startFreq + halton(hindex, 0) * HSR_BANDWIDTH;
-                Guided g{halton(hindex, 1 + kGet2DFirst), halton(hindex, 1 + kGet2DSecond), 1.f, cf{0.f, 0.f}};
-                if (fl.doGuiding) g.pdf = guide_sample(pc.samp_child, pc.samp_p, g.x0, g.x1);
-                f3 o, d;
+            if constexpr (kLocal) {
+                const bool mine = s < gen_end;
+                float freq = 0.f;
+                Guided g{0.f, 0.f, 1.f, cf{0.f, 0.f}};
+                f3 o = mk3(0.f, 0.f, 0.f), d = mk3(0.f, 0.f, 1.f);
                 c3 H;
-                f3 ldir = mk3(0.f, 0.f, 0.f);  // kLazy: the local direction the field is formed from
-                const bool deferred = kLazy && fl.onlyIndirect;
-                if (kFF) {
-                    ff_sample(S.ff[0], g.x0, g.x1, o, d, H);
-                    H = c3_scl(H, 1.f / g.pdf);
-                } else if (kLazy) {
-                    o = pc.tx.pos;
-                    ldir = uniform_sample_sphere<kPhase == HSR_PHASE_REFERENCE_FP32>(g.x0, g.x1);
-                    d = mulv(pc.tx.rot, ldir);
-                    if (!deferred) H = c3_scl(antenna_field(pc.tx, ldir), 1.f / g.pdf);
-                } else {
+                bool onward = false;
+                if (mine) {
+                    const uint64_t hindex = uint64_t(pc.offset + s);
+                    freq = rf.startFreq + halton(hindex, 0) * HSR_BANDWIDTH;
+                    g.x0 = halton(hindex, 1 + kGet2DFirst);
+                    g.x1 = halton(hindex, 1 + kGet2DSecond);
+                    if (fl.doGuiding) g.pdf = guide_sample(pc.samp_child, pc.samp_p, g.x0, g.x1);
                     o = pc.tx.pos;
                     antenna_sample<kPhase == HSR_PHASE_REFERENCE_FP32>(pc.tx, g.x0, g.x1, d, H);
                     H = c3_scl(H, 1.f / g.pdf);
-                }
-                if (!fl.onlyIndirect) {
-                    NeeOut ne;
-                    if (nee_eval<kPhase, false, kFF, false, kLocal>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, 0, o, d,
-                                                     mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f), H, H, 0.f, 0.0, 0.f,
-                                                     1.f, freq, pc.weight, ne, nullptr, nullptr, &S.ff[1],
-                                                     local ? &L : nullptr) &&
-                        ne.splat) {
-                        if (pc.fine_row) {
-                            splat_fine(pc.fine_row, p.fine_bins, ne.sample, ne.value);
-                        } else {
-                            item = splat_item(ne.sample, ne.value);
-                            has_item = true;
+                    if (!fl.onlyIndirect) {
+                        NeeOut ne;
+                        if (nee_eval<kPhase, false>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, 0, o, d,
+                                                         mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f), H, H, 0.f, 0.0, 0.f,
+                                                         1.f, freq, pc.weight, ne, nullptr, nullptr, nullptr,
+                                                         local ? &L : nullptr) &&
+                            ne.splat) {
+                            if (pc.fine_row) {
+                                splat_fine(pc.fine_row, p.fine_bins, ne.sample, ne.value);
+                            } else {
+                                item = splat_item(ne.sample, ne.value);
+                                has_item = true;
+                            }
                         }
                     }
+                    onward = !(0 >= fl.maxDepth || 0.f >= HSR_MAXDIST) && !c3_is_zero(H);
                 }
-                bool alive = false;
-                if (!(0 >= fl.maxDepth || 0.f >= HSR_MAXDIST) && (deferred || !c3_is_zero(H))) {
-                    float time = 0.f, r = 0.f, cosT;
-                    double plen = 0.0;
-                    f3 hp, n;
-                    bool hit, pending = false;
-                    if (local) {
-                        const int slot = closest_local(L, HSR_TRIS, o, d, cosT);
-                        pending = slot < 0;
-                        hit = !pending && arrive(HSR_TRIS, slot, cosT, o, d, time, r, plen, hp, n, cosT);
+                float time = 0.f, r = 0.f, cosT = 1.f;
+                double plen = 0.0;
+                f3 hp = o, n = d;
+                const int tri = warp_closest(onward, local, L, p, HSR_NODES, HSR_TRIS, o, d, cosT);
+                // what the list did not settle goes to the BVH in a stage of its own
+                const bool pending = local && onward && tri < 0;
+                const bool alive =
+                    pending || (tri >= 0 && arrive(HSR_TRIS, tri, cosT, o, d, time, r, plen, hp, n, cosT));
+                const int slot = claim_slot(S, alive, pending || !(local && local_holds(L, hp)));
+                if (alive)
+                    store_path<kPhase>(S, gst, slot, pending ? o : hp, d, H, n, time, r, cosT, freq,
+                                       pending ? kRayPending : 1, plen, g);
+                else if (mine)
+                    guide_train(pc, pc.train_child, s_g, 1, g.gw, g.pdf, g.x0, g.x1);
+            } else {
+                if (s < gen_end) {
+                    const uint64_t hindex = uint64_t(pc.offset + s);
+                    const float freq = rf.startFreq + halton(hindex, 0) * HSR_BANDWIDTH;
+                    Guided g{halton(hindex, 1 + kGet2DFirst), halton(hindex, 1 + kGet2DSecond), 1.f, cf{0.f, 0.f}};
+                    if (fl.doGuiding) g.pdf = guide_sample(pc.samp_child, pc.samp_p, g.x0, g.x1);
+                    f3 o, d;
+                    c3 H;
+                    f3 ldir = mk3(0.f, 0.f, 0.f);  // kLazy: the local direction the field is formed from
+                    const bool deferred = kLazy && fl.onlyIndirect;
+                    if (kFF) {
+                        ff_sample(S.ff[0], g.x0, g.x1, o, d, H);
+                        H = c3_scl(H, 1.f / g.pdf);
+                    } else if (kLazy) {
+                        o = pc.tx.pos;
+                        ldir = uniform_sample_sphere<kPhase == HSR_PHASE_REFERENCE_FP32>(g.x0, g.x1);
+                        d = mulv(pc.tx.rot, ldir);
+                        if (!deferred) H = c3_scl(antenna_field(pc.tx, ldir), 1.f / g.pdf);
                     } else {
-                        hit = walk<kLocal>(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n, cosT);
+                        o = pc.tx.pos;
+                        antenna_sample<kPhase == HSR_PHASE_REFERENCE_FP32>(pc.tx, g.x0, g.x1, d, H);
+                        H = c3_scl(H, 1.f / g.pdf);
                     }
-                    if (hit || pending) {
-                        // deferred: the field now (the same operations as antenna_sample); a
-                        // zero field ends the path as the reference's test before tracing would
-                        if (deferred) H = c3_scl(antenna_field(pc.tx, ldir), 1.f / g.pdf);
-                        if (!deferred || !c3_is_zero(H)) {
-                            push_path<kPhase, kLocal, kCap>(S, gst, pending ? o : hp, d, H, n, time, r, cosT, freq,
-                                                            pending ? kRayPending : 1, plen, g,
-                                                            pending || (kLocal && !(local && local_holds(L, hp))));
-                            alive = true;
+                    if (!fl.onlyIndirect) {
+                        NeeOut ne;
+                        if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, 0, o, d,
+                                                         mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f), H, H, 0.f, 0.0, 0.f,
+                                                         1.f, freq, pc.weight, ne, nullptr, nullptr, &S.ff[1]) &&
+                            ne.splat) {
+                            if (pc.fine_row) {
+                                splat_fine(pc.fine_row, p.fine_bins, ne.sample, ne.value);
+                            } else {
+                                item = splat_item(ne.sample, ne.value);
+                                has_item = true;
+                            }
                         }
                     }
+                    bool alive = false;
+                    if (!(0 >= fl.maxDepth || 0.f >= HSR_MAXDIST) && (deferred || !c3_is_zero(H))) {
+                        float time = 0.f, r = 0.f, cosT;
+                        double plen = 0.0;
+                        f3 hp, n;
+                        if (walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n, cosT)) {
+                            // deferred: the field now (the same operations as antenna_sample); a
+                            // zero field ends the path as the reference's test before tracing would
+                            if (deferred) H = c3_scl(antenna_field(pc.tx, ldir), 1.f / g.pdf);
+                            if (!deferred || !c3_is_zero(H)) {
+                                push_path<kPhase>(S, gst, hp, d, H, n, time, r, cosT, freq, 1, plen, g);
+                                alive = true;
+                            }
+                        }
+                    }
+                    if (!alive) guide_train(pc, pc.train_child, s_g, 1, g.gw, g.pdf, g.x0, g.x1);
                 }
-                if (!alive) guide_train(pc, pc.train_child, s_g, 1, g.gw, g.pdf, g.x0, g.x1);
             }
             if (!fl.onlyIndirect) splat_warp(s_re, s_im, HSR_N, has_item, item);
             __syncthreads();
@@ -492,18 +576,58 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
             __syncthreads();
             bool has_item = false;
             float4 item = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (mine) {
+            if constexpr (kLocal) {
                 f3 d = din;
                 c3 H = Hin;
-                const bool resumed = kLocal && (depth & kRayPending);  // its estimate is done
-                if (kLocal) depth &= kRayPending - 1;
-                bool onward = resumed;
-                if (!resumed) {
+                NeeState ne{};
+                bool estimate = false, onward = false;
+                if (mine) {
+                    const bool resumed = depth & kRayPending;  // its estimate is done
+                    depth &= kRayPending - 1;
+                    onward = resumed;
+                    if (!resumed) {
+                        reflect(nrm, d, H);
+                        estimate = nee_begin<false, false>(p, pc.tx, pc.rx, depth, o, d, din, nrm, Hin, H, time, plen, r,
+                                                         cosT, freq, pc.weight, nullptr, ne);
+                        onward = !(depth >= fl.maxDepth || r >= HSR_MAXDIST) && !c3_is_zero(H);
+                    }
+                }
+                const bool hidden = warp_occluded(estimate && ne.ask, local, L, p, HSR_NODES, HSR_TRIS, o, ne.nd,
+                                                          ne.dist);
+                if (estimate && !hidden) {
+                    NeeOut out;
+                    nee_end<kPhase>(rf, HSR_N, ne, pc.weight, out);
+                    g.gw = cadd(g.gw, out.gw_add);
+                    if (out.splat) {
+                        if (pc.fine_row) {
+                            splat_fine(pc.fine_row, p.fine_bins, out.sample, out.value);
+                        } else {
+                            item = splat_item(out.sample, out.value);
+                            has_item = true;
+                        }
+                    }
+                }
+                f3 hp = o, n2 = d;
+                float cosT2 = 1.f;
+                const int tri = warp_closest(onward, local, L, p, HSR_NODES, HSR_TRIS, o, d, cosT2);
+                const bool unsettled = local && onward && tri < 0;
+                const bool alive =
+                    unsettled || (tri >= 0 && arrive(HSR_TRIS, tri, cosT2, o, d, time, r, plen, hp, n2, cosT2));
+                const int to = claim_slot(S, alive, unsettled || !(L.planes > 0 && local_holds(L, hp)));
+                if (alive)
+                    store_path<kPhase>(S, gst, to, unsettled ? o : hp, d, H, n2, time, r, cosT2, freq,
+                                       unsettled ? depth | kRayPending : depth + 1, plen, g);
+                else if (mine)
+                    guide_train(pc, pc.train_child, s_g, 1, g.gw, g.pdf, g.x0, g.x1);
+            } else {
+                if (mine) {
+                    f3 d = din;
+                    c3 H = Hin;
                     reflect(nrm, d, H);
                     NeeOut ne;
-                    if (nee_eval<kPhase, false, kFF, false, kLocal>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, depth, o, d, din,
+                    if (nee_eval<kPhase, false, kFF>(p, HSR_NODES, HSR_TRIS, rf, HSR_N, pc.tx, pc.rx, depth, o, d, din,
                                                      nrm, Hin, H, time, plen, r, cosT, freq, pc.weight, ne, nullptr,
-                                                     nullptr, &S.ff[1], local ? &L : nullptr)) {
+                                                     nullptr, &S.ff[1])) {
                         g.gw = cadd(g.gw, ne.gw_add);
                         if (ne.splat) {
                             if (pc.fine_row) {
@@ -514,29 +638,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
                             }
                         }
                     }
-                    onward = !(depth >= fl.maxDepth || r >= HSR_MAXDIST) && !c3_is_zero(H);
-                }
-                bool alive = false;
-                if (onward) {
-                    f3 hp, n2;
-                    float cosT2;
-                    bool hit, unsettled = false;
-                    if (local) {
-                        const int slot = closest_local(L, HSR_TRIS, o, d, cosT2);
-                        unsettled = slot < 0;
-                        hit = !unsettled && arrive(HSR_TRIS, slot, cosT2, o, d, time, r, plen, hp, n2, cosT2);
-                    } else {
-                        hit = walk<kLocal>(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n2, cosT2);
+                    bool alive = false;
+                    if (!(depth >= fl.maxDepth || r >= HSR_MAXDIST) && !c3_is_zero(H)) {
+                        f3 hp, n2;
+                        float cosT2;
+                        if (walk(p, HSR_NODES, HSR_TRIS, o, d, time, r, plen, hp, n2, cosT2)) {
+                            push_path<kPhase>(S, gst, hp, d, H, n2, time, r, cosT2, freq, depth + 1, plen, g);
+                            alive = true;
+                        }
                     }
-                    if (hit || unsettled) {
-                        push_path<kPhase, kLocal, kCap>(S, gst, unsettled ? o : hp, d, H, n2, time, r, cosT2, freq,
-                                                        unsettled ? depth | kRayPending : depth + 1, plen, g,
-                                                        unsettled ||
-                                                            (kLocal && !(L.planes > 0 && local_holds(L, hp))));
-                        alive = true;
-                    }
+                    if (!alive) guide_train(pc, pc.train_child, s_g, 1, g.gw, g.pdf, g.x0, g.x1);
                 }
-                if (!alive) guide_train(pc, pc.train_child, s_g, 1, g.gw, g.pdf, g.x0, g.x1);
             }
             splat_warp(s_re, s_im, HSR_N, has_item, item);
             __syncthreads();

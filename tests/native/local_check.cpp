@@ -55,26 +55,33 @@ int main(int argc, char **argv) {
     L.cx = c.x;
     L.cy = c.y;
     L.cz = c.z;
-    L.h = local_half_edge(order[kLocalTris].first, c);
+    L.h = local_clear(order[kLocalTris].first, c);
     std::vector<std::vector<int>> group;
     for (int j = 0; j < kLocalTris; ++j) {
-        float e;
-        const float4 pl = local_plane(tris[order[j].second], c, L.h, e);
-        L.eps = std::max(L.eps, e);
+        const float4 pl = local_tri(tris[order[j].second], c, L.h).plane;
         size_t g = 0;
         while (g < group.size() && !local_same_plane(L.plane[g], pl, L.h)) ++g;
         if (g == group.size()) {
             L.plane[g] = pl;
+            L.range[g].y = local_clear(order[j].first, c);
             group.emplace_back();
         }
         group[g].push_back(order[j].second);
     }
-    L.eps += local_merge_margin(L.h);
     L.planes = int(group.size());
     int at = 0;
     for (size_t g = 0; g < group.size(); ++g) {
         L.start[g] = (unsigned char)at;
-        for (int s : group[g]) L.slot[at++] = s;
+        float eps = 0.f;
+        for (int s : group[g]) {
+            const LocalTri t = local_tri(tris[s], c, L.h);
+            L.u[at] = t.u;
+            L.v[at] = t.v;
+            L.uv_eps[at] = t.uv_eps;
+            eps = std::max(eps, t.plane_eps);
+            L.slot[at++] = s;
+        }
+        L.range[g].x = eps + local_merge_margin(L.h);
     }
     L.start[group.size()] = (unsigned char)at;
 
