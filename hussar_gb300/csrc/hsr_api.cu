@@ -1381,11 +1381,11 @@ hsr_status hsr_autotune_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
     }
     // store the shape explicitly: a threshold of 0 means "the default" to the kernel, but
     // the serving ticks read the scene's tuned threshold to pick their path stack
-    if (best.queue_threshold <= 0) best.queue_threshold = kWaveDefaultQueue;
+    if (best.queue_threshold <= 0) best.queue_threshold = kWaveMaxQueueThreshold;
     d.tuned = best;
     out_best->tile = best.tile > 0 ? best.tile : kTile;
     out_best->ctas_per_sm = best.ctas_per_sm;
-    out_best->queue_threshold = best.queue_threshold > 0 ? best.queue_threshold : kWaveDefaultQueue;
+    out_best->queue_threshold = best.queue_threshold;
     out_best->field_on_hit = best.field_on_hit;
     out_best->coherent_order = best.coherent_order;
     out_best->trace_ms = best_ms;

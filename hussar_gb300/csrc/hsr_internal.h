@@ -37,8 +37,8 @@ struct LaunchConfig {
     int32_t coherent_order = 0;   // see TraceParams::coherent_order
 };
 // wavefront path stacks: 256 + the GENERATE threshold entries; three capacities
-constexpr int kWaveMaxQueueThreshold = 256;  // thresholds above 128: the 512-entry stack
-constexpr int kWaveDefaultQueue = 128;       // threshold 0 (the default) and up to 128: 384 entries
+constexpr int kWaveMaxQueueThreshold = 256;  // above 128, and threshold 0: the 512-entry stack
+constexpr int kWaveDefaultQueue = 128;       // thresholds up to 128, guided, far-field: 384 entries
 constexpr int kWaveSmallQueue = 64;          // thresholds up to this run with a 320-entry stack
 constexpr int kWaveLocalQueue = 128;         // launches with neighbourhood lists: 384 entries
 // The work items of a wavefront launch whose tile (the most samples a CTA takes at once;

@@ -42,7 +42,7 @@ constexpr int kPrimaryCells = 8;
 
 // A CTA's live path states: a stack of kThreads + kQueue entries, where kQueue bounds the
 // paths left when GENERATE runs (the queue threshold). Three capacities are built: 384
-// entries (the default, thresholds up to 128), 320 (up to 64), whose 5 KB less shared
+// entries (thresholds up to 128), 320 (up to 64), whose 5 KB less shared
 // memory per CTA leaves more of the SM's L1 to the BVH (4 % on the dense boxes scenes,
 // which the autotuner runs at threshold 32 or 64), and 512 (up to 256), whose fuller
 // EXTEND stages pay where the BVH stays in L1 anyway (7 % on the sphere bench).
@@ -703,10 +703,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
 }
 
 // The stack capacity (as its GENERATE threshold) a launch with threshold q runs: 64 for
-// 1..64, 256 above 128, else (0 = the default, or 65..128) 128.
-inline int wave_capacity(int32_t q) {
-    return (q > 0 && q <= kWaveSmallQueue) ? kWaveSmallQueue : (q > kWaveDefaultQueue ? kWaveMaxQueueThreshold
-                                                                                      : kWaveDefaultQueue);
+// 1..64, 128 for 65..128, 256 above. The default (q = 0) is 256, whose fuller stages take
+// 5 % off the sphere (725 -> 690 us at 2^22 samples) and 1.5 % off the urban frame; dense
+// scenes, which want the L1 instead, have a form of their own. Guided launches, whose stack
+// holds more per path, and long rows keep 128 (256 would leave three CTAs per SM).
+inline int wave_capacity(int32_t q, int32_t samples, bool guided) {
+    if (q == 0) q = guided || samples > 1536 ? kWaveDefaultQueue : kWaveMaxQueueThreshold;
+    return q <= kWaveSmallQueue ? kWaveSmallQueue : q > kWaveDefaultQueue ? kWaveMaxQueueThreshold : kWaveDefaultQueue;
 }
 
 // The launch of one instantiation.
@@ -731,8 +734,8 @@ template <int kPhase, int kQueue> void wave_uniform(const TraceParams &p, int gr
 // tick asks for a threshold above 64 (its default: on the serving mix of dense boxes
 // and urban scenes it gives 1.18x the capacity of the 384-entry stack).
 template <int kPhase> void wave_dispatch(const TraceParams &p, int grid, cudaStream_t st) {
-    const int cap = wave_capacity(p.queue_threshold);
-    if (p.ff_tx) {  // far-field runs: the uniform form at the default capacity
+    const int cap = wave_capacity(p.queue_threshold, p.samples, p.do_guide != 0);
+    if (p.ff_tx) {  // far-field runs: the uniform form at one capacity
         wave_instance<kPhase, false, kWaveDefaultQueue, true>(p, grid, st);
     } else if (p.local) {
         if (p.jobs)
