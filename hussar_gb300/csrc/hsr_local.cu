@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ 
         }
         L.range[j].x = eps + local_merge_margin(half);
     }
+    const int whole = (groups + kLocalGroup - 1) / kLocalGroup * kLocalGroup;
+    if (groups + lane < whole) local_fill(L, groups + lane);
     if (lane == 0) {
         L.cx = c.x;
         L.cy = c.y;

@@ -23,12 +23,12 @@
 // answer.
 //
 // Whole calls without and with the lists: 96 poses on 1 M triangles (14 M paths, 4 bounces) 91
-// and 14.4 ms, 33 poses on 100 k triangles (reference phase) 17 and 3.9 ms, 1999 short poses on
-// 20 k triangles 19.9 (9 of it on the host) and 4.4 ms, served mix of 24 requests (two of three
-// scenes dense) 31 and 9.3 ms. On the first two: 64 triangles 15.3 and 4.4, 128 triangles
-// 14.4 and 3.9; every triangle of 64 through tri_test 19.3 and 5.6, grouped by plane 17.1 and
-// 5.1, 16.2 and 5.0 with the queries by the BVH in step. The lists take one warp per pose
-// and 0.13 ms before the launch.
+// and 13.3 ms, 33 poses on 100 k triangles (reference phase) 17 and 3.7 ms, 1999 short poses on
+// 20 k triangles 19.9 (9 of it on the host) and 4.2 ms, served mix of 24 requests (two of three
+// scenes dense) 31 and 8.8 ms. On the first two: 128 triangles 13.1 and 3.7; one plane at a
+// time instead of groups of 8 (kLocalGroup) 14.5 and 4.0, and so with 64 triangles 15.3 and
+// 4.4; every triangle of 64 through tri_test 19.3 and 5.6. The lists take one warp per pose and
+// 0.13 ms before the launch.
 #pragma once
 #include <math_constants.h>
 
@@ -107,6 +107,19 @@ __device__ __forceinline__ float local_inverse(float x) {
 #endif
 }
 
+__device__ __forceinline__ int local_lowest(unsigned m) { return __ffs(int(m)) - 1; }
+
+// Planes are tested kLocalGroup at a time for being crossed at all; then each lane takes the
+// ones it crosses one by one, its own at the same time as the other lanes theirs (groups of
+// 4: 13.2 and 3.8 ms on the workloads above, of 16: 13.4 and 3.7). The list is filled up to
+// whole groups with planes that are never crossed.
+constexpr int kLocalGroup = 8;
+static_assert(kLocalTris % kLocalGroup == 0, "whole groups");
+__device__ __forceinline__ void local_fill(LocalList &L, int j) {
+    L.plane[j] = make_float4(0.f, 0.f, 0.f, 1.f);
+    L.range[j] = make_float2(0.f, CUDART_INF_F);
+}
+
 // Where a point of its plane lies in triangle k: -1 outside, 1 inside, 0 too near an edge (or
 // no number) to tell. `scale`: the coordinates' margin in units of the list's.
 __device__ __forceinline__ int local_inside(const LocalList &L, int k, f3 p, float scale) {
@@ -147,31 +160,40 @@ __device__ __forceinline__ int closest_local(const LocalList &L, const DTri *__r
     float near = t_exit, slack = 0.f;
     const float from = local_radius(q);
     float reach = L.h;  // of the segment up to `near`: what lies further out cannot be met
-    for (int j = 0; j < L.planes; ++j) {
-        const float4 n = L.plane[j];
-        const float eps = L.range[j].x;
-        if (L.range[j].y > reach) break;
-        const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
-        const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
-        const float se = __fmaf_rn(s1, near + slack, s0);
-        if (fminf(s0, se) > eps || fmaxf(s0, se) < -eps) continue;
-        const float inv = local_inverse(s1), steep = fabsf(inv);
-        const float t = -s0 * inv, tol = 2.f * eps * steep;
-        if (t < kEpsilon - tol || t > near + slack + tol) continue;
-        const f3 p = mk3(__fmaf_rn(t, d.x, q.x), __fmaf_rn(t, d.y, q.y), __fmaf_rn(t, d.z, q.z));
-        for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
-            const int in = local_inside(L, k, p, 1.f + steep);
-            if (in < 0) continue;
-            if (in > 0 && t > kEpsilon + tol && t + tol < near - slack) {
-                cand = L.slot[k];
-                near = t;
-                slack = tol;
-                reach = fmaxf(from, local_radius(p)) + tol;
-            } else {
-                verify(L.slot[k]);
-                if (t_best < near) {
-                    near = t_best;
-                    slack = 0.f;
+    for (int j0 = 0; j0 < L.planes && !(L.range[j0].y > reach); j0 += kLocalGroup) {
+        unsigned crossed = 0;
+#pragma unroll 4
+        for (int k = 0; k < kLocalGroup; ++k) {
+            const float4 n = L.plane[j0 + k];
+            const float eps = L.range[j0 + k].x;
+            const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
+            const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
+            const float se = __fmaf_rn(s1, near + slack, s0);
+            if (!(fminf(s0, se) > eps || fmaxf(s0, se) < -eps)) crossed |= 1u << k;
+        }
+        for (; crossed; crossed &= crossed - 1) {
+            const int j = j0 + local_lowest(crossed);
+            const float4 n = L.plane[j];
+            const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
+            const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
+            const float inv = local_inverse(s1), steep = fabsf(inv);
+            const float t = -s0 * inv, tol = 2.f * L.range[j].x * steep;
+            if (t < kEpsilon - tol || t > near + slack + tol) continue;
+            const f3 p = mk3(__fmaf_rn(t, d.x, q.x), __fmaf_rn(t, d.y, q.y), __fmaf_rn(t, d.z, q.z));
+            for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
+                const int in = local_inside(L, k, p, 1.f + steep);
+                if (in < 0) continue;
+                if (in > 0 && t > kEpsilon + tol && t + tol < near - slack) {
+                    cand = L.slot[k];
+                    near = t;
+                    slack = tol;
+                    reach = fmaxf(from, local_radius(p)) + tol;
+                } else {
+                    verify(L.slot[k]);
+                    if (t_best < near) {
+                        near = t_best;
+                        slack = 0.f;
+                    }
                 }
             }
         }
@@ -185,23 +207,31 @@ __device__ __forceinline__ int closest_local(const LocalList &L, const DTri *__r
 __device__ __forceinline__ bool any_local(const LocalList &L, const DTri *__restrict__ tris, f3 o, f3 d, float dist) {
     const f3 q = mk3(o.x - L.cx, o.y - L.cy, o.z - L.cz);
     const float reach = local_radius(q);
-    for (int j = 0; j < L.planes; ++j) {
-        const float4 n = L.plane[j];
-        const float eps = L.range[j].x;
-        if (L.range[j].y > reach) break;
-        const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
-        if (fminf(s0, -n.w) > eps || fmaxf(s0, -n.w) < -eps) continue;
-        const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
-        const float inv = local_inverse(s1), steep = fabsf(inv);
-        const float t = -s0 * inv, tol = 2.f * eps * steep;
-        if (t < kEpsilon - tol || t > dist + tol) continue;
-        const f3 p = mk3(__fmaf_rn(t, d.x, q.x), __fmaf_rn(t, d.y, q.y), __fmaf_rn(t, d.z, q.z));
-        for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
-            const int in = local_inside(L, k, p, 1.f + steep);
-            if (in < 0) continue;
-            if (in > 0 && t > kEpsilon + tol && t < dist - tol) return true;
-            float th;
-            if (tri_test(load_tri(tris, L.slot[k]), o, d, kEpsilon, dist, th)) return true;
+    for (int j0 = 0; j0 < L.planes && !(L.range[j0].y > reach); j0 += kLocalGroup) {
+        unsigned crossed = 0;
+#pragma unroll 4
+        for (int k = 0; k < kLocalGroup; ++k) {
+            const float4 n = L.plane[j0 + k];
+            const float eps = L.range[j0 + k].x;
+            const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
+            if (!(fminf(s0, -n.w) > eps || fmaxf(s0, -n.w) < -eps)) crossed |= 1u << k;
+        }
+        for (; crossed; crossed &= crossed - 1) {
+            const int j = j0 + local_lowest(crossed);
+            const float4 n = L.plane[j];
+            const float s0 = __fmaf_rn(n.x, q.x, __fmaf_rn(n.y, q.y, __fmaf_rn(n.z, q.z, -n.w)));
+            const float s1 = __fmaf_rn(n.x, d.x, __fmaf_rn(n.y, d.y, n.z * d.z));
+            const float inv = local_inverse(s1), steep = fabsf(inv);
+            const float t = -s0 * inv, tol = 2.f * L.range[j].x * steep;
+            if (t < kEpsilon - tol || t > dist + tol) continue;
+            const f3 p = mk3(__fmaf_rn(t, d.x, q.x), __fmaf_rn(t, d.y, q.y), __fmaf_rn(t, d.z, q.z));
+            for (int k = L.start[j]; k < L.start[j + 1]; ++k) {
+                const int in = local_inside(L, k, p, 1.f + steep);
+                if (in < 0) continue;
+                if (in > 0 && t > kEpsilon + tol && t < dist - tol) return true;
+                float th;
+                if (tri_test(load_tri(tris, L.slot[k]), o, d, kEpsilon, dist, th)) return true;
+            }
         }
     }
     return false;

@@ -84,6 +84,7 @@ int main(int argc, char **argv) {
         L.range[g].x = eps + local_merge_margin(L.h);
     }
     L.start[group.size()] = (unsigned char)at;
+    for (int j = L.planes; j % kLocalGroup; ++j) local_fill(L, j);
 
     long settled = 0, wrong = 0, missed = 0, any_wrong = 0, occluded = 0;
     auto brute = [&](f3 o, f3 d, float &t_best) {
