@@ -11,7 +11,8 @@ namespace {
 
 constexpr int kFrontier = 1024;    // nodes of one tree level a search holds
 constexpr int kCandidates = 1024;  // triangles a search holds
-constexpr int kNearest = 3 * kLocalTris;  // triangles that are ranked
+constexpr int kNearest = 3 * kLocalTris;   // triangles that are ranked: at most,
+constexpr int kFewNearest = kLocalTris + 32;  // and where their distances allow it
 constexpr int kSearchSteps = 14;
 
 // A scene whose point queries visit fewer nodes than this keeps to the BVH: the list's
@@ -25,7 +26,7 @@ struct Search {
     float dist[kCandidates];
     int near_slot[kNearest];
     float near_dist[kNearest];
-    int next, found;
+    int leaf[kCandidates];  // leaf references
 };
 
 // Chebyshev distance of a point to a box.
@@ -34,67 +35,85 @@ __device__ __forceinline__ float box_distance(f3 c, float lx, float hx, float ly
 }
 
 // The triangles whose bounding boxes come within h of c, by one warp, level by level down
-// the tree. Returns their number (S.slot, S.dist), or -1 when there are more than fit;
+// the tree and then over the leaves met, whose triangles' loads need not wait for one
+// another. Returns their number (S.slot, S.dist), or -1 when there are more than fit;
 // `visited` counts the nodes whose children were looked at.
 __device__ int collect(Search &S, const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 c, float h,
                        int &visited) {
     const int lane = threadIdx.x;
-    int cur = 0, n = 1;
+    const unsigned before = (1u << lane) - 1u;
+    int cur = 0, n = 1, leaves = 0, found = 0;
     visited = 0;
-    if (lane == 0) {
-        S.frontier[0][0] = 0;
-        S.found = 0;
-    }
+    if (lane == 0) S.frontier[0][0] = 0;
     while (n > 0) {
-        if (lane == 0) S.next = 0;
         __syncwarp();
         visited += n;
-        for (int i = lane; i < n; i += 32) {
-            const DNode N = load_node(nodes, S.frontier[cur][i]);
+        int next = 0;
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            DNode N;
+            float dist[2] = {CUDART_INF_F, CUDART_INF_F};
+            if (i0 + lane < n) {
+                N = load_node(nodes, S.frontier[cur][i0 + lane]);
+                dist[0] = box_distance(c, N.a.x, N.a.y, N.a.z, N.a.w, N.c.x, N.c.y);
+                dist[1] = box_distance(c, N.b.x, N.b.y, N.b.z, N.b.w, N.c.z, N.c.w);
+            }
+#pragma unroll
             for (int w = 0; w < 2; ++w) {
-                const float dist = w == 0 ? box_distance(c, N.a.x, N.a.y, N.a.z, N.a.w, N.c.x, N.c.y)
-                                          : box_distance(c, N.b.x, N.b.y, N.b.z, N.b.w, N.c.z, N.c.w);
-                if (!(dist <= h)) continue;
                 const int child = w == 0 ? N.d.x : N.d.y;
-                if (child >= 0) {
-                    const int k = atomicAdd(&S.next, 1);
-                    if (k < kFrontier) S.frontier[cur ^ 1][k] = child;
-                    continue;
+                const bool in = i0 + lane < n && dist[w] <= h;
+                const unsigned inner = __ballot_sync(0xffffffffu, in && child >= 0);
+                const unsigned leaf = __ballot_sync(0xffffffffu, in && child < 0);
+                if (in) {
+                    const int k = child >= 0 ? next + __popc(inner & before) : leaves + __popc(leaf & before);
+                    if (child >= 0 && k < kFrontier) S.frontier[cur ^ 1][k] = child;
+                    if (child < 0 && k < kCandidates) S.leaf[k] = ~child;
                 }
-                const int first = ~child >> 3, last = first + (~child & 7);
-                for (int s = first; s <= last; ++s) {
-                    const DTri T = load_tri(tris, s);
-                    const float ax = T.v0.x + T.e1.x, bx = T.v0.x + T.e2.x;
-                    const float ay = T.v0.y + T.e1.y, by = T.v0.y + T.e2.y;
-                    const float az = T.v0.z + T.e1.z, bz = T.v0.z + T.e2.z;
-                    const float td = box_distance(
-                        c, fminf(T.v0.x, fminf(ax, bx)), fmaxf(T.v0.x, fmaxf(ax, bx)), fminf(T.v0.y, fminf(ay, by)),
-                        fmaxf(T.v0.y, fmaxf(ay, by)), fminf(T.v0.z, fminf(az, bz)), fmaxf(T.v0.z, fmaxf(az, bz)));
-                    if (!(td <= h)) continue;
-                    const int k = atomicAdd(&S.found, 1);
-                    if (k < kCandidates) {
-                        S.slot[k] = s;
-                        S.dist[k] = td;
-                    }
-                }
+                next += __popc(inner);
+                leaves += __popc(leaf);
             }
         }
-        __syncwarp();
-        n = S.next;
+        n = next;
         cur ^= 1;
-        if (n > kFrontier || S.found > kCandidates) return -1;
-        __syncwarp();
+        if (n > kFrontier || leaves > kCandidates) return -1;
     }
-    return S.found;
+    __syncwarp();
+    for (int i0 = 0; i0 < leaves; i0 += 32) {
+        const int ref = i0 + lane < leaves ? S.leaf[i0 + lane] : 0, count = i0 + lane < leaves ? (ref & 7) + 1 : 0;
+        for (int k = 0; __any_sync(0xffffffffu, k < count); ++k) {
+            const int s = (ref >> 3) + k;
+            float td = CUDART_INF_F;
+            if (k < count) {
+                const DTri T = load_tri(tris, s);
+                const float ax = T.v0.x + T.e1.x, bx = T.v0.x + T.e2.x;
+                const float ay = T.v0.y + T.e1.y, by = T.v0.y + T.e2.y;
+                const float az = T.v0.z + T.e1.z, bz = T.v0.z + T.e2.z;
+                td = box_distance(c, fminf(T.v0.x, fminf(ax, bx)), fmaxf(T.v0.x, fmaxf(ax, bx)),
+                                  fminf(T.v0.y, fminf(ay, by)), fmaxf(T.v0.y, fmaxf(ay, by)),
+                                  fminf(T.v0.z, fminf(az, bz)), fmaxf(T.v0.z, fmaxf(az, bz)));
+            }
+            const bool in = k < count && td <= h;
+            const unsigned mask = __ballot_sync(0xffffffffu, in);
+            const int at = found + __popc(mask & before);
+            if (in && at < kCandidates) {
+                S.slot[at] = s;
+                S.dist[at] = td;
+            }
+            found += __popc(mask);
+        }
+    }
+    __syncwarp();
+    return found > kCandidates ? -1 : found;
 }
 
 // The more than kLocalTris and at most kNearest triangles nearest c (S.near_slot,
 // S.near_dist; their number is returned), or 0 where there are no such. A search down the
 // tree costs 20 us, most of it latency (25 levels of dependent loads), so it takes in up to 1024
 // triangles around a first radius `h` and the radius is then narrowed on their distances:
-// one or two searches for most poses. Searching again until 65 to 192 triangles were in
-// reach, the lists of 96 poses (1 M triangles) took 220 us, now 129; those of 1999 poses
-// (20 k triangles) 228, now 188.
+// one or two searches for most poses. Lists of 96 poses (1 M triangles) took 220 us when
+// the search was repeated until 65 to 192 triangles were in reach and 129 with this; with the
+// leaves after the descent, slots by ballots instead of shared atomics, and ranks and
+// groups in loops that need not wait for their loads, 85. Those of 1999 poses (20 k
+// triangles): 228, 188 and 130.
 __device__ int find_nearest(Search &S, const DNode *__restrict__ nodes, const DTri *__restrict__ tris, f3 c, float h) {
     const int lane = threadIdx.x;
     float lo = 0.f, hi = 0.f;  // too few within lo, too many within hi (0: not known)
@@ -110,22 +129,26 @@ __device__ int find_nearest(Search &S, const DNode *__restrict__ nodes, const DT
         __syncwarp();
     }
     if (n <= kLocalTris) return 0;
-    // bisection for a distance that at most kNearest and more than kLocalTris are within
+    // bisection for a distance that at most kFewNearest and more than kLocalTris are within, or
+    // the nearest to it up to kNearest
     auto within = [&](float t) {
         int m = 0;
         for (int i = lane; i < n; i += 32) m += S.dist[i] <= t;
         return __reduce_add_sync(0xffffffffu, m);
     };
-    float below = 0.f, t = h;
+    float below = 0.f, above = h, t = h;
     int m = n;
-    for (int step = 0; step < 24 && (m > kNearest || m <= kLocalTris); ++step) {
-        const float mid = 0.5f * (below + h);
-        m = within(mid);
-        if (m > kNearest) h = mid;
-        if (m <= kLocalTris) below = mid;
-        t = mid;
+    for (int step = 0; step < 24 && m > kFewNearest; ++step) {
+        const float mid = 0.5f * (below + above);
+        const int k = within(mid);
+        if (k > kLocalTris) {
+            above = t = mid;
+            m = k;
+        } else {
+            below = mid;
+        }
     }
-    if (m > kNearest || m <= kLocalTris) return 0;  // too many at one distance
+    if (m > kNearest) return 0;  // too many at one distance
     int at = 0;
     for (int i = lane; i - lane < n; i += 32) {
         const bool in = i < n && S.dist[i] <= t;
@@ -146,7 +169,11 @@ __device__ __forceinline__ int rank_of(const Search &S, int n, int i) {
     const float di = S.near_dist[i];
     const int si = S.near_slot[i];
     int rank = 0;
-    for (int k = 0; k < n; ++k) rank += S.near_dist[k] < di || (S.near_dist[k] == di && S.near_slot[k] < si);
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) {
+        const float dk = S.near_dist[k];
+        rank += int(dk < di) | (int(dk == di) & int(S.near_slot[k] < si));
+    }
     return rank;
 }
 
@@ -190,32 +217,56 @@ __global__ void __launch_bounds__(32) k_local_build(const PoseJob *__restrict__ 
     for (int j = lane; j < kLocalTris; j += 32) near_plane[j] = local_tri(load_tri(tris, near_slot[j]), c, half).plane;
     __syncwarp();
     // the planes in order of their nearest triangle: each triangle joins the first group
-    // whose plane it shares (a lane compares with the groups l, l + 32, ...)
+    // whose plane it shares. First every triangle's earlier likenesses, as bits (a lane has
+    // the triangles l, l + 32, ...), then which of them lead a group, one after the other.
     constexpr int kPerLane = kLocalTris / 32;
-    static_assert(kLocalTris % 32 == 0 && kLocalTris < 256, "whole lanes of groups, offsets in a byte");
-    int groups = 0, size[kPerLane] = {};
-    for (int j = 0; j < kLocalTris; ++j) {
-        const float4 pl = near_plane[j];
-        int g = groups;
+    static_assert(kLocalTris % 32 == 0 && kLocalTris < 256, "whole lanes of triangles, offsets in a byte");
+    unsigned like[kPerLane][kPerLane] = {};
 #pragma unroll
-        for (int w = kPerLane - 1; w >= 0; --w) {
-            const unsigned same = __ballot_sync(
-                0xffffffffu, lane + 32 * w < groups && local_same_plane(L.plane[lane + 32 * w], pl, half));
-            if (same) g = 32 * w + __ffs(int(same)) - 1;
-        }
-        if (g == groups) {
-            if (lane == 0) {
-                L.plane[g] = pl;
-                L.range[g].y = local_clear(near_dist[j], c);
-            }
-            ++groups;
-        }
-        if (lane == 0) near_group[j] = (unsigned char)g;
+    for (int w = 0; w < kPerLane; ++w) {
+        const float4 mine = near_plane[lane + 32 * w];
 #pragma unroll
-        for (int w = 0; w < kPerLane; ++w)
-            if (lane + 32 * w == g) ++size[w];
-        __syncwarp();
+        for (int v = 0; v <= w; ++v) {
+            unsigned bits = 0;
+#pragma unroll 8
+            for (int i = 0; i < 32; ++i)
+                bits |= unsigned(local_same_plane(near_plane[32 * v + i], mine, half)) << i;
+            like[w][v] = v == w ? bits & ((1u << lane) - 1u) : bits;
+        }
     }
+    unsigned leads[kPerLane] = {};
+    int groups = 0, size[kPerLane] = {};
+#pragma unroll
+    for (int w = 0; w < kPerLane; ++w)
+        for (int i = 0; i < 32; ++i) {
+            int lead = 32 * w + i;  // its own, unless an earlier leader is like it
+#pragma unroll
+            for (int v = w; v >= 0; --v) {
+                const unsigned m = __shfl_sync(0xffffffffu, like[w][v], i) & leads[v];
+                if (m) lead = 32 * v + __ffs(int(m)) - 1;
+            }
+            int g = groups;
+            if (lead == 32 * w + i) {
+                leads[w] |= 1u << i;
+                if (lane == 0) {
+                    L.plane[g] = near_plane[lead];
+                    L.range[g].y = local_clear(near_dist[lead], c);
+                }
+                ++groups;
+            } else {
+                g = 0;
+#pragma unroll
+                for (int v = 0; v < kPerLane; ++v)
+                    g += lead >= 32 * v + 32 ? __popc(leads[v])
+                         : lead >= 32 * v    ? __popc(leads[v] & ((1u << (lead & 31)) - 1u))
+                                             : 0;
+            }
+            if (lane == 0) near_group[32 * w + i] = (unsigned char)g;
+#pragma unroll
+            for (int v = 0; v < kPerLane; ++v)
+                if (lane + 32 * v == g) ++size[v];
+        }
+    __syncwarp();
     // where each group starts, then its triangles
     int total = 0;
 #pragma unroll
