@@ -63,6 +63,16 @@ static hsr_status validate_phase(int32_t phase_mode, int32_t splat_mode) {
     return HSR_OK;
 }
 
+// Whether kernels on this device reach pageable host memory through the host's page tables
+// (the coherent link of a Grace-Blackwell board).
+static bool reaches_host_memory() {
+    int dev = 0, access = 0, tables = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess &&
+           access && tables;
+}
+
 // Per-batch scratch for P poses with N bins, carved from one allocation owned by the scene.
 struct Scratch {
     hsr_antenna *tx, *rx;
@@ -76,7 +86,13 @@ struct Scratch {
     float *rows;
     LocalList *local;    // neighbourhood lists (dense scenes)
     unsigned *counters;  // [0] status word, [2..3] 64-bit work counter
-    bool fresh = false;  // the next pass clears the status word
+    bool fresh = false;  // the next pass clears the status word and takes in what follows
+    // host memory the first pass copies to the device (host_direct), and the budgets there
+    const char *host_src[2] = {nullptr, nullptr};
+    char *host_dst[2] = {nullptr, nullptr};
+    size_t host_bytes[2] = {0, 0};
+    const int64_t *host_budget = nullptr;
+    unsigned *status_out = nullptr;  // where the rows' kernel puts the status word (host_direct)
     size_t bytes;
 };
 
@@ -166,7 +182,7 @@ static hsr_status synthesise(SceneDev &sc, const Scratch &s, int32_t P, float sa
                              int normalise, float *d_out_rows, cudaStream_t st) {
     std::string err;
     if (synth_run(sc.synth, s.fine, P, sc.synth_scratch, g_synth_engine, s.budget, sample_weight, tw, normalise,
-                  d_out_rows, s.counters, st, err) != 0)
+                  d_out_rows, s.counters, s.status_out, st, err) != 0)
         return fail(HSR_ERR_CUDA, err);
     return HSR_OK;
 }
@@ -208,7 +224,12 @@ static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_conf
     const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile : kTile;
     const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     PrepareParams q{};
-    q.budget = s.budget;
+    q.budget = s.fresh && s.host_budget ? s.host_budget : s.budget;
+    for (int k = 0; k < 2 && s.fresh; ++k) {
+        q.copy_src[k] = reinterpret_cast<const uint32_t *>(s.host_src[k]);
+        q.copy_dst[k] = reinterpret_cast<uint32_t *>(s.host_dst[k]);
+        q.copy_words[k] = int64_t(s.host_bytes[k] / 4);
+    }
     q.pose_count = P;
     q.tile = items.samples;
     q.tile_start = s.tile_start;
@@ -307,7 +328,8 @@ static hsr_status run_plain(SceneDev &sc, const Scratch &s, const hsr_rf_config 
                                 PassClear{fine ? nullptr : s.acc, nullptr}, records, max_rec, counters);
     if (r != HSR_OK) return r;
     if (fine) return synthesise(sc, s, P, sample_weight, nullptr, normalise, d_out_rows, st);
-    if (launch_finalize(s.acc, P, N, s.budget, sample_weight, nullptr, normalise, d_out_rows, st) != 0)
+    if (launch_finalize(s.acc, P, N, s.budget, sample_weight, nullptr, normalise, d_out_rows, st, s.counters,
+                        s.status_out) != 0)
         return cuda_fail(cudaGetLastError(), "finalize launch");
     return HSR_OK;
 }
@@ -366,13 +388,17 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
     if (launch_guide_reset(P, g.samp_child, g.samp_p, g.train_child, g.train_acc, g.train_count, st) != 0)
         return cuda_fail(cudaGetLastError(), "guide reset");
     if (K > size_t(kGuideMaxIters)) return fail(HSR_ERR_INVALID_ARGUMENT, "guided budget needs too many iterations");
-    // every iteration's schedule, uploaded once: the iterations then run back to back
+    // every iteration's schedule, uploaded once: the iterations then run back to back. A host
+    // call waits for its passes, so its first one can take the schedule in itself.
+    const bool direct = s.host_src[0] != nullptr;
     const size_t it_bytes = 32 * size_t(P);
-    std::vector<unsigned char> blk(K * it_bytes + 8 * size_t(P));
+    std::vector<char> local_blk, &blk = direct ? sc.stage_sched : local_blk;
+    if (blk.size() < K * it_bytes + 8 * size_t(P)) blk.resize(K * it_bytes + 8 * size_t(P));
+    const size_t blk_bytes = K * it_bytes + 8 * size_t(P);
     std::vector<double> tw(P, 0.0);
     std::vector<char> any_clear(K, 0), any_active(K, 0);
     for (size_t k = 0; k < K; ++k) {
-        unsigned char *h = blk.data() + k * it_bytes;
+        char *h = blk.data() + k * it_bytes;
         int64_t *b = reinterpret_cast<int64_t *>(h);
         int64_t *o = b + P;
         float *w = reinterpret_cast<float *>(o + P);
@@ -403,7 +429,8 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
     }
     std::memcpy(blk.data() + K * it_bytes, tw.data(), 8 * size_t(P));
     const double *d_tw = reinterpret_cast<const double *>(g.sched + K * it_bytes);
-    if ((e = cudaMemcpyAsync(g.sched, blk.data(), blk.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess)
+    if (!direct &&
+        (e = cudaMemcpyAsync(g.sched, blk.data(), blk_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return cuda_fail(e, "schedule upload");
     for (size_t k = 0; k < K; ++k) {
         if (interrupt_flag) {
@@ -421,6 +448,12 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
         si.clear = si.train + P;
         si.active = si.clear + P;
         si.fresh = s.fresh && k == 0;
+        if (direct && k == 0) {  // the first pass takes the whole schedule in
+            si.host_src[1] = blk.data();
+            si.host_dst[1] = reinterpret_cast<char *>(g.sched);
+            si.host_bytes[1] = blk_bytes;
+            si.host_budget = reinterpret_cast<const int64_t *>(blk.data());
+        }
         PassClear clr;
         if (fine) {
             if (any_clear[k] && launch_clear_rows_f(s.fine, P, kFineRowPerBin * N, si.clear, st) != 0)
@@ -437,7 +470,8 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
     if (fine) {
         r = synthesise(sc, s, P, 1.f, d_tw, normalise, d_out_rows, st);
         if (r != HSR_OK) return r;
-    } else if (launch_finalize(s.acc, P, N, s.budget, 1.f, d_tw, normalise, d_out_rows, st) != 0) {
+    } else if (launch_finalize(s.acc, P, N, s.budget, 1.f, d_tw, normalise, d_out_rows, st, s.counters,
+                               s.status_out) != 0) {
         return cuda_fail(cudaGetLastError(), "finalize launch");
     }
     if (h_total_weight)
@@ -468,32 +502,46 @@ static hsr_status read_status(const Scratch &s, cudaStream_t st) {
     return HSR_OK;
 }
 
-// A host call's poses, budgets and offsets in one upload (tx .. offset, or budget .. ff_rx
-// for far-field antennas, lie together in the scratch). The copy has left the staging
-// block when it returns (pageable memory).
-static hsr_status upload_block(SceneDev &sc, char *first, char *last,
+// A host call's poses, budgets and offsets together (tx .. offset, or budget .. ff_rx for
+// far-field antennas, lie together in the scratch): staged in the scene's host memory, from
+// where the call's first pass copies them if the device reaches it, or uploaded at once (the
+// copy has left the staging block when it returns).
+static hsr_status upload_block(SceneDev &sc, Scratch &s, char *first, char *last,
                                std::initializer_list<std::pair<void *, std::pair<const void *, size_t>>> parts,
                                cudaStream_t st) {
     const size_t bytes = size_t(last - first);
+    if (sc.host_in_use) {  // the last call returned early, with its passes in flight
+        cudaDeviceSynchronize();
+        sc.host_in_use = false;
+    }
     if (sc.stage.size() < bytes) sc.stage.resize(bytes);
     for (const auto &p : parts)
         std::memcpy(sc.stage.data() + (static_cast<char *>(p.first) - first), p.second.first, p.second.second);
+    if (sc.host_direct) {
+        sc.host_in_use = true;
+        s.host_src[0] = sc.stage.data();
+        s.host_dst[0] = first;
+        s.host_bytes[0] = bytes;
+        s.host_budget =
+            reinterpret_cast<const int64_t *>(sc.stage.data() + (reinterpret_cast<char *>(s.budget) - first));
+        return HSR_OK;
+    }
     const cudaError_t e = cudaMemcpyAsync(first, sc.stage.data(), bytes, cudaMemcpyHostToDevice, st);
     return e == cudaSuccess ? HSR_OK : cuda_fail(e, "pose upload");
 }
 
-static hsr_status upload_poses(SceneDev &sc, const Scratch &s, int32_t P, const hsr_antenna *tx, const hsr_antenna *rx,
+static hsr_status upload_poses(SceneDev &sc, Scratch &s, int32_t P, const hsr_antenna *tx, const hsr_antenna *rx,
                                const int64_t *budget, const int64_t *offset, cudaStream_t st) {
     const size_t a = sizeof(hsr_antenna) * size_t(P), n = sizeof(int64_t) * size_t(P);
-    return upload_block(sc, reinterpret_cast<char *>(s.tx), reinterpret_cast<char *>(s.offset) + n,
+    return upload_block(sc, s, reinterpret_cast<char *>(s.tx), reinterpret_cast<char *>(s.offset) + n,
                         {{s.tx, {tx, a}}, {s.rx, {rx, a}}, {s.budget, {budget, n}}, {s.offset, {offset, n}}}, st);
 }
 
-static hsr_status upload_poses_ff(SceneDev &sc, const Scratch &s, int32_t P, const hsr_ff_antenna *tx,
+static hsr_status upload_poses_ff(SceneDev &sc, Scratch &s, int32_t P, const hsr_ff_antenna *tx,
                                   const hsr_ff_antenna *rx, const int64_t *budget, const int64_t *offset,
                                   cudaStream_t st) {
     const size_t a = sizeof(hsr_ff_antenna) * size_t(P), n = sizeof(int64_t) * size_t(P);
-    return upload_block(sc, reinterpret_cast<char *>(s.budget), reinterpret_cast<char *>(s.ff_rx) + a,
+    return upload_block(sc, s, reinterpret_cast<char *>(s.budget), reinterpret_cast<char *>(s.ff_rx) + a,
                         {{s.budget, {budget, n}}, {s.offset, {offset, n}}, {s.ff_tx, {tx, a}}, {s.ff_rx, {rx, a}}}, st);
 }
 
@@ -506,19 +554,40 @@ static void use_device_poses(Scratch &s, const hsr_antenna *tx, const hsr_antenn
     s.offset = const_cast<int64_t *>(offset);
 }
 
+constexpr size_t kSmallRows = 256 << 10;  // bytes
+constexpr size_t kRowsHead = 256;         // the status word before them
+
+// Where a host call's rows are written: the scratch, or for small rows the scene's host memory
+// if the device reaches it (with the status word before them).
+static float *rows_target(SceneDev &sc, Scratch &s, size_t floats) {
+    const size_t bytes = kRowsHead + sizeof(float) * floats;
+    if (!sc.host_direct || bytes > kSmallRows) return s.rows;
+    if (sc.stage_rows.size() < bytes) sc.stage_rows.resize(bytes);
+    s.status_out = reinterpret_cast<unsigned *>(sc.stage_rows.data());
+    return reinterpret_cast<float *>(sc.stage_rows.data() + kRowsHead);
+}
+
 // Ends a host call: `floats` of the rows (or of `src`) to the host, then the status. Small
-// rows come with the status word before them in one download.
-static hsr_status fetch_rows(const Scratch &s, float *out, size_t floats, cudaStream_t st,
+// rows come with the status word before them, in one download where they are not in host
+// memory already.
+static hsr_status fetch_rows(SceneDev &sc, const Scratch &s, float *out, size_t floats, cudaStream_t st,
                              const float *src = nullptr) {
-    constexpr size_t kTogether = 256 << 10;
     const size_t bytes = sizeof(float) * floats;
     cudaError_t e;
-    if (!src && bytes <= kTogether) {
+    if (s.status_out) {
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "run");
+        sc.host_in_use = false;
+        std::memcpy(out, sc.stage_rows.data() + kRowsHead, bytes);
+        const unsigned bits = *s.status_out;
+        return bits ? fail(HSR_ERR_DEVICE, status_text(bits)) : HSR_OK;
+    }
+    if (!src && bytes <= kSmallRows) {
         const size_t head = size_t(reinterpret_cast<char *>(s.rows) - reinterpret_cast<char *>(s.counters));
         std::vector<char> host(head + bytes);
         if ((e = cudaMemcpyAsync(host.data(), s.counters, head + bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
             (e = cudaStreamSynchronize(st)) != cudaSuccess)
             return cuda_fail(e, "row download");
+        sc.host_in_use = false;
         unsigned bits;
         std::memcpy(&bits, host.data(), sizeof(bits));
         std::memcpy(out, host.data() + head, bytes);
@@ -527,6 +596,7 @@ static hsr_status fetch_rows(const Scratch &s, float *out, size_t floats, cudaSt
     if ((e = cudaMemcpyAsync(out, src ? src : s.rows, bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
         return cuda_fail(e, "row download");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "run");
+    sc.host_in_use = false;
     return read_status(s, st);
 }
 
@@ -610,6 +680,7 @@ hsr_status hsr_scene_create(const float *vertices, int64_t vertex_count, const i
     SceneDev &d = s->dev;
     cudaGetDevice(&d.device);
     cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, d.device);
+    d.host_direct = reaches_host_memory();
     float *dv = nullptr;
     int32_t *di = nullptr;
     std::string err;
@@ -805,16 +876,6 @@ hsr_status hsr_scene_bvh_stats(const hsr_scene *s, int64_t *out_nodes, int32_t *
     return HSR_OK;
 }
 
-// Whether kernels on this device reach pageable host memory through the host's page tables
-// (the coherent link of a Grace-Blackwell board).
-static bool reaches_host_memory() {
-    int dev = 0, access = 0, tables = 0;
-    return cudaGetDevice(&dev) == cudaSuccess &&
-           cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess &&
-           cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess &&
-           access && tables;
-}
-
 // The caller's arrays are read and written where they are when the device reaches them,
 // otherwise through copies: 1 M rays' 60 MB went over in seven pageable copies, which with
 // the hits' kernel took 4.3 ms for an intersect and a visible call, in place 3.7.
@@ -823,7 +884,7 @@ static hsr_status ray_queries(const hsr_scene *s, int64_t count, const float *o,
     if (!s || count < 0) return fail(HSR_ERR_INVALID_ARGUMENT, "bad scene or count");
     if (count == 0) return HSR_OK;
     if (!o || !d || !tfar) return fail(HSR_ERR_INVALID_ARGUMENT, "null ray arrays");
-    const bool direct = reaches_host_memory();
+    const bool direct = s->dev.host_direct;
     RayQueries q{s->dev.nodes, s->dev.tris, count, o, d, tfar, t, p, n, prim, vis, nullptr};
     // status word, then the copies (floats per ray: 7 in; 1 out, or 8)
     std::string err;
@@ -962,10 +1023,11 @@ hsr_status hsr_backend_run(const hsr_scene *cs, const hsr_rf_config *rf, const h
     cudaStream_t strm = 0;
     if ((st = ensure_scratch(s->dev, 1, N, sc)) != HSR_OK) return st;
     if ((st = upload_poses(s->dev, sc, 1, tx, rx, &budget, &index_offset, strm)) != HSR_OK) return st;
-    st = run_plain(s->dev, sc, rf, N, fl, 1, sample_weight, phase_mode, HSR_SPLAT_DIRICHLET16, 0, sc.rows, strm);
+    st = run_plain(s->dev, sc, rf, N, fl, 1, sample_weight, phase_mode, HSR_SPLAT_DIRICHLET16, 0,
+                   rows_target(s->dev, sc, 2 * size_t(N)), strm);
     if (st != HSR_OK) return st;
     std::vector<float> row(2 * size_t(N));
-    if ((st = fetch_rows(sc, row.data(), row.size(), strm)) != HSR_OK) return st;
+    if ((st = fetch_rows(s->dev, sc, row.data(), row.size(), strm)) != HSR_OK) return st;
     // the reference writes only chirp 0 / channel 0 (path.h:130, 291-292)
     const int C = frame->channelCount;
     for (int32_t k = 0; k < N; ++k) {
@@ -1115,10 +1177,11 @@ hsr_status hsr_backend_run_guided(hsr_scene *s, const hsr_rf_config *rf, const h
     if ((st = enqueue_pass(s->dev, sc, rf, N, &g, 1, sample_weight, false, phase_mode, HSR_SPLAT_DIRICHLET16, strm,
                            &guide->g, PassClear{sc.acc, nullptr})) != HSR_OK)
         return st;
-    if (launch_finalize(sc.acc, 1, N, sc.budget, sample_weight, nullptr, 0, sc.rows, strm) != 0)
+    if (launch_finalize(sc.acc, 1, N, sc.budget, sample_weight, nullptr, 0, rows_target(s->dev, sc, 2 * size_t(N)), strm,
+                        sc.counters, sc.status_out) != 0)
         return cuda_fail(cudaGetLastError(), "finalize launch");
     std::vector<float> row(2 * size_t(N));
-    if ((st = fetch_rows(sc, row.data(), row.size(), strm)) != HSR_OK) return st;
+    if ((st = fetch_rows(s->dev, sc, row.data(), row.size(), strm)) != HSR_OK) return st;
     const int C = frame->channelCount;
     for (int32_t k = 0; k < N; ++k) {
         size_t id = size_t(k) * C;
@@ -1158,10 +1221,10 @@ hsr_status hsr_path_tracer_run(hsr_scene *s, const hsr_rf_config *rf, const hsr_
     if ((st = upload_poses(s->dev, sc, 1, tx, rx, &samples, &zero, strm)) != HSR_OK) return st;
     double tw = 0.0;
     st = run_guided(s->dev, sc, rf, N, fl, 1, std::vector<int64_t>{samples}, std::vector<int64_t>{0}, phase_mode,
-                    HSR_SPLAT_DIRICHLET16, 0, sc.rows, strm, &tw, interrupt_flag);
+                    HSR_SPLAT_DIRICHLET16, 0, rows_target(s->dev, sc, 2 * size_t(N)), strm, &tw, interrupt_flag);
     if (st != HSR_OK) return st;
     std::vector<float> row(2 * size_t(N));
-    if ((st = fetch_rows(sc, row.data(), row.size(), strm)) != HSR_OK) return st;
+    if ((st = fetch_rows(s->dev, sc, row.data(), row.size(), strm)) != HSR_OK) return st;
     const int C = frame->channelCount;
     for (int32_t k = 0; k < N; ++k) {
         size_t id = size_t(k) * C;
@@ -1216,15 +1279,16 @@ hsr_status hsr_simulate_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
     if ((st = ensure_scratch(s->dev, P, N, sc, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
     if ((st = upload_poses(s->dev, sc, P, tx, rx, budget, offset, strm)) != HSR_OK) return st;
+    float *target = rows_target(s->dev, sc, 2 * size_t(P) * N);
     if (!fl->doGuiding) {
-        st = run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, sc.rows, strm);
+        st = run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, target, strm);
     } else {
         st = run_guided(s->dev, sc, rf, N, fl, P, std::vector<int64_t>(budget, budget + P),
-                        std::vector<int64_t>(offset, offset + P), phase_mode, splat_mode, 1, sc.rows, strm, nullptr,
+                        std::vector<int64_t>(offset, offset + P), phase_mode, splat_mode, 1, target, strm, nullptr,
                         nullptr);
     }
     if (st != HSR_OK) return st;
-    return fetch_rows(sc, out_rows, 2 * size_t(P) * N, strm);
+    return fetch_rows(s->dev, sc, out_rows, 2 * size_t(P) * N, strm);
 }
 
 hsr_status hsr_simulate_frame(hsr_scene *s, const hsr_rf_config *rf, const hsr_frame_config *frame,
@@ -1269,7 +1333,7 @@ hsr_status hsr_simulate_frame(hsr_scene *s, const hsr_rf_config *rf, const hsr_f
     float *d_frame = static_cast<float *>(s->dev.frame_buf);
     if (launch_assemble_frame(sc.rows, frame->chirpCount, N, C, d_frame, strm) != 0)
         return cuda_fail(cudaGetLastError(), "frame assembly");
-    return fetch_rows(sc, frame_out, bytes / sizeof(float), strm, d_frame);
+    return fetch_rows(s->dev, sc, frame_out, bytes / sizeof(float), strm, d_frame);
 }
 
 hsr_status hsr_simulate_batch_ff(hsr_scene *s, const hsr_rf_config *rf, int32_t N, const hsr_tracer_flags *fl,
@@ -1292,9 +1356,10 @@ hsr_status hsr_simulate_batch_ff(hsr_scene *s, const hsr_rf_config *rf, int32_t 
     if ((st = ensure_scratch(s->dev, P, N, sc)) != HSR_OK) return st;
     sc.far_field = true;
     if ((st = upload_poses_ff(s->dev, sc, P, tx, rx, budget, offset, strm)) != HSR_OK) return st;
-    st = run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, HSR_SPLAT_DIRICHLET16, 1, sc.rows, strm);
+    st = run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, HSR_SPLAT_DIRICHLET16, 1,
+                   rows_target(s->dev, sc, 2 * size_t(P) * N), strm);
     if (st != HSR_OK) return st;
-    return fetch_rows(sc, out_rows, 2 * size_t(P) * N, strm);
+    return fetch_rows(s->dev, sc, out_rows, 2 * size_t(P) * N, strm);
 }
 
 // ---- autotuning of the plain wavefront launch --------------------------------------

@@ -74,7 +74,11 @@ struct SceneDev {
     // scratch
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
-    std::vector<char> stage;     // host copy of a call's poses and budgets (one upload)
+    // host memory of a call: its poses and budgets, a guided call's schedule, and its rows
+    // where the device writes them there itself (host_direct)
+    std::vector<char> stage, stage_sched, stage_rows;
+    bool host_direct = false;    // kernels reach pageable host memory (hsr_api.cu)
+    bool host_in_use = false;    // a call that uses those blocks has not been waited for
     void *guide = nullptr;       // guiding trees + step scratch, sized for guide_cap poses
     int guide_cap = 0;
     SynthOperand synth;          // cached twiddle operand (fine-histogram synthesis)
@@ -281,8 +285,8 @@ int synth_build_operand(SynthOperand &op, int N, cudaStream_t st, std::string &e
 void synth_free_operand(SynthOperand &op);
 size_t synth_scratch_bytes(const SynthOperand &op, int P);
 int synth_run(const SynthOperand &op, const double *fine, int P, void *scratch, int engine, const int64_t *budget,
-              float sample_weight, const double *tw, int normalise, float *out_rows, unsigned *status, cudaStream_t st,
-              std::string &err);
+              float sample_weight, const double *tw, int normalise, float *out_rows, unsigned *status,
+              unsigned *status_out, cudaStream_t st, std::string &err);
 int launch_clear_rows_f(double *rows, int32_t pose_count, int32_t len, const int *clear, cudaStream_t st);
 // 0: tensor cores (tcgen05, split BF16); 1: CUDA cores (FP32)
 extern int g_synth_engine;
@@ -300,10 +304,16 @@ struct PrepareParams {
     double *rows;           // [pose_count][row_len] accumulators to clear; nullptr: none
     int64_t row_len;
     const int *clear;       // per pose; nullptr: every row
+    // blocks of words to copy (host memory the device reaches, to the device), 0 words: none
+    const uint32_t *copy_src[2];
+    uint32_t *copy_dst[2];
+    int64_t copy_words[2];
 };
 int launch_prepare(const PrepareParams &q, cudaStream_t st);
+// status_out (optional): where the status word goes with the rows.
 int launch_finalize(const double *acc, int32_t pose_count, int32_t samples, const int64_t *budget, float sample_weight,
-                    const double *total_weight, int normalise, float *out_rows, cudaStream_t st);
+                    const double *total_weight, int normalise, float *out_rows, cudaStream_t st,
+                    const unsigned *status = nullptr, unsigned *status_out = nullptr);
 // A MIMO radar cube [chirp][sample][channel] from per-channel rows (hsr_simulate_frame).
 int launch_assemble_frame(const float *rows, int32_t chirps, int32_t samples, int32_t channels, float *frame,
                           cudaStream_t st);

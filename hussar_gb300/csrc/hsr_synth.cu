@@ -426,8 +426,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
 // divided by the pose's total weight
 __global__ void k_synth_finalize(const float *__restrict__ c, int slices, int64_t slice, int P, int N, int ldc,
                                  const int64_t *__restrict__ budget, float sample_weight,
-                                 const double *__restrict__ tw, int normalise, float *__restrict__ out) {
+                                 const double *__restrict__ tw, int normalise, float *__restrict__ out,
+                                 const unsigned *__restrict__ status, unsigned *__restrict__ status_out) {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i == 0 && status_out) *status_out = *status;
     if (i >= int64_t(P) * N) return;
     const int p = int(i / N), m = int(i % N);
     float re = 0.f, im = 0.f;
@@ -579,8 +581,8 @@ size_t synth_scratch_bytes(const SynthOperand &op, int P) {
 
 // fine histograms (P x KK FP64 sums, row stride KK) -> frame rows (P x N complex64)
 int synth_run(const SynthOperand &op, const double *fine, int P, void *scratch, int engine, const int64_t *budget,
-              float sample_weight, const double *tw, int normalise, float *out_rows, unsigned *status, cudaStream_t st,
-              std::string &err) {
+              float sample_weight, const double *tw, int normalise, float *out_rows, unsigned *status,
+              unsigned *status_out, cudaStream_t st, std::string &err) {
     const int Mpad = (P + kBM - 1) / kBM * kBM;
     float *c = static_cast<float *>(scratch);  // the partial slices, [split][Mpad][NCpad]
     const int64_t slice = int64_t(Mpad) * op.NCpad;
@@ -617,7 +619,8 @@ int synth_run(const SynthOperand &op, const double *fine, int P, void *scratch, 
     }
     const int64_t n = int64_t(P) * op.N;
     k_synth_finalize<<<unsigned((n + 255) / 256), 256, 0, st>>>(c, slices, slice, P, op.N, op.NCpad, budget,
-                                                                sample_weight, tw, normalise, out_rows);
+                                                                sample_weight, tw, normalise, out_rows, status,
+                                                                status_out);
     note_launches(1);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -208,14 +208,20 @@ __global__ void __launch_bounds__(256, 2) k_trace(TraceParams p) {
 // What a pass needs set up, in one launch: block 0 forms the work items' prefix over the
 // poses and zeroes the work counter (and the status word); the other blocks clear the
 // accumulator rows of every pose, or of those with clear[pose] != 0 (clearFrame,
-// path.h:147-150). With three memsets, a clearing kernel and a prefix kernel instead (and a
-// copy per array of the call) a pose of 2^14 samples on the dihedral took 97 us, now 83; a
-// guided run of 2^18, 399, now 359.
+// path.h:147-150), and copy in what a call's host memory holds. Bound by the launch and, for
+// the copy, one round trip over the link. With three memsets, a clearing kernel and a prefix
+// kernel instead (and a copy per array of the call) a pose of 2^14 samples on the dihedral
+// took 97 us, with one upload and one download 71, with neither 63; a guided run of 2^18,
+// 399, 364 and 349.
 __global__ void __launch_bounds__(1024) k_prepare(PrepareParams q) {
     const int tid = threadIdx.x;
     if (blockIdx.x > 0) {
-        const int64_t n = int64_t(q.pose_count) * q.row_len, step = int64_t(gridDim.x - 1) * blockDim.x;
-        for (int64_t i = int64_t(blockIdx.x - 1) * blockDim.x + tid; i < n; i += step)
+        const int64_t n = q.rows ? int64_t(q.pose_count) * q.row_len : 0, step = int64_t(gridDim.x - 1) * blockDim.x;
+        const int64_t at = int64_t(blockIdx.x - 1) * blockDim.x + tid;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            for (int64_t i = at; i < q.copy_words[k]; i += step) q.copy_dst[k][i] = q.copy_src[k][i];
+        for (int64_t i = at; i < n; i += step)
             if (!q.clear || q.clear[i / q.row_len]) q.rows[i] = 0.0;
         return;
     }
@@ -257,9 +263,11 @@ __global__ void __launch_bounds__(1024) k_prepare(PrepareParams q) {
 // (plain runs) or the schedule's accumulated weight (total_weight, guided runs)
 __global__ void k_finalize(const double *__restrict__ acc, int32_t pose_count, int32_t samples,
                            const int64_t *__restrict__ budget, float sample_weight,
-                           const double *__restrict__ total_weight, int normalise, float *__restrict__ out) {
+                           const double *__restrict__ total_weight, int normalise, float *__restrict__ out,
+                           const unsigned *__restrict__ status, unsigned *__restrict__ status_out) {
     int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     int64_t n = int64_t(pose_count) * samples;
+    if (i == 0 && status_out) *status_out = *status;
     if (i >= n) return;
     int pose = int(i / samples);
     float re = float(acc[2 * i]), im = float(acc[2 * i + 1]);
@@ -390,7 +398,8 @@ int launch_clear_rows_f(double *rows, int32_t pose_count, int32_t len, const int
 }
 
 int launch_prepare(const PrepareParams &q, cudaStream_t st) {
-    const int64_t n = q.rows ? int64_t(q.pose_count) * q.row_len : 0;
+    const int64_t n =
+        std::max(q.rows ? int64_t(q.pose_count) * q.row_len : 0, std::max(q.copy_words[0], q.copy_words[1]));
     const unsigned clearing = unsigned(std::min<int64_t>((n + 1023) / 1024, 512));
     k_prepare<<<1 + clearing, 1024, 0, st>>>(q);
     note_launches(1);
@@ -398,10 +407,11 @@ int launch_prepare(const PrepareParams &q, cudaStream_t st) {
 }
 
 int launch_finalize(const double *acc, int32_t pose_count, int32_t samples, const int64_t *budget, float sample_weight,
-                    const double *total_weight, int normalise, float *out_rows, cudaStream_t st) {
+                    const double *total_weight, int normalise, float *out_rows, cudaStream_t st,
+                    const unsigned *status, unsigned *status_out) {
     int64_t n = int64_t(pose_count) * samples;
     k_finalize<<<unsigned((n + 255) / 256), 256, 0, st>>>(acc, pose_count, samples, budget, sample_weight,
-                                                           total_weight, normalise, out_rows);
+                                                           total_weight, normalise, out_rows, status, status_out);
     note_launches(1);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
