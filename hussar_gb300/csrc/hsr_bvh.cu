@@ -20,7 +20,7 @@
 //      cheaper than visiting their nodes (k_leaf_cost); the triangle records are reordered so that every
 //      leaf's triangles are contiguous (k_leaf_group, radix sort, k_permute_tris) and
 //      the links of the remaining nodes rewritten (k_relink).
-//   8. the reachable nodes renumbered depth first and the array shrunk to them (host).
+//   8. the reachable nodes renumbered depth first and the array shrunk to them.
 // Node i stores the boxes of both its children; node 0 is the root. A child reference
 // c >= 0 is an internal node; c < 0 a leaf of ((~c) & 7) + 1 triangles from slot
 // (~c) >> 3. A node's first child, when internal, is node i + 1.
@@ -237,6 +237,7 @@ __global__ void k_leaf_depth(int64_t n, const int32_t *__restrict__ parent_inter
 
 // ---------------- PLOC ----------------
 constexpr int kPlocRadius = 256;
+constexpr int kPlocLanes = 8;  // per cluster in k_ploc_nearest
 
 struct Cluster {
     int id;       // node encoding: >= 0 internal node, < 0 leaf slot (~slot)
@@ -265,33 +266,53 @@ __device__ __forceinline__ float merged_area(const float *a, const float *b) {
 }
 
 // nearest[i]: the cluster within +-R whose union with i has the smallest surface area
-// (ties: the lower index), read through a shared-memory window.
+// (ties: the lower index), read through a shared-memory window by eight lanes per cluster.
+// Bound by instruction issue while many clusters are left, then by the window's chain of
+// comparisons, which eight lanes make an eighth as long. One lane per cluster: 114 us at
+// 250 k clusters and 32 us at any count from 500 to 37 k; this 109, 20 at 37 k and 7 from
+// 5 k down (a build of 250 k triangles, 69 iterations: 2.39 -> 0.95 ms).
 __global__ void __launch_bounds__(256) k_ploc_nearest(int n, const Cluster *__restrict__ cl, int *__restrict__ nearest) {
-    __shared__ float sb[256 + 2 * kPlocRadius][6];
-    const int base = blockIdx.x * 256;
-    for (int k = threadIdx.x; k < 256 + 2 * kPlocRadius; k += 256) {
+    constexpr int L = kPlocLanes, kClusters = 256 / L, kRows = kClusters + 2 * kPlocRadius;
+    __shared__ float2 sb[kRows][3];
+    const int base = blockIdx.x * kClusters;
+    for (int k = threadIdx.x; k < kRows; k += 256) {
         const int j = base - kPlocRadius + k;
         if (j >= 0 && j < n) {
 #pragma unroll
-            for (int a = 0; a < 6; ++a) sb[k][a] = cl[j].b[a];
+            for (int a = 0; a < 3; ++a) sb[k][a] = make_float2(cl[j].b[2 * a], cl[j].b[2 * a + 1]);
         }
     }
     __syncthreads();
-    const int i = base + threadIdx.x;
-    if (i >= n) return;
-    const float *bi = sb[threadIdx.x + kPlocRadius];
+    const int own = threadIdx.x / L, lane = threadIdx.x % L, i = base + own;
     float best = __int_as_float(0x7f800000);
     int bj = -1;
-    const int j0 = max(0, i - kPlocRadius), j1 = min(n - 1, i + kPlocRadius);
-    for (int j = j0; j <= j1; ++j) {
-        if (j == i) continue;
-        const float a = merged_area(bi, sb[j - base + kPlocRadius]);
-        if (a < best) {
+    if (i < n) {
+        const float2 *si = sb[own + kPlocRadius];
+        const float bi[6] = {si[0].x, si[0].y, si[1].x, si[1].y, si[2].x, si[2].y};
+        const int j0 = max(0, i - kPlocRadius), j1 = min(n - 1, i + kPlocRadius);
+#pragma unroll 4
+        for (int j = j0 + lane; j <= j1; j += L) {
+            if (j == i) continue;
+            const float2 *sj = sb[j - base + kPlocRadius];
+            const float2 u = sj[0], v = sj[1], w = sj[2];
+            const float bb[6] = {u.x, u.y, v.x, v.y, w.x, w.y};
+            const float a = merged_area(bi, bb);
+            if (a < best) {
+                best = a;
+                bj = j;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o /= 2) {
+        const float a = __shfl_xor_sync(~0u, best, o);
+        const int j = __shfl_xor_sync(~0u, bj, o);
+        if (a < best || (a == best && unsigned(j) < unsigned(bj))) {
             best = a;
             bj = j;
         }
     }
-    nearest[i] = bj;
+    if (i < n && lane == 0) nearest[i] = bj;
 }
 
 // Mutual nearest pairs merge into a new internal node (allocated from the top so that the
@@ -525,10 +546,9 @@ __global__ void k_reins_init(int m, const DNode *__restrict__ nodes, const int32
     tree[i] = reins_node(box_union(child_box(nd, 0), child_box(nd, 1)), k[0], k[1]);
 }
 
-// Depth of every node (the root 0) and the deepest leaf; bad: a parent chain that does not
-// end at node 0 within the bound.
-__global__ void k_reins_depth(int total, int m, const int *__restrict__ rpar, int *depth, int *max_depth,
-                              int *bad) {
+// The deepest leaf (the root's depth is 0); bad: a parent chain that does not end at node 0
+// within the bound.
+__global__ void k_reins_depth(int total, int m, const int *__restrict__ rpar, int *max_depth, int *bad) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     int d = 0, x = i;
@@ -536,7 +556,6 @@ __global__ void k_reins_depth(int total, int m, const int *__restrict__ rpar, in
         x = rpar[x];
         ++d;
     }
-    depth[i] = d;
     if (x != 0 || d >= 1024) atomicOr(bad, 1);
     if (i >= m) atomicMax(max_depth, d);
 }
@@ -551,8 +570,9 @@ __global__ void k_reins_depth(int total, int m, const int *__restrict__ rpar, in
 // larger than n would not pay.
 // A best-first search of the same space from the root, with the removal's shrunk boxes and
 // a 384-entry heap in local memory (5.8 KB per thread), visited fewer nodes but took 2.4 ms
-// per pass on 250 k triangles; this one 0.39 (0.65 with the descent as a loop inside the
-// climb), to trees of the same node visits per ray (boxes 126, urban 18.6).
+// per pass on 250 k triangles; this one 0.37 (0.39 with a stack of nodes whose children a
+// visit has to look up first, 0.65 with the descent as a loop inside the climb), to trees of
+// the same node visits per ray (boxes 126, urban 18.6).
 __global__ void __launch_bounds__(128) k_reins_search(int total, const int *__restrict__ rpar,
                                                       const ReinsNode *__restrict__ tree, float min_gain, int *mv_x,
                                                       float *mv_gain) {
@@ -569,8 +589,8 @@ __global__ void __launch_bounds__(128) k_reins_search(int total, const int *__re
     const int S = pn.kx == n ? pn.ky : pn.kx;
     float saved = box_area(box_of(pn)), best = min_gain;
     int bx = -1, visits = 0;
-    int stack[kReinsStack];
-    float grown[kReinsStack];
+    int2 stack[kReinsStack];  // an open node's children: known when it is opened, so that a
+    float grown[kReinsStack]; // visit waits for one load only
     int sp = 0;
     // node x as a place under ancestors that grow by d; its own growth added to d tells
     // whether its subtree is opened
@@ -585,35 +605,34 @@ __global__ void __launch_bounds__(128) k_reins_search(int total, const int *__re
         d += au - box_area(b);
         return t.kx >= 0;
     };
-    auto open = [&](int x, float d) {
+    auto open = [&](const ReinsNode &t, float d) {
         if (sp < kReinsStack && saved - d - an > best) {
-            stack[sp] = x;
+            stack[sp] = make_int2(t.kx, t.ky);
             grown[sp++] = d;
         }
     };
     const ReinsNode sn = reins_load(tree, S);
     Box cur = box_of(sn);  // the path's box without n
-    if (sn.kx >= 0) open(S, saved - box_area(cur));  // below the sibling (beside it is where n is)
+    if (sn.kx >= 0) open(sn, saved - box_area(cur));  // below the sibling (beside it is where n is)
     int child = P, y = G, steps = 0;
     float saved_next = saved;  // `saved` once the open subtrees are done
     // one loop for both kinds of step, so that a lane that climbs does not wait for one that
     // descends
     while (true) {
         if (sp > 0 && visits < kReinsVisits) {
-            const int x = stack[--sp];
+            const int2 t = stack[--sp];
             const float d = grown[sp];
             if (!(saved - d - an > best)) continue;
             ++visits;
-            const ReinsNode t = reins_load(tree, x);
-            const ReinsNode l = reins_load(tree, t.kx), r = reins_load(tree, t.ky);
+            const ReinsNode l = reins_load(tree, t.x), r = reins_load(tree, t.y);
             float dl = d, dr = d;
-            const bool kl = consider(t.kx, l, dl), kr = consider(t.ky, r, dr);
+            const bool kl = consider(t.x, l, dl), kr = consider(t.y, r, dr);
             if (dl < dr) {
-                if (kr) open(t.ky, dr);
-                if (kl) open(t.kx, dl);
+                if (kr) open(r, dr);
+                if (kl) open(l, dl);
             } else {
-                if (kl) open(t.kx, dl);
-                if (kr) open(t.ky, dr);
+                if (kl) open(l, dl);
+                if (kr) open(r, dr);
             }
             continue;
         }
@@ -632,7 +651,7 @@ __global__ void __launch_bounds__(128) k_reins_search(int total, const int *__re
         const int c = yn.kx == child ? yn.ky : yn.kx;
         const ReinsNode cn = reins_load(tree, c);
         float d = 0.f;
-        if (consider(c, cn, d)) open(c, d);
+        if (consider(c, cn, d)) open(cn, d);
         cur = box_union(cur, box_of(cn));
         saved_next = saved + (box_area(box_of(yn)) - box_area(cur));
         child = y;
@@ -773,27 +792,57 @@ int g_bvh_builder = 0;  // 0: PLOC, 1: LBVH (Karras)
 int g_bvh_leaf_max = 4;  // triangles per leaf (1..8)
 int g_bvh_optimize = 32;  // largest number of insertion passes after the build (0: none)
 
+// The temporaries of one stage of the build, in one allocation (each piece on a 256-byte
+// boundary). With one each, 47 allocations and their releases took 2.3 ms of a build of
+// 250 k triangles.
+struct Temps {
+    void *block = nullptr;
+    std::vector<std::pair<void **, size_t>> parts;
+    template <typename T> void want(T **p, size_t bytes) {
+        parts.emplace_back(reinterpret_cast<void **>(p), (bytes + 255) & ~size_t(255));
+    }
+    bool get(std::string &err) {
+        size_t sum = 0;
+        for (const auto &q : parts) sum += q.second;
+        if (!dev_alloc(&block, sum, err)) return false;
+        char *at = static_cast<char *>(block);
+        for (const auto &q : parts) {
+            *q.first = at;
+            at += q.second;
+        }
+        return true;
+    }
+    ~Temps() { cudaFree(block); }
+};
+
 // Insertion passes over the binary tree of a build (par_i/par_l and the DNodes, leaves
 // referenced as ~slot); stops when a pass moves fewer than 1 in 20,000 nodes (stopping
-// at 1 in 4,000 left the urban scene 8 % more node visits per ray). Returns 0
+// at 1 in 4,000 left the urban scene 8 % more node visits per ray; searching every node in the
+// first and last passes only and a quarter of the rest between built 250 k triangles in 18.8
+// ms instead of 23.1, to trees in which the urban frame took 0-8 % longer). Returns 0
 // (also when the result failed its checks and the build's tree was kept), 2 or 3.
 static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l, cudaStream_t st,
                          std::string &err) {
     if (g_bvh_optimize <= 0 || nt < 4 || nt >= (int64_t(1) << 30)) return 0;
     const int m = int(nt - 1), total = int(2 * nt - 1);
-    int *rpar = nullptr, *depth = nullptr, *mv_x = nullptr, *counters = nullptr, *scal = nullptr;
+    int *rpar = nullptr, *mv_x = nullptr, *counters = nullptr, *scal = nullptr;
     ReinsNode *tree = nullptr;
     float *mv_gain = nullptr;
     unsigned long long *lock = nullptr;
     char *moving = nullptr, *keep = nullptr;
     int rc = 0;
+    Temps t;
     do {
-        if (!dev_alloc(&rpar, sizeof(int) * total, err) || !dev_alloc(&depth, sizeof(int) * total, err) ||
-            !dev_alloc(&mv_x, sizeof(int) * total, err) || !dev_alloc(&counters, sizeof(int) * m, err) ||
-            !dev_alloc(&scal, sizeof(int) * 4, err) || !dev_alloc(&tree, sizeof(ReinsNode) * total, err) ||
-            !dev_alloc(&mv_gain, sizeof(float) * total, err) ||
-            !dev_alloc(&lock, sizeof(unsigned long long) * total, err) || !dev_alloc(&moving, size_t(total), err) ||
-            !dev_alloc(&keep, size_t(total), err)) {
+        t.want(&rpar, sizeof(int) * total);
+        t.want(&mv_x, sizeof(int) * total);
+        t.want(&counters, sizeof(int) * m);
+        t.want(&scal, sizeof(int) * 4);
+        t.want(&tree, sizeof(ReinsNode) * total);
+        t.want(&mv_gain, sizeof(float) * total);
+        t.want(&lock, sizeof(unsigned long long) * total);
+        t.want(&moving, size_t(total));
+        t.want(&keep, size_t(total));
+        if (!t.get(err)) {
             rc = 3;
             break;
         }
@@ -814,14 +863,13 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
             cudaMemsetAsync(scal, 0, sizeof(int) * 4, st);
             cudaMemsetAsync(lock, 0, sizeof(unsigned long long) * total, st);
             cudaMemsetAsync(counters, 0, sizeof(int) * m, st);
-            k_reins_depth<<<blocks_for(total, T), T, 0, st>>>(total, m, rpar, depth, scal + 2, scal + 1);
             k_reins_search<<<blocks_for(total, 128), 128, 0, st>>>(total, rpar, tree, min_gain, mv_x, mv_gain);
             k_reins_lock<<<blocks_for(total, T), T, 0, st>>>(total, rpar, tree, mv_x, mv_gain, lock);
             k_reins_claim<<<blocks_for(total, T), T, 0, st>>>(total, rpar, tree, mv_x, mv_gain, lock, moving);
             k_reins_keep<<<blocks_for(total, T), T, 0, st>>>(total, rpar, mv_x, moving, keep);
             k_reins_apply<<<blocks_for(total, T), T, 0, st>>>(total, rpar, tree, mv_x, keep, scal);
             k_reins_refit<<<blocks_for(nt, T), T, 0, st>>>(total, m, rpar, tree, counters, scal + 1);
-            note_launches(7);
+            note_launches(6);
             if (cudaMemcpyAsync(h, scal, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess) {
                 err = "BVH optimisation pass failed";
@@ -830,9 +878,10 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
             }
             if (h[1] || h[0] < std::max(1, total / 20000)) break;
         }
-        if (rc || h[1]) break;  // a failed check keeps the build's own tree
+        // a failed check keeps the build's own tree (every loop of a pass is bounded on any links)
+        if (rc || h[1]) break;
         cudaMemsetAsync(scal, 0, sizeof(int) * 4, st);
-        k_reins_depth<<<blocks_for(total, T), T, 0, st>>>(total, m, rpar, depth, scal + 2, scal + 1);
+        k_reins_depth<<<blocks_for(total, T), T, 0, st>>>(total, m, rpar, scal + 2, scal + 1);
         note_launches(1);
         if (cudaMemcpyAsync(h, scal, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
@@ -848,16 +897,6 @@ static int optimize_tree(SceneDev &s, int64_t nt, int32_t *par_i, int32_t *par_l
             rc = 2;
         }
     } while (false);
-    cudaFree(rpar);
-    cudaFree(depth);
-    cudaFree(mv_x);
-    cudaFree(counters);
-    cudaFree(scal);
-    cudaFree(tree);
-    cudaFree(mv_gain);
-    cudaFree(lock);
-    cudaFree(moving);
-    cudaFree(keep);
     return rc;
 }
 
@@ -875,14 +914,28 @@ static int collapse_leaves(SceneDev &s, int64_t nt, const int32_t *par_i, const 
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
     int rc = 0;
+    Temps t;
     do {
-        if (!dev_alloc(&count, sizeof(int) * n_nodes, err) || !dev_alloc(&cost, sizeof(float) * n_nodes, err) ||
-            !dev_alloc(&collapse, size_t(n_nodes), err) || !dev_alloc(&is_root, size_t(n_nodes), err) ||
-            !dev_alloc(&group_min, sizeof(int) * n_nodes, err) || !dev_alloc(&start, sizeof(int) * n_nodes, err) ||
-            !dev_alloc(&group, sizeof(int32_t) * nt, err) || !dev_alloc(&ids, sizeof(int32_t) * nt, err) ||
-            !dev_alloc(&ids2, sizeof(int32_t) * nt, err) || !dev_alloc(&new_slot, sizeof(int32_t) * nt, err) ||
-            !dev_alloc(&keys, sizeof(uint64_t) * nt, err) || !dev_alloc(&keys2, sizeof(uint64_t) * nt, err) ||
-            !dev_alloc(&tris2, sizeof(DTri) * nt, err)) {
+        if (cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, ids, ids2, int(nt), 0, 64, st) !=
+            cudaSuccess) {
+            err = "leaf sort size query failed";
+            rc = 2;
+            break;
+        }
+        t.want(&tmp, tmp_bytes);
+        t.want(&count, sizeof(int) * n_nodes);
+        t.want(&cost, sizeof(float) * n_nodes);
+        t.want(&collapse, size_t(n_nodes));
+        t.want(&is_root, size_t(n_nodes));
+        t.want(&group_min, sizeof(int) * n_nodes);
+        t.want(&start, sizeof(int) * n_nodes);
+        t.want(&group, sizeof(int32_t) * nt);
+        t.want(&ids, sizeof(int32_t) * nt);
+        t.want(&ids2, sizeof(int32_t) * nt);
+        t.want(&new_slot, sizeof(int32_t) * nt);
+        t.want(&keys, sizeof(uint64_t) * nt);
+        t.want(&keys2, sizeof(uint64_t) * nt);
+        if (!t.get(err) || !dev_alloc(&tris2, sizeof(DTri) * nt, err)) {
             rc = 3;
             break;
         }
@@ -902,13 +955,6 @@ static int collapse_leaves(SceneDev &s, int64_t nt, const int32_t *par_i, const 
                                                        is_root);
         k_leaf_keys<<<blocks_for(nt, T), T, 0, st>>>(nt, group, group_min, keys, ids);
         note_launches(2);
-        if (cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, ids, ids2, int(nt), 0, 64, st) !=
-                cudaSuccess ||
-            !dev_alloc(&tmp, tmp_bytes, err)) {
-            if (err.empty()) err = "leaf sort size query failed";
-            rc = tmp ? 2 : 3;
-            break;
-        }
         if (cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, ids, ids2, int(nt), 0, 64, st) !=
             cudaSuccess) {
             err = "leaf sort failed";
@@ -927,20 +973,7 @@ static int collapse_leaves(SceneDev &s, int64_t nt, const int32_t *par_i, const 
         }
         std::swap(s.tris, tris2);
     } while (false);
-    cudaFree(count);
-    cudaFree(cost);
-    cudaFree(collapse);
-    cudaFree(is_root);
-    cudaFree(group_min);
-    cudaFree(start);
-    cudaFree(group);
-    cudaFree(ids);
-    cudaFree(ids2);
-    cudaFree(new_slot);
-    cudaFree(keys);
-    cudaFree(keys2);
     cudaFree(tris2);
-    cudaFree(tmp);
     return rc;
 }
 
@@ -954,15 +987,17 @@ static int build_ploc(SceneDev &s, int64_t nt, const int32_t *ids2, const float 
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
     int rc = 0;
+    Temps t;
     do {
-        if (!dev_alloc(&c0, sizeof(Cluster) * n0, err) || !dev_alloc(&c1, sizeof(Cluster) * n0, err) ||
-            !dev_alloc(&nearest, sizeof(int) * n0, err) || !dev_alloc(&counter, sizeof(int) * 2, err) ||
-            !dev_alloc(&num_sel, sizeof(int) * 2, err) || !dev_alloc(&keep, size_t(n0), err)) {
-            rc = 3;
-            break;
-        }
         cub::DeviceSelect::Flagged(nullptr, tmp_bytes, c0, keep, c1, num_sel, n0, st);
-        if (!dev_alloc(&tmp, tmp_bytes, err)) {
+        t.want(&tmp, tmp_bytes);
+        t.want(&c0, sizeof(Cluster) * n0);
+        t.want(&c1, sizeof(Cluster) * n0);
+        t.want(&nearest, sizeof(int) * n0);
+        t.want(&counter, sizeof(int) * 2);
+        t.want(&num_sel, sizeof(int) * 2);
+        t.want(&keep, size_t(n0));
+        if (!t.get(err)) {
             rc = 3;
             break;
         }
@@ -972,7 +1007,7 @@ static int build_ploc(SceneDev &s, int64_t nt, const int32_t *ids2, const float 
         int n = n0;
         int iterations = 0;
         while (n > 1 && iterations < 100000) {
-            k_ploc_nearest<<<blocks_for(n, 256), 256, 0, st>>>(n, c0, nearest);
+            k_ploc_nearest<<<blocks_for(n, 256 / kPlocLanes), 256, 0, st>>>(n, c0, nearest);
             k_ploc_merge<<<blocks_for(n, 256), 256, 0, st>>>(n, nearest, c0, keep, s.nodes, counter, n0 - 1, par_i,
                                                              par_l);
             if (cub::DeviceSelect::Flagged(tmp, tmp_bytes, c0, keep, c1, num_sel, n, st) != cudaSuccess) {
@@ -1002,13 +1037,6 @@ static int build_ploc(SceneDev &s, int64_t nt, const int32_t *ids2, const float 
         note_launches(1);
     } while (false);
     cudaStreamSynchronize(st);
-    cudaFree(c0);
-    cudaFree(c1);
-    cudaFree(nearest);
-    cudaFree(counter);
-    cudaFree(num_sel);
-    cudaFree(keep);
-    cudaFree(tmp);
     return rc;
 }
 
@@ -1180,17 +1208,31 @@ int bvh_build(SceneDev &s, const float *d_v, int64_t nv, const int32_t *d_idx, i
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
     int rc = 0;
+    Temps t;
     auto fail = [&](int code) {
         rc = code;
         return code;
     };
     do {
-        if (!dev_alloc(&lo, sizeof(float) * 3 * nt, err) || !dev_alloc(&hi, sizeof(float) * 3 * nt, err) ||
-            !dev_alloc(&cb, sizeof(unsigned) * 6, err) || !dev_alloc(&keys, sizeof(uint64_t) * nt, err) ||
-            !dev_alloc(&keys2, sizeof(uint64_t) * nt, err) || !dev_alloc(&ids, sizeof(int32_t) * nt, err) ||
-            !dev_alloc(&ids2, sizeof(int32_t) * nt, err) || !dev_alloc(&par_i, sizeof(int32_t) * n_nodes, err) ||
-            !dev_alloc(&par_l, sizeof(int32_t) * nt, err) || !dev_alloc(&counters, sizeof(int) * n_nodes, err) ||
-            !dev_alloc(&depth, sizeof(int) * 2, err)) {
+        if (cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, ids, ids2, (int)nt, 0, 63, st) !=
+            cudaSuccess) {
+            err = "radix sort size query failed";
+            fail(2);
+            break;
+        }
+        t.want(&tmp, tmp_bytes);
+        t.want(&lo, sizeof(float) * 3 * nt);
+        t.want(&hi, sizeof(float) * 3 * nt);
+        t.want(&cb, sizeof(unsigned) * 6);
+        t.want(&keys, sizeof(uint64_t) * nt);
+        t.want(&keys2, sizeof(uint64_t) * nt);
+        t.want(&ids, sizeof(int32_t) * nt);
+        t.want(&ids2, sizeof(int32_t) * nt);
+        t.want(&par_i, sizeof(int32_t) * n_nodes);
+        t.want(&par_l, sizeof(int32_t) * nt);
+        t.want(&counters, sizeof(int) * n_nodes);
+        t.want(&depth, sizeof(int) * 2);
+        if (!t.get(err)) {
             fail(3);
             break;
         }
@@ -1203,16 +1245,6 @@ int bvh_build(SceneDev &s, const float *d_v, int64_t nv, const int32_t *d_idx, i
         k_bounds<<<blocks_for(nt, T), T, 0, st>>>(d_v, d_idx, nt, lo, hi, cb);
         k_morton<<<blocks_for(nt, T), T, 0, st>>>(lo, hi, nt, cb, keys, ids);
         note_launches(2);
-        if (cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, ids, ids2, (int)nt, 0, 63, st) !=
-            cudaSuccess) {
-            err = "radix sort size query failed";
-            fail(2);
-            break;
-        }
-        if (!dev_alloc(&tmp, tmp_bytes, err)) {
-            fail(3);
-            break;
-        }
         if (cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, ids, ids2, (int)nt, 0, 63, st) !=
             cudaSuccess) {
             err = "radix sort failed";
@@ -1269,18 +1301,6 @@ int bvh_build(SceneDev &s, const float *d_v, int64_t nv, const int32_t *d_idx, i
             break;
         }
     } while (false);
-    cudaFree(lo);
-    cudaFree(hi);
-    cudaFree(cb);
-    cudaFree(keys);
-    cudaFree(keys2);
-    cudaFree(ids);
-    cudaFree(ids2);
-    cudaFree(par_i);
-    cudaFree(par_l);
-    cudaFree(counters);
-    cudaFree(depth);
-    cudaFree(tmp);
     return rc;
 }
 
