@@ -204,7 +204,7 @@ static hsr_status ensure_guide(SceneDev &sc, int P, GuideMem &out) {
     return HSR_OK;
 }
 
-static constexpr int32_t kTile = 4096;  // most samples a CTA takes at once
+static constexpr int32_t kTile = 4096;  // samples per work item of k_trace
 
 // The accumulator rows a pass starts from zero: none, all (poses null), or those flagged.
 struct PassClear {
@@ -221,7 +221,7 @@ static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_conf
                                unsigned long long *counters = nullptr) {
     const bool wave = g_path_kernel == 0 && fl->useGeometricalOptics && !records && !counters;
     const bool tuned = !fl->doGuiding;
-    const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile : kTile;
+    const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile : wave ? kWaveTile : kTile;
     const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     PrepareParams q{};
     q.budget = s.fresh && s.host_budget ? s.host_budget : s.budget;
@@ -1448,7 +1448,7 @@ hsr_status hsr_autotune_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
     // the serving ticks read the scene's tuned threshold to pick their path stack
     if (best.queue_threshold <= 0) best.queue_threshold = kWaveMaxQueueThreshold;
     d.tuned = best;
-    out_best->tile = best.tile > 0 ? best.tile : kTile;
+    out_best->tile = best.tile > 0 ? best.tile : kWaveTile;
     out_best->ctas_per_sm = best.ctas_per_sm;
     out_best->queue_threshold = best.queue_threshold;
     out_best->field_on_hit = best.field_on_hit;

@@ -42,10 +42,11 @@ constexpr int kWaveDefaultQueue = 128;       // thresholds up to 128, guided, fa
 constexpr int kWaveSmallQueue = 64;          // thresholds up to this run with a 320-entry stack
 constexpr int kWaveLocalQueue = 128;         // launches with neighbourhood lists: 384 entries
 // The work items of a wavefront launch whose tile (the most samples a CTA takes at once;
-// 4096 where none was chosen) is `tile`: one GENERATE stage each, pulled in runs of up to a
+// kWaveTile where none was chosen) is `tile`: one GENERATE stage each, pulled in runs of up to a
 // tile that shrink towards the end of the launch (pull_items in hsr_wave.cuh). A tile that
 // is no multiple of the stage is pulled whole.
 constexpr int32_t kWaveItem = 256;
+constexpr int32_t kWaveTile = 16384;
 struct WaveItems {
     int32_t samples;  // TraceParams::tile
     int32_t run;      // TraceParams::item_run

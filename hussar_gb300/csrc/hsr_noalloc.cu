@@ -130,10 +130,10 @@ extern "C" hsr_status hsr_simulate_batch_device_noalloc(hsr_scene *scene, const 
     // must not be destroyed while this call's work is in flight
     std::lock_guard<std::mutex> lk(*scene_mutex(scene));
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
-    // the scene's tuned tile where it has one, else 4096 samples (the prefix holds
+    // the scene's tuned tile where it has one, else the default (the prefix holds
     // pose_count + 1 entries whatever the tile)
     const bool wave = g_path_kernel == 0 && flags->useGeometricalOptics != 0;
-    const int32_t tile = sc->tuned.tile > 0 ? sc->tuned.tile : 4096;
+    const int32_t tile = sc->tuned.tile > 0 ? sc->tuned.tile : wave ? kWaveTile : 4096;
     const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     int64_t *tile_start = reinterpret_cast<int64_t *>(s->tile_start);
     PrepareParams q{};

@@ -240,7 +240,7 @@ __device__ __forceinline__ float chirp_bandwidth(const hsr_rf_config &rf) { retu
 
 // Pulls the run of work items a CTA takes next: [S.item, S.item_end), empty (false) once
 // the counter has passed `total`. With p.item_run = 0 it is one item. With p.item_run = R
-// it is half the CTA's share of what is left, between 1 and R items (guided
+// it is a third of the CTA's share of what is left, between 1 and R items (guided
 // self-scheduling, Polychronopoulos and Kuck 1987): long runs of one pose while there is
 // plenty, which drain the path stack and flush the row rarely, and single 256-sample items
 // at the end, so that the CTAs finish together. What is left is estimated from the CTA's
@@ -252,12 +252,17 @@ __device__ __forceinline__ float chirp_bandwidth(const hsr_rf_config &rf) { retu
 // 100 k triangles of boxes (1.7 M samples) 21.9 -> 12.2 ms; 27 far-field poses x 2^14
 // 747 -> 480 us; urban, 12 x 2^19 samples, 8.3 -> 7.3 ms; 96 poses on 1 M triangles (14 M
 // samples) 101 -> 91 ms.
+// A CTA that changes pose drains its stack and reads the next pose's list, so runs are as
+// long as the balance allows: half the share was too much for poses that differ in cost
+// (96 boxes poses of 2^13 .. 2^18 samples 14.4 ms with R = 64 items; a third 12.7, a quarter
+// 12.8, a sixth 13.1), and R = 16 items too little for large batches (256 boxes poses of
+// 2^16 .. 2^22 samples 0.88e9 paths/s, R = 32 1.04e9, R = 64 1.20e9, R = 256 1.20e9).
 template <class Shared>
 __device__ __forceinline__ bool pull_items(const TraceParams &p, Shared &S, long long total) {
     long long want = 1;
     if (p.item_run > 0) {
         const long long left = total - S.item_end - S.item_want * (long long)gridDim.x;
-        want = min((long long)p.item_run, max(1ll, left / (2ll * gridDim.x)));
+        want = min((long long)p.item_run, max(1ll, left / (3ll * gridDim.x)));
         S.item_want = int(want);
     }
     S.item = (long long)atomicAdd((unsigned long long *)p.work_counter, (unsigned long long)want);
