@@ -2,11 +2,10 @@
 // default, path.h:156): the same per-path arithmetic as the one-thread-per-sample
 // kernel, reorganised so that warps stay converged.
 //
-// A persistent CTA of 256 threads keeps a stack of up to 384 live path states in
-// shared memory (four CTAs per SM: 64 registers; ~32 KB of shared memory each plus the
-// range row, so that four CTAs leave about 90 KB of the SM's L1 to the BVH) and
-// alternates two stages:
-//   GENERATE  (at most 128 live paths, or the autotuned queue threshold): 256 new
+// A persistent CTA of 256 threads keeps a stack of up to 512 live path states in
+// shared memory (four CTAs per SM: 64 registers; 27 to 43 KB of shared memory each plus the
+// range row; the rest of the SM's 256 KB is L1 for the BVH) and alternates two stages:
+//   GENERATE  (at most 256 live paths, or the queue threshold of the launch): 256 new
 //             samples, one per thread: Halton point,
 //             antenna ray, closest hit; paths that hit something are pushed.
 //   EXTEND    (otherwise): 256 paths popped, one per thread: specular reflection,
@@ -44,7 +43,7 @@ constexpr int kPrimaryCells = 8;
 // paths left when GENERATE runs (the queue threshold). Three capacities are built: 384
 // entries (thresholds up to 128), 320 (up to 64), whose 5 KB less shared
 // memory per CTA leaves more of the SM's L1 to the BVH (4 % on the dense boxes scenes,
-// which the autotuner runs at threshold 32 or 64), and 512 (up to 256), whose fuller
+// before their neighbourhood lists), and 512 (up to 256), whose fuller
 // EXTEND stages pay where the BVH stays in L1 anyway (7 % on the sphere bench).
 template <int kCap> struct WaveShared {
     float ox[kCap], oy[kCap], oz[kCap];  // hit point (origin of the next segment)
