@@ -876,15 +876,20 @@ hsr_status hsr_scene_bvh_stats(const hsr_scene *s, int64_t *out_nodes, int32_t *
     return HSR_OK;
 }
 
-// The caller's arrays are read and written where they are when the device reaches them,
-// otherwise through copies: 1 M rays' 60 MB went over in seven pageable copies, which with
-// the hits' kernel took 4.3 ms for an intersect and a visible call, in place 3.7.
+// The caller's arrays are read and written where they are when the device reaches them and
+// they allow it (usable_in_place), otherwise through copies: 1 M rays' 60 MB went over in
+// seven pageable copies, which with the hits' kernel took 4.3 ms for an intersect and a
+// visible call, in place 3.7.
 static hsr_status ray_queries(const hsr_scene *s, int64_t count, const float *o, const float *d, const float *tfar,
                               float *t, float *p, float *n, int32_t *prim, int32_t *vis) {
     if (!s || count < 0) return fail(HSR_ERR_INVALID_ARGUMENT, "bad scene or count");
     if (count == 0) return HSR_OK;
     if (!o || !d || !tfar) return fail(HSR_ERR_INVALID_ARGUMENT, "null ray arrays");
-    const bool direct = s->dev.host_direct;
+    const size_t words = sizeof(float) * size_t(count);
+    const bool direct =
+        s->dev.host_direct &&
+        usable_in_place({{o, 3 * words, 4}, {d, 3 * words, 4}, {tfar, words, 4}},
+                        {{t, words, 4}, {p, 3 * words, 4}, {n, 3 * words, 4}, {prim, words, 4}, {vis, words, 4}});
     RayQueries q{s->dev.nodes, s->dev.tris, count, o, d, tfar, t, p, n, prim, vis, nullptr};
     // status word, then the copies (floats per ray: 7 in; 1 out, or 8)
     std::string err;

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -53,6 +54,32 @@ struct WaveItems {
 };
 inline WaveItems wave_items(int32_t tile) {
     return tile % kWaveItem == 0 ? WaveItems{kWaveItem, tile / kWaveItem} : WaveItems{tile, 0};
+}
+
+// A caller's array and what its elements are aligned to where a kernel reads or writes them.
+struct CallerArray {
+    const void *at;  // null: not given
+    size_t bytes, align;
+};
+// Whether kernels may use a caller's arrays where they are. A misaligned access is a fault of
+// the GPU, where a copy takes any address; and a result that overlaps an input or another
+// result would change what later threads read, where copied inputs are what the call was given.
+inline bool usable_in_place(std::initializer_list<CallerArray> in, std::initializer_list<CallerArray> out) {
+    const auto at = [](const CallerArray &a) { return reinterpret_cast<uintptr_t>(a.at); };
+    const auto aligned = [&](const CallerArray &a) { return at(a) % a.align == 0; };
+    const auto apart = [&](const CallerArray &a, const CallerArray &b) {
+        return !a.at || !b.at || at(a) + a.bytes <= at(b) || at(b) + b.bytes <= at(a);
+    };
+    for (const CallerArray &r : in)
+        if (!aligned(r)) return false;
+    for (const CallerArray &w : out) {
+        if (!aligned(w)) return false;
+        for (const CallerArray &r : in)
+            if (!apart(w, r)) return false;
+        for (const CallerArray &o : out)
+            if (&o != &w && !apart(w, o)) return false;
+    }
+    return true;
 }
 
 // A resident scene: triangles + BVH on the device, plus per-scene scratch reused by
