@@ -278,6 +278,13 @@ class BatchGraph:
             pass
 
 
+def _check_rays(n, directions, tfar):
+    """The device reads n directions and limits where they lie: past the end of a shorter array
+    that is memory it may not reach."""
+    if len(directions) < n or tfar.size < n:
+        raise ValueError("%d origins with %d directions and %d limits" % (n, len(directions), tfar.size))
+
+
 class _GB300:
     """Namespace mirroring hussar::gb300 (the drop-in for hussar::cpu / hussar::gpu)."""
 
@@ -385,6 +392,7 @@ class _GB300:
             d = np.ascontiguousarray(directions, np.float32).reshape(-1, 3)
             n = len(o)
             tf = np.full(n, np.inf, np.float32) if tfar is None else np.ascontiguousarray(tfar, np.float32)
+            _check_rays(n, d, tf)
             t = np.empty(n, np.float32)
             p = np.empty((n, 3), np.float32)
             nn = np.empty((n, 3), np.float32)
@@ -398,6 +406,7 @@ class _GB300:
             o = np.ascontiguousarray(origins, np.float32).reshape(-1, 3)
             d = np.ascontiguousarray(directions, np.float32).reshape(-1, 3)
             tf = np.ascontiguousarray(tfar, np.float32).reshape(-1)
+            _check_rays(len(o), d, tf)
             vis = np.empty(len(o), np.int32)
             _lib.check(_lib.lib().hsr_visible(self._scene, len(o), _lib.ptr(o), _lib.ptr(d), _lib.ptr(tf),
                                                _lib.ptr(vis)))
