@@ -129,10 +129,11 @@ class FFAntenna:
 
 
 def _pack(antennas, count, cls, struct, columns):
-    """`count` C structures (float fields only) of a sequence of antennas, as a float32 array:
+    """`count` C structures (float fields only) of an iterable of antennas, as a float32 array:
     the columns of all of them at once where each is a plain `cls`, its to_c() otherwise;
-    zeros where the sequence is shorter. Two thousand poses' TX and RX take 0.8 ms, a ctypes
+    zeros where there are fewer. Two thousand poses' TX and RX take 0.8 ms, a ctypes
     structure filled for each 9."""
+    antennas = list(antennas)
     if len(antennas) > count:
         raise IndexError("%d antennas for %d poses" % (len(antennas), count))
     out = np.zeros((count, ctypes.sizeof(struct) // 4), np.float32)
@@ -159,12 +160,12 @@ def _ff_columns(rows, antennas):
 
 
 def _antenna_array(antennas, count):
-    """hsr_antenna[count] of a sequence of NFAntenna."""
+    """hsr_antenna[count] of an iterable of NFAntenna."""
     return _pack(antennas, count, NFAntenna, _lib.AntennaC, _nf_columns)
 
 
 def _ff_antenna_array(antennas, count):
-    """hsr_ff_antenna[count] of a sequence of FFAntenna."""
+    """hsr_ff_antenna[count] of an iterable of FFAntenna."""
     return _pack(antennas, count, FFAntenna, _lib.FfAntennaC, _ff_columns)
 
 
