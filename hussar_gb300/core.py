@@ -128,17 +128,17 @@ class FFAntenna:
         return a
 
 
-def _pack(antennas, count, cls, struct, columns):
+def _pack(antennas, count, cls, struct, columns, regular=lambda antennas: True):
     """`count` C structures (float fields only) of an iterable of antennas, as a float32 array:
-    the columns of all of them at once where each is a plain `cls`, its to_c() otherwise;
-    zeros where there are fewer. Two thousand poses' TX and RX take 0.8 ms, a ctypes
-    structure filled for each 9."""
+    the columns of all of them at once where each is a plain `cls` and they are `regular`,
+    to_c() of each otherwise; zeros where there are fewer. Two thousand poses' TX and RX take
+    0.8 ms, a ctypes structure filled for each 9."""
     antennas = list(antennas)
     if len(antennas) > count:
         raise IndexError("%d antennas for %d poses" % (len(antennas), count))
     out = np.zeros((count, ctypes.sizeof(struct) // 4), np.float32)
     rows = out[:len(antennas)]
-    if len(antennas) and all(type(a) is cls for a in antennas):
+    if len(antennas) and all(type(a) is cls for a in antennas) and regular(antennas):
         columns(rows, antennas)
     else:
         for row, a in zip(rows, antennas):
@@ -159,6 +159,13 @@ def _ff_columns(rows, antennas):
     rows[:, 12] = [a.radius for a in antennas]
 
 
+def _ff_regular(antennas):
+    """Whether every antenna's vectors, which its user may have set, are as its constructor makes
+    them: side by side, one of another length would shift those after it."""
+    return all(getattr(v, "shape", None) == (3,) for a in antennas
+               for v in (a.direction, a.polarization, a.scene_center))
+
+
 def _antenna_array(antennas, count):
     """hsr_antenna[count] of an iterable of NFAntenna."""
     return _pack(antennas, count, NFAntenna, _lib.AntennaC, _nf_columns)
@@ -166,7 +173,7 @@ def _antenna_array(antennas, count):
 
 def _ff_antenna_array(antennas, count):
     """hsr_ff_antenna[count] of an iterable of FFAntenna."""
-    return _pack(antennas, count, FFAntenna, _lib.FfAntennaC, _ff_columns)
+    return _pack(antennas, count, FFAntenna, _lib.FfAntennaC, _ff_columns, _ff_regular)
 
 
 class Scene:

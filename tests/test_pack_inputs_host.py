@@ -17,3 +17,21 @@ def test_any_iterable(wrap):
     assert core._ff_antenna_array(wrap(far), 5).tobytes() == core._ff_antenna_array(far, 5).tobytes()
     with pytest.raises(IndexError):
         core._antenna_array(wrap(nf), 4)
+
+
+@pytest.mark.parametrize("field", ["direction", "polarization", "scene_center"])
+def test_vectors_of_another_length_are_refused(field):
+    """Two antennas whose lengths are off by opposite amounts fill as many floats as two good ones."""
+    far = ff(4)
+    setattr(far[1], field, getattr(far[1], field)[:2])
+    setattr(far[2], field, np.concatenate([getattr(far[2], field), getattr(far[2], field)[:1]]))
+    with pytest.raises(ValueError):
+        core._ff_antenna_array(far, 4)
+
+
+def test_vectors_as_lists():
+    far = ff(4)
+    want = core._ff_antenna_array(far, 4).tobytes()
+    for a in far[1:3]:
+        a.direction, a.scene_center = a.direction.tolist(), a.scene_center.tolist()
+    assert core._ff_antenna_array(far, 4).tobytes() == want
