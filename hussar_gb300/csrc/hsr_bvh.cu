@@ -1044,13 +1044,15 @@ namespace {
 
 // Nodes of every subtree, from the nodes with two leaves up: the second of two internal
 // children to arrive goes on. Climbs out of a collapsed leaf end where the parent no longer
-// refers to the node.
+// refers to the node. A tree can be as deep as it has nodes (triangles on one place merge one
+// by one, and a tree that deep keeps no insertion pass), so that bounds the climb; at any
+// depth it is one visit per node.
 __global__ void k_tree_sizes(int64_t n, const DNode *__restrict__ nodes, const int32_t *__restrict__ par_i, int *size,
                              int *arrived) {
     const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (t >= n || nodes[t].d.x >= 0 || nodes[t].d.y >= 0) return;
     int i = int(t), s = 1;
-    for (int steps = 0; steps < 1024; ++steps) {
+    for (int64_t steps = 0; steps < n; ++steps) {
         __stcg(&size[i], s);
         if (i == 0) return;
         const int p = par_i[i];
@@ -1069,6 +1071,8 @@ __global__ void k_tree_sizes(int64_t n, const DNode *__restrict__ nodes, const i
 
 // A reachable node's place in depth-first order: a first child follows its parent, a second
 // one its sibling's subtree; summed over the path to the root. placed: how many there were.
+// The climbs add up to half the depth squared on a chain, as k_leaf_depth's do; one of 20,000
+// triangles on one place builds in 0.81 s, with the host's walk it took 1.31.
 __global__ void k_tree_place(int64_t n, const DNode *__restrict__ nodes, const int32_t *__restrict__ par_i,
                              const int *__restrict__ size, int64_t out_count, DNode *__restrict__ out, int *placed) {
     const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -1076,9 +1080,9 @@ __global__ void k_tree_place(int64_t n, const DNode *__restrict__ nodes, const i
     auto first = [&](const int4 &d) { return d.x >= 0 ? size[d.x] : 0; };
     int64_t id = 0;
     int c = int(t);
-    for (int steps = 0; c != 0; ++steps) {
+    for (int64_t steps = 0; c != 0; ++steps) {
         const int p = par_i[c];
-        if (p < 0 || steps >= 1024) return;
+        if (p < 0 || steps >= n) return;
         const int4 d = nodes[p].d;
         if (d.x == c)
             id += 1;
