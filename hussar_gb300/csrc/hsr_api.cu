@@ -204,7 +204,19 @@ static hsr_status ensure_guide(SceneDev &sc, int P, GuideMem &out) {
     return HSR_OK;
 }
 
-static constexpr int32_t kTile = 4096;  // samples per work item of k_trace
+static constexpr int32_t kTile = 4096;  // samples per work item of k_trace, at most
+
+// Samples per work item of a guided k_trace pass over `samples`: about four items per resident
+// CTA, as k_trace pulls its items one by one (k_wave's runs shrink by themselves). The
+// schedule's first pass is 2^14 samples, four items of kTile for 304 CTAs: guided runs of the
+// dihedral without geometrical optics, of 2^16, 2^18 and 2^20 samples, took 0.27, 2.5 and 9.3
+// ms with kTile, with this 0.14, 0.49 and 2.4.
+static int32_t guided_trace_tile(const SceneDev &sc, int64_t samples) {
+    const int64_t per_item = (samples + 8 * int64_t(sc.sm_count) - 1) / (8 * int64_t(sc.sm_count));
+    int32_t tile = 256;
+    while (tile < kTile && tile < per_item) tile *= 2;
+    return tile;
+}
 
 // The accumulator rows a pass starts from zero: none, all (poses null), or those flagged.
 struct PassClear {
@@ -213,15 +225,19 @@ struct PassClear {
 };
 
 // One trace launch over the poses' current budgets/offsets/weights in scratch.
-// The autotuned tile, CTAs per SM and queue threshold apply to plain passes.
+// The autotuned tile, CTAs per SM and queue threshold apply to plain passes; guided ones say
+// how many samples they have (guided_samples).
 static hsr_status enqueue_pass(SceneDev &sc, const Scratch &s, const hsr_rf_config *rf, int32_t N,
                                const hsr_tracer_flags *fl, int32_t P, float sample_weight, bool per_pose_weights,
                                int32_t phase_mode, int32_t splat_mode, cudaStream_t st, const GuideMem *g,
-                               const PassClear &clr, void *records = nullptr, int max_rec = 0,
+                               int64_t guided_samples, const PassClear &clr, void *records = nullptr, int max_rec = 0,
                                unsigned long long *counters = nullptr) {
     const bool wave = g_path_kernel == 0 && fl->useGeometricalOptics && !records && !counters;
     const bool tuned = !fl->doGuiding;
-    const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile : wave ? kWaveTile : kTile;
+    const int32_t tile = tuned && sc.tuned.tile > 0 ? sc.tuned.tile
+                         : wave                     ? kWaveTile
+                         : tuned                    ? kTile
+                                                    : guided_trace_tile(sc, guided_samples);
     const WaveItems items = wave ? wave_items(tile) : WaveItems{tile, 0};
     PrepareParams q{};
     q.budget = s.fresh && s.host_budget ? s.host_budget : s.budget;
@@ -324,7 +340,7 @@ static hsr_status run_plain(SceneDev &sc, const Scratch &s, const hsr_rf_config 
     }
     hsr_tracer_flags plain = *fl;
     plain.doGuiding = 0;
-    hsr_status r = enqueue_pass(sc, s, rf, N, &plain, P, sample_weight, false, phase_mode, splat_mode, st, nullptr,
+    hsr_status r = enqueue_pass(sc, s, rf, N, &plain, P, sample_weight, false, phase_mode, splat_mode, st, nullptr, 0,
                                 PassClear{fine ? nullptr : s.acc, nullptr}, records, max_rec, counters);
     if (r != HSR_OK) return r;
     if (fine) return synthesise(sc, s, P, sample_weight, nullptr, normalise, d_out_rows, st);
@@ -397,6 +413,7 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
     const size_t blk_bytes = K * it_bytes + 8 * size_t(P);
     std::vector<double> tw(P, 0.0);
     std::vector<char> any_clear(K, 0), any_active(K, 0);
+    std::vector<int64_t> iter_samples(K, 0);
     for (size_t k = 0; k < K; ++k) {
         char *h = blk.data() + k * it_bytes;
         int64_t *b = reinterpret_cast<int64_t *>(h);
@@ -417,6 +434,7 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
                 if (it.clear) tw[p] = 0.0;
                 tw[p] += double(it.budget) * double(it.weight);  // path.h:445, 466-475
                 active[p] = k + 1 < sched[p].size() ? 1 : 0;
+                iter_samples[k] += it.budget;
             } else {
                 b[p] = 0;
                 o[p] = 0;
@@ -461,7 +479,7 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
         } else if (k == 0 || any_clear[k]) {
             clr = PassClear{s.acc, k == 0 ? nullptr : si.clear};
         }
-        r = enqueue_pass(sc, si, rf, N, fl, P, 1.f, true, phase_mode, splat_mode, st, &g, clr);
+        r = enqueue_pass(sc, si, rf, N, fl, P, 1.f, true, phase_mode, splat_mode, st, &g, iter_samples[k], clr);
         if (r != HSR_OK) return r;
         if (any_active[k] &&
             launch_guide_step(P, si.active, g.samp_child, g.samp_p, g.train_child, g.train_acc, g.train_count, st) != 0)
@@ -1180,7 +1198,7 @@ hsr_status hsr_backend_run_guided(hsr_scene *s, const hsr_rf_config *rf, const h
     hsr_tracer_flags g = *fl;
     g.doGuiding = 1;
     if ((st = enqueue_pass(s->dev, sc, rf, N, &g, 1, sample_weight, false, phase_mode, HSR_SPLAT_DIRICHLET16, strm,
-                           &guide->g, PassClear{sc.acc, nullptr})) != HSR_OK)
+                           &guide->g, budget, PassClear{sc.acc, nullptr})) != HSR_OK)
         return st;
     if (launch_finalize(sc.acc, 1, N, sc.budget, sample_weight, nullptr, 0, rows_target(s->dev, sc, 2 * size_t(N)), strm,
                         sc.counters, sc.status_out) != 0)
