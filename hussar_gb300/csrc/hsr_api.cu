@@ -1470,13 +1470,14 @@ hsr_status hsr_autotune_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
         d.tuned = saved;
         return st;
     }
-    // store the shape explicitly: a threshold of 0 means "the default" to the kernel, but
-    // the serving ticks read the scene's tuned threshold to pick their path stack
-    if (best.queue_threshold <= 0) best.queue_threshold = kWaveMaxQueueThreshold;
+    // the caller gets the shape in numbers; the scene keeps the zeros of the default, which
+    // stand for another shape at another number of bins (the serving ticks tell a scene whose
+    // default won from one never tuned by default_queue)
+    best.default_queue = wave_default_queue(N, false);
     d.tuned = best;
-    out_best->tile = best.tile > 0 ? best.tile : kWaveTile;
+    out_best->tile = best.tile > 0 ? best.tile : g_path_kernel == 0 ? kWaveTile : kTile;
     out_best->ctas_per_sm = best.ctas_per_sm;
-    out_best->queue_threshold = best.queue_threshold;
+    out_best->queue_threshold = best.queue_threshold > 0 ? best.queue_threshold : best.default_queue;
     out_best->field_on_hit = best.field_on_hit;
     out_best->coherent_order = best.coherent_order;
     out_best->trace_ms = best_ms;
@@ -1507,7 +1508,8 @@ hsr_status hsr_get_launch_config(const hsr_scene *s, hsr_launch_config *out) {
     if (!s || !out) return fail(HSR_ERR_INVALID_ARGUMENT, "null argument");
     out->tile = s->dev.tuned.tile;
     out->ctas_per_sm = s->dev.tuned.ctas_per_sm;
-    out->queue_threshold = s->dev.tuned.queue_threshold;
+    const LaunchConfig &t = s->dev.tuned;
+    out->queue_threshold = t.queue_threshold > 0 ? t.queue_threshold : t.default_queue;
     out->field_on_hit = s->dev.tuned.field_on_hit;
     out->coherent_order = s->dev.tuned.coherent_order;
     out->trace_ms = 0.f;

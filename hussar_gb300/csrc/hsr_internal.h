@@ -36,12 +36,22 @@ struct LaunchConfig {
     int32_t queue_threshold = 0;  // see TraceParams::queue_threshold
     int32_t field_on_hit = 0;     // see TraceParams::field_on_hit
     int32_t coherent_order = 0;   // see TraceParams::coherent_order
+    // what queue_threshold 0 stood for in the batch the autotuner timed (0: not its choice).
+    // The threshold itself stays 0 where the default won: it depends on a launch's bins
+    int32_t default_queue = 0;
 };
 // wavefront path stacks: 256 + the GENERATE threshold entries; three capacities
 constexpr int kWaveMaxQueueThreshold = 256;  // above 128, and threshold 0: the 512-entry stack
 constexpr int kWaveDefaultQueue = 128;       // thresholds up to 128, guided, far-field: 384 entries
 constexpr int kWaveSmallQueue = 64;          // thresholds up to this run with a 320-entry stack
 constexpr int kWaveLocalQueue = 128;         // launches with neighbourhood lists: 384 entries
+// The GENERATE threshold a launch takes where none was chosen (0): 256, whose fuller stages
+// take 5 % off the sphere (725 -> 690 us at 2^22 samples) and 1.5 % off the urban frame; dense
+// scenes, which want the L1 instead, have a form of their own. Guided launches, whose stack
+// holds more per path, and long rows keep 128 (256 would leave three CTAs per SM).
+inline int32_t wave_default_queue(int32_t samples, bool guided) {
+    return guided || samples > 1536 ? kWaveDefaultQueue : kWaveMaxQueueThreshold;
+}
 // The work items of a wavefront launch whose tile (the most samples a CTA takes at once;
 // kWaveTile where none was chosen) is `tile`: one GENERATE stage each, pulled in runs of up to a
 // tile that shrink towards the end of the launch (pull_items in hsr_wave.cuh). A tile that

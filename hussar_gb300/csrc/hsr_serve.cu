@@ -472,8 +472,11 @@ bool hsr_server::build_tick(TickSlot &t, bool busy, int64_t &ticks_launched) {
             }
             tile[P + 1] = tile[P] + (chunk[i] + items.samples - 1) / items.samples;
             maxN = std::max(maxN, q->r.samples_per_chirp);
-            queue_threshold = std::min(queue_threshold, std::max(q->scene->tuned.queue_threshold, kWaveSmallQueue));
-            if (q->scene->tuned.queue_threshold <= kWaveSmallQueue) queue_threshold = kWaveSmallQueue;
+            const LaunchConfig &tuned = q->scene->tuned;
+            const int32_t threshold = tuned.queue_threshold > 0  ? tuned.queue_threshold
+                                      : tuned.default_queue > 0 ? wave_default_queue(q->r.samples_per_chirp, guided)
+                                                                : kWaveSmallQueue;
+            queue_threshold = std::min(queue_threshold, std::max(threshold, kWaveSmallQueue));
             coherent = coherent && q->scene->tuned.coherent_order != 0;
             ++P;
             q->scheduled += chunk[i];

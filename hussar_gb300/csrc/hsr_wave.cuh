@@ -707,12 +707,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave(TraceParams p) {
 }
 
 // The stack capacity (as its GENERATE threshold) a launch with threshold q runs: 64 for
-// 1..64, 128 for 65..128, 256 above. The default (q = 0) is 256, whose fuller stages take
-// 5 % off the sphere (725 -> 690 us at 2^22 samples) and 1.5 % off the urban frame; dense
-// scenes, which want the L1 instead, have a form of their own. Guided launches, whose stack
-// holds more per path, and long rows keep 128 (256 would leave three CTAs per SM).
+// 1..64, 128 for 65..128, 256 above; 0 takes wave_default_queue.
 inline int wave_capacity(int32_t q, int32_t samples, bool guided) {
-    if (q == 0) q = guided || samples > 1536 ? kWaveDefaultQueue : kWaveMaxQueueThreshold;
+    if (q == 0) q = wave_default_queue(samples, guided);
     return q <= kWaveSmallQueue ? kWaveSmallQueue : q > kWaveDefaultQueue ? kWaveMaxQueueThreshold : kWaveDefaultQueue;
 }
 
