@@ -1450,18 +1450,22 @@ hsr_status hsr_autotune_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
         if ((st = trial(c, ms)) != HSR_OK) break;
         if (better()) best_ms = ms, best = c;
     }
-    for (int32_t k = 0; st == HSR_OK && k < 4; ++k) {
+    // launches with neighbourhood lists have one path stack, which holds the two largest
+    // thresholds alike, and neither of the last two forms: a trial of those would measure noise
+    // (5 % on a small batch) and the scene's launches without lists would run what it chose
+    const bool lists = sc.local && g_path_kernel == 0;
+    for (int32_t k = 0; st == HSR_OK && k < (lists ? 2 : 4); ++k) {
         LaunchConfig c = best;
         c.queue_threshold = thresholds[k];
         if ((st = trial(c, ms)) != HSR_OK) break;
         if (better()) best_ms = ms, best = c;
     }
-    if (st == HSR_OK) {  // the primary field formed on a hit (pays where most primaries miss)
+    if (st == HSR_OK && !lists) {  // the primary field formed on a hit (pays where most primaries miss)
         LaunchConfig c = best;
         c.field_on_hit = 1;
         if ((st = trial(c, ms)) == HSR_OK && better()) best_ms = ms, best = c;
     }
-    if (st == HSR_OK) {  // coherent stage order (pays where traversal dominates)
+    if (st == HSR_OK && !lists) {  // coherent stage order (pays where traversal dominates)
         LaunchConfig c = best;
         c.coherent_order = 1;
         if ((st = trial(c, ms)) == HSR_OK && better()) best_ms = ms, best = c;
@@ -1473,7 +1477,7 @@ hsr_status hsr_autotune_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, 
     // the caller gets the shape in numbers; the scene keeps the zeros of the default, which
     // stand for another shape at another number of bins (the serving ticks tell a scene whose
     // default won from one never tuned by default_queue)
-    best.default_queue = wave_default_queue(N, false);
+    best.default_queue = lists ? kWaveLocalQueue : wave_default_queue(N, false);
     d.tuned = best;
     out_best->tile = best.tile > 0 ? best.tile : g_path_kernel == 0 ? kWaveTile : kTile;
     out_best->ctas_per_sm = best.ctas_per_sm;

@@ -432,6 +432,8 @@ hsr_status hsr_debug_sincos_sweep(float lo, float hi, int64_t *out_checked, int6
  * holds at most this many live paths; at most 256: thresholds up to 64 run a 320-entry
  * path stack, up to 128 a 384-entry one, above 128 a 512-entry one). Zero fields mean
  * the default shape (tile 16384, threshold 256; 128 for chirps of over 1536 samples).
+ * Scenes dense enough for neighbourhood lists run one 384-entry stack (thresholds up to
+ * 128) without the two forms that follow.
  * field_on_hit = 1 forms a primary ray's antenna field
  * only once the ray has hit something (for indirect-only paths: the field of a ray that
  * misses is never used), which pays where most primary rays miss and costs registers
