@@ -172,6 +172,10 @@ extern "C" hsr_status hsr_simulate_batch_device_noalloc(hsr_scene *scene, const 
     if (wave) {
         if (sc->tuned.ctas_per_sm > 0) per_sm = std::min(per_sm, sc->tuned.ctas_per_sm);
         p.queue_threshold = sc->tuned.queue_threshold;
+        // this call has no neighbourhood lists, and a dense scene's tree wants the L1 that the
+        // default's larger path stack takes: 24 poses of 2^15 samples on 1 M triangles of boxes
+        // 7.2 ms with that, 5.9 with the smaller one; of 2^13 on 20 k 1.87 and 1.65 ms
+        if (p.queue_threshold == 0 && sc->local_radius > 0.f) p.queue_threshold = kWaveDefaultQueue;
         p.field_on_hit = sc->tuned.field_on_hit;
         p.coherent_order = sc->tuned.coherent_order;
     }
