@@ -563,13 +563,27 @@ static hsr_status upload_poses_ff(SceneDev &sc, Scratch &s, int32_t P, const hsr
                         {{s.budget, {budget, n}}, {s.offset, {offset, n}}, {s.ff_tx, {tx, a}}, {s.ff_rx, {rx, a}}}, st);
 }
 
-// Poses that are on the device already are read where they are.
-static void use_device_poses(Scratch &s, const hsr_antenna *tx, const hsr_antenna *rx, const int64_t *budget,
-                             const int64_t *offset) {
-    s.tx = const_cast<hsr_antenna *>(tx);
-    s.rx = const_cast<hsr_antenna *>(rx);
-    s.budget = const_cast<int64_t *>(budget);
-    s.offset = const_cast<int64_t *>(offset);
+// Poses that are on the device already are read where they are to the end of the call, or
+// copied first where rows written over them would change what is read, or kernels can't
+// use them at their addresses.
+static hsr_status use_device_poses(Scratch &s, int32_t P, int32_t N, const hsr_antenna *tx, const hsr_antenna *rx,
+                                   const int64_t *budget, const int64_t *offset, const float *rows, cudaStream_t st) {
+    const size_t a = sizeof(hsr_antenna) * size_t(P), n = sizeof(int64_t) * size_t(P);
+    const size_t r = sizeof(float) * 2 * size_t(P) * size_t(N);
+    if (usable_in_place({{tx, a, 4}, {rx, a, 4}, {budget, n, 8}, {offset, n, 8}}, {{rows, r, 4}})) {
+        s.tx = const_cast<hsr_antenna *>(tx);
+        s.rx = const_cast<hsr_antenna *>(rx);
+        s.budget = const_cast<int64_t *>(budget);
+        s.offset = const_cast<int64_t *>(offset);
+        return HSR_OK;
+    }
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(s.tx, tx, a, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(s.rx, rx, a, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(s.budget, budget, n, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(s.offset, offset, n, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+        return cuda_fail(e, "pose copy");
+    return HSR_OK;
 }
 
 constexpr size_t kSmallRows = 256 << 10;  // bytes
@@ -1271,7 +1285,7 @@ hsr_status hsr_simulate_batch_device(hsr_scene *s, const hsr_rf_config *rf, int3
     Scratch sc;
     cudaStream_t strm = static_cast<cudaStream_t>(stream);
     if ((st = ensure_scratch(s->dev, P, N, sc, splat_mode == HSR_SPLAT_FINE_SYNTH)) != HSR_OK) return st;
-    use_device_poses(sc, d_tx, d_rx, d_budget, d_offset);
+    if ((st = use_device_poses(sc, P, N, d_tx, d_rx, d_budget, d_offset, d_out_rows, strm)) != HSR_OK) return st;
     if (!fl->doGuiding)
         return run_plain(s->dev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, d_out_rows, strm);
     // the guided schedule is planned on the host: it reads the budgets back (synchronising)
@@ -1710,7 +1724,6 @@ hsr_status hsr_batch_graph_create(hsr_scene *s, const hsr_rf_config *rf, int32_t
         }
     }
     Scratch sc = carve(g->scratch, P, N, fine, local);
-    use_device_poses(sc, d_tx, d_rx, d_budget, d_offset);
     g->status = sc.counters;
     cudaStream_t cs = nullptr;
     if ((e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking)) != cudaSuccess) {
@@ -1721,7 +1734,8 @@ hsr_status hsr_batch_graph_create(hsr_scene *s, const hsr_rf_config *rf, int32_t
     if ((e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) {
         rst = cuda_fail(e, "begin capture");
     } else {
-        rst = run_plain(gdev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, d_out_rows, cs);
+        rst = use_device_poses(sc, P, N, d_tx, d_rx, d_budget, d_offset, d_out_rows, cs);
+        if (rst == HSR_OK) rst = run_plain(gdev, sc, rf, N, fl, P, 1.f, phase_mode, splat_mode, 1, d_out_rows, cs);
         cudaGraph_t graph = nullptr;
         e = cudaStreamEndCapture(cs, &graph);
         g->graph = graph;
