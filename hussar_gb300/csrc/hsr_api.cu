@@ -405,10 +405,12 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
         return cuda_fail(cudaGetLastError(), "guide reset");
     if (K > size_t(kGuideMaxIters)) return fail(HSR_ERR_INVALID_ARGUMENT, "guided budget needs too many iterations");
     // every iteration's schedule, uploaded once: the iterations then run back to back. A host
-    // call waits for its passes, so its first one can take the schedule in itself.
+    // call waits for its passes, so its first one can take the schedule in itself. In either
+    // form it is the scene's memory that is read, after this returns too: the caller has
+    // begun staging, and ends it once the stream has been waited for.
     const bool direct = s.host_src[0] != nullptr;
     const size_t it_bytes = 32 * size_t(P);
-    std::vector<char> local_blk, &blk = direct ? sc.stage_sched : local_blk;
+    std::vector<char> &blk = sc.stage_sched;
     if (blk.size() < K * it_bytes + 8 * size_t(P)) blk.resize(K * it_bytes + 8 * size_t(P));
     const size_t blk_bytes = K * it_bytes + 8 * size_t(P);
     std::vector<double> tw(P, 0.0);
@@ -520,23 +522,26 @@ static hsr_status read_status(const Scratch &s, cudaStream_t st) {
     return HSR_OK;
 }
 
+// A call is about to write the scene's host blocks. They may still be read: by the passes of
+// a call that returned early, or by the copy that uploads one (from pageable memory it need
+// not be done when it returns).
+static void begin_staging(SceneDev &sc) {
+    if (sc.host_in_use) cudaDeviceSynchronize();
+    sc.host_in_use = true;
+}
+
 // A host call's poses, budgets and offsets together (tx .. offset, or budget .. ff_rx for
 // far-field antennas, lie together in the scratch): staged in the scene's host memory, from
-// where the call's first pass copies them if the device reaches it, or uploaded at once (the
-// copy has left the staging block when it returns).
+// where the call's first pass copies them if the device reaches it, or uploaded at once.
 static hsr_status upload_block(SceneDev &sc, Scratch &s, char *first, char *last,
                                std::initializer_list<std::pair<void *, std::pair<const void *, size_t>>> parts,
                                cudaStream_t st) {
     const size_t bytes = size_t(last - first);
-    if (sc.host_in_use) {  // the last call returned early, with its passes in flight
-        cudaDeviceSynchronize();
-        sc.host_in_use = false;
-    }
+    begin_staging(sc);
     if (sc.stage.size() < bytes) sc.stage.resize(bytes);
     for (const auto &p : parts)
         std::memcpy(sc.stage.data() + (static_cast<char *>(p.first) - first), p.second.first, p.second.second);
     if (sc.host_direct) {
-        sc.host_in_use = true;
         s.host_src[0] = sc.stage.data();
         s.host_dst[0] = first;
         s.host_bytes[0] = bytes;
@@ -1295,9 +1300,12 @@ hsr_status hsr_simulate_batch_device(hsr_scene *s, const hsr_rf_config *rf, int3
         (e = cudaMemcpyAsync(o.data(), d_offset, 8 * P, cudaMemcpyDeviceToHost, strm)) != cudaSuccess ||
         (e = cudaStreamSynchronize(strm)) != cudaSuccess)
         return cuda_fail(e, "budget read-back");
+    begin_staging(s->dev);
     st = run_guided(s->dev, sc, rf, N, fl, P, b, o, phase_mode, splat_mode, 1, d_out_rows, strm, nullptr, nullptr);
-    if (st == HSR_OK && (e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "guided batch");
-    return st;
+    if (st != HSR_OK) return st;
+    if ((e = cudaStreamSynchronize(strm)) != cudaSuccess) return cuda_fail(e, "guided batch");
+    s->dev.host_in_use = false;
+    return HSR_OK;
 }
 
 hsr_status hsr_simulate_batch(hsr_scene *s, const hsr_rf_config *rf, int32_t N, const hsr_tracer_flags *fl, int32_t P,

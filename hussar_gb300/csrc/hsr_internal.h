@@ -116,7 +116,7 @@ struct SceneDev {
     // where the device writes them there itself (host_direct)
     std::vector<char> stage, stage_sched, stage_rows;
     bool host_direct = false;    // kernels reach pageable host memory (hsr_api.cu)
-    bool host_in_use = false;    // a call that uses those blocks has not been waited for
+    bool host_in_use = false;    // a call that uses those blocks has not been waited for (begin_staging)
     void *guide = nullptr;       // guiding trees + step scratch, sized for guide_cap poses
     int guide_cap = 0;
     SynthOperand synth;          // cached twiddle operand (fine-histogram synthesis)
