@@ -128,17 +128,17 @@ class FFAntenna:
         return a
 
 
-def _pack(antennas, count, cls, struct, columns, regular=lambda antennas: True):
+def _pack(antennas, count, cls, struct, columns):
     """`count` C structures (float fields only) of an iterable of antennas, as a float32 array:
-    the columns of all of them at once where each is a plain `cls` and they are `regular`,
-    to_c() of each otherwise; zeros where there are fewer. Two thousand poses' TX and RX take
-    0.8 ms, a ctypes structure filled for each 9."""
+    the columns of all of them at once where each is a plain `cls`, its to_c() otherwise;
+    zeros where there are fewer. Two thousand poses' TX and RX take 0.8 ms, a ctypes
+    structure filled for each 9."""
     antennas = list(antennas)
     if len(antennas) > count:
         raise IndexError("%d antennas for %d poses" % (len(antennas), count))
     out = np.zeros((count, ctypes.sizeof(struct) // 4), np.float32)
     rows = out[:len(antennas)]
-    if len(antennas) and all(type(a) is cls for a in antennas) and regular(antennas):
+    if set(map(type, antennas)) == {cls}:
         columns(rows, antennas)
     else:
         for row, a in zip(rows, antennas):
@@ -152,18 +152,20 @@ def _nf_columns(rows, antennas):
 
 
 def _ff_columns(rows, antennas):
-    rows[:, :3] = np.concatenate([a.direction for a in antennas]).reshape(-1, 3)
-    h = np.concatenate([a.polarization for a in antennas]).reshape(-1, 3)
-    rows[:, 3:9:2], rows[:, 4:9:2] = h.real, h.imag
-    rows[:, 9:12] = np.concatenate([a.scene_center for a in antennas]).reshape(-1, 3)
+    n = len(antennas)
+    v = _threes([a.direction for a in antennas] + [a.scene_center for a in antennas])
+    rows[:, :3], rows[:, 9:12] = v[:n], v[n:]
+    h = np.ascontiguousarray(_threes([a.polarization for a in antennas]), np.complex64)
+    rows[:, 3:9] = h.view(np.float32).reshape(n, 6)
     rows[:, 12] = [a.radius for a in antennas]
 
 
-def _ff_regular(antennas):
-    """Whether every antenna's vectors, which its user may have set, are as its constructor makes
-    them: side by side, one of another length would shift those after it."""
-    return all(getattr(v, "shape", None) == (3,) for a in antennas
-               for v in (a.direction, a.polarization, a.scene_center))
+def _threes(vectors):
+    """Vectors of three, which an antenna's user may have set, as rows: end to end, one of another
+    length would shift those after it."""
+    if set(map(len, vectors)) != {3}:
+        raise ValueError("an antenna's vectors have three components")
+    return np.concatenate(vectors).reshape(-1, 3)
 
 
 def _antenna_array(antennas, count):
@@ -173,7 +175,7 @@ def _antenna_array(antennas, count):
 
 def _ff_antenna_array(antennas, count):
     """hsr_ff_antenna[count] of an iterable of FFAntenna."""
-    return _pack(antennas, count, FFAntenna, _lib.FfAntennaC, _ff_columns, _ff_regular)
+    return _pack(antennas, count, FFAntenna, _lib.FfAntennaC, _ff_columns)
 
 
 class Scene:
