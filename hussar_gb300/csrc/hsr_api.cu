@@ -432,6 +432,8 @@ static hsr_status run_guided(SceneDev &sc, const Scratch &s, const hsr_rf_config
                 o[p] = it.offset + offsets[p];
                 w[p] = it.weight;
                 train[p] = it.train ? 1 : 0;
+                // never in the first iteration: its rows are zero already, and its flags still
+                // on their way to the device when it starts
                 clear[p] = (k > 0 && it.clear) ? 1 : 0;
                 if (it.clear) tw[p] = 0.0;
                 tw[p] += double(it.budget) * double(it.weight);  // path.h:445, 466-475
@@ -591,7 +593,11 @@ static hsr_status use_device_poses(Scratch &s, int32_t P, int32_t N, const hsr_a
     return HSR_OK;
 }
 
-constexpr size_t kSmallRows = 256 << 10;  // bytes
+// Rows up to this many bytes come in the fewest steps. Written to host memory by the device
+// against a download and a look at the status word (short dihedral batches, whole calls): 2 KB
+// 75 and 90 us, 64 KB 103 and 117, 128 KB 128 and 139, 254 KB 177 and 175, 512 KB 265 and
+// 247, 4 MB 1507 and 1286.
+constexpr size_t kSmallRows = 256 << 10;
 constexpr size_t kRowsHead = 256;         // the status word before them
 
 // Where a host call's rows are written: the scratch, or for small rows the scene's host memory

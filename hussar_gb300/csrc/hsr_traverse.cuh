@@ -290,8 +290,8 @@ struct Walk {
 
 // closest_hit's answer.
 __device__ __forceinline__ int closest_hit_in_step(bool active, const DNode *__restrict__ nodes,
-                                                   const DTri *__restrict__ tris, f3 o, f3 d, float tnear, float tfar, float &t_best, int &prim_best,
-                                                   unsigned *status) {
+                                                   const DTri *__restrict__ tris, f3 o, f3 d, float tnear,
+                                                   float tfar, float &t_best, int &prim_best, unsigned *status) {
     const RayPre rp = ray_pre(o, d);
     Walk w(active);
     int best = -1;

@@ -245,17 +245,18 @@ __device__ __forceinline__ float chirp_bandwidth(const hsr_rf_config &rf) { retu
 // at the end, so that the CTAs finish together. What is left is estimated from the CTA's
 // last run, assuming that every other CTA has pulled as much since: a fresh look at the
 // counter would cost a second trip to the L2 per pull.
-// Fixed 4096-sample items left the chip idle wherever a launch had few of them, since one
-// item is milliseconds of a CTA's time on a dense scene. Whole calls, fixed items -> runs:
-// one dihedral pose of 2^14 samples (4 items for 608 CTAs) 137 -> 98 us; 33 poses on
-// 100 k triangles of boxes (1.7 M samples) 21.9 -> 12.2 ms; 27 far-field poses x 2^14
-// 747 -> 480 us; urban, 12 x 2^19 samples, 8.3 -> 7.3 ms; 96 poses on 1 M triangles (14 M
-// samples) 101 -> 91 ms.
+// Fixed 4096-sample items left the chip idle wherever a launch had few of them. Whole calls,
+// fixed items -> runs, on the tree-walking forms (dense scenes did not have lists yet): one
+// dihedral pose of 2^14 samples (4 items for 608 CTAs) 137 -> 98 us; 33 poses on 100 k
+// triangles of boxes (1.7 M samples) 21.9 -> 12.2 ms; 27 far-field poses x 2^14 747 -> 480
+// us; urban, 12 x 2^19 samples, 8.3 -> 7.3 ms; 96 poses on 1 M triangles (14 M samples)
+// 101 -> 91 ms.
 // A CTA that changes pose drains its stack and reads the next pose's list, so runs are as
 // long as the balance allows: half the share was too much for poses that differ in cost
-// (96 boxes poses of 2^13 .. 2^18 samples 14.4 ms with R = 64 items; a third 12.7, a quarter
-// 12.8, a sixth 13.1), and R = 16 items too little for large batches (256 boxes poses of
-// 2^16 .. 2^22 samples 0.88e9 paths/s, R = 32 1.04e9, R = 64 1.20e9, R = 256 1.20e9).
+// (with lists, 96 boxes poses of 2^13 .. 2^18 samples 14.4 ms with R = 64 items; a third
+// 12.7, a quarter 12.8, a sixth 13.1), and R = 16 items too little for large batches (256
+// boxes poses of 2^16 .. 2^22 samples 0.88e9 paths/s, R = 32 1.04e9, R = 64 1.20e9, R = 256
+// 1.20e9).
 template <class Shared>
 __device__ __forceinline__ bool pull_items(const TraceParams &p, Shared &S, long long total) {
     long long want = 1;

@@ -187,7 +187,8 @@ hsr_status hsr_scene_bvh_stats(const hsr_scene *scene, int64_t *out_nodes,
  * kernel.cu:24-43). Rays start at tnear = 5e-5 (hussar.h:52, cpu.cpp:12).
  * origins/directions: count x 3 floats; tfar: count floats.
  * Outputs: t (inf on miss), hit point p (count x 3), faceforwarded unit normal n
- * (count x 3), primitive id (-1 on miss) / visible flags (1 = unoccluded). */
+ * (count x 3), primitive id (-1 on miss) / visible flags (1 = unoccluded). The arrays may
+ * lie at any address and outputs may overlap inputs (such calls go through copies). */
 hsr_status hsr_intersect(const hsr_scene *scene, int64_t count, const float *origins,
                          const float *directions, const float *tfar, float *out_t,
                          float *out_p, float *out_n, int32_t *out_prim);
@@ -276,9 +277,11 @@ hsr_status hsr_path_tracer_run(hsr_scene *scene, const hsr_rf_config *rf,
  * channel, path.h:291-292); complex64 interleaved.
  * All pointer arguments are DEVICE pointers (inputs already resident). Asynchronous
  * on `stream`; scratch is owned by the scene and reused across calls on it, so calls
- * on one scene must not overlap. With flags->doGuiding every pose runs the guided
- * schedule of hsr_path_tracer_run (its own tree); the schedule is planned on the host,
- * so that form reads the budgets back and synchronises between iterations. */
+ * on one scene must not overlap. Poses, budgets and offsets are read where they are until
+ * the work on `stream` is done, or copied first where d_out_rows overlaps them. With
+ * flags->doGuiding every pose runs the guided schedule of hsr_path_tracer_run (its own
+ * tree); the schedule is planned on the host, so that form reads the budgets back and
+ * returns once the work is done. */
 hsr_status hsr_simulate_batch_device(hsr_scene *scene, const hsr_rf_config *rf,
                                      int32_t samples_per_chirp, const hsr_tracer_flags *flags,
                                      int32_t pose_count, const hsr_antenna *d_tx,
@@ -339,7 +342,8 @@ hsr_status hsr_simulate_frame(hsr_scene *scene, const hsr_rf_config *rf, const h
  * call on a device looks the array's address up (make it before any stream capture).
  * The call must be issued with the scene's device current, uses the scene's tuned launch
  * shape and the kernel hsr_set_path_kernel selects, and returns before the GPU has run:
- * read its device status with hsr_noalloc_status. */
+ * read its device status with hsr_noalloc_status. It has no room for neighbourhood lists:
+ * on a dense scene every query walks the tree, at about four times the time. */
 hsr_status hsr_simulate_batch_device_noalloc(hsr_scene *scene, const hsr_rf_config *rf,
                                              int32_t samples_per_chirp,
                                              const hsr_tracer_flags *flags, int32_t pose_count,
@@ -427,13 +431,14 @@ hsr_status hsr_debug_sincos_sweep(float lo, float hi, int64_t *out_checked, int6
                                   int64_t *out_slow);
 
 /* ---- Autotuning of the plain wavefront launch ---------------------------------------
- * No counterpart in the reference. The launch shape of a plain batch: samples per work
- * item (tile), persistent CTAs per SM, and the queue threshold (GENERATE runs while a CTA
- * holds at most this many live paths; at most 256: thresholds up to 64 run a 320-entry
- * path stack, up to 128 a 384-entry one, above 128 a 512-entry one). Zero fields mean
- * the default shape (tile 16384, threshold 256; 128 for chirps of over 1536 samples).
- * Scenes dense enough for neighbourhood lists run one 384-entry stack (thresholds up to
- * 128) without the two forms that follow.
+ * No counterpart in the reference. The launch shape of a plain batch: the most samples a
+ * CTA takes at once (tile: of a multiple of 256 in runs of 256-sample items that shrink
+ * towards the end of the launch, of another size whole), persistent CTAs per SM, and the
+ * queue threshold (GENERATE runs while a CTA holds at most this many live paths; at most
+ * 256: thresholds up to 64 run a 320-entry path stack, up to 128 a 384-entry one, above 128
+ * a 512-entry one). Zero fields mean the default shape (tile 16384, threshold 256; 128 for
+ * chirps of over 1536 samples). Scenes dense enough for neighbourhood lists run one
+ * 384-entry stack (thresholds up to 128) without the two forms that follow.
  * field_on_hit = 1 forms a primary ray's antenna field
  * only once the ray has hit something (for indirect-only paths: the field of a ray that
  * misses is never used), which pays where most primary rays miss and costs registers
@@ -501,10 +506,10 @@ hsr_status hsr_last_kernel_ms(const hsr_scene *scene, float *out_ms);
  *
  * No counterpart in the reference (its GPU backend launches one pose per call). Captures
  * hsr_simulate_batch_device's plain method (doGuiding = 0) with the given phase and splat
- * modes for fixed device buffers once; every launch replays the whole batch (pose upload,
- * work-item prefix, the persistent trace launch, then the fetchFrame rows, or with
- * HSR_SPLAT_FINE_SYNTH the tensor-core synthesis of the rows) as one graph launch and
- * reads the buffers' current contents, so poses, budgets and offsets may change between
+ * modes for fixed device buffers once; every launch replays the whole batch (work-item
+ * prefix, on dense scenes the poses' neighbourhood lists, the persistent trace launch, then
+ * the fetchFrame rows, or with HSR_SPLAT_FINE_SYNTH the tensor-core synthesis of the rows)
+ * as one graph launch and reads the buffers' current contents, so poses, budgets and offsets may change between
  * launches (the pose count, N, chirp and flags may not). The graph owns its scratch (and,
  * for synthesis, its own twiddle operand); it uses the scene's BVH and launch shape, so
  * destroy it before the scene. hsr_launch_count counts a replay as the kernels it runs. */
