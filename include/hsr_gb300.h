@@ -465,6 +465,8 @@ hsr_status hsr_autotune_batch(hsr_scene *scene, const hsr_rf_config *rf, int32_t
                               int32_t phase_mode, int32_t splat_mode, hsr_launch_config *out_best);
 /* Sets the scene's launch shape (NULL: the default). */
 hsr_status hsr_set_launch_config(hsr_scene *scene, const hsr_launch_config *config);
+/* The scene's launch shape: zeros where it is the default's, except for the threshold of a
+ * default that won hsr_autotune_batch, which is the one it ran the batch with. */
 hsr_status hsr_get_launch_config(const hsr_scene *scene, hsr_launch_config *out);
 
 /* Which trace kernel the simulate calls use (process-wide): 0 (default) = the wavefront
